@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "../../include/jcg.h"
+#include "jcg_px.cuh"
 
 namespace jcg {
 
@@ -97,6 +98,7 @@ struct ConstTables {
   float2 atab_chi_ff[NCHI];    // pair copy of atab_chi
   float2 chi_h6_ff[NCHI];      // (lna_chi[i] - lna_chi[i - 1]) / 6 as pairs (i >= 1; 0 at i = 0)
   float2 romb_w_ff[NROMB];     // pair copy of romb_w
+  alignas(16) PxTab px;        // tables of the pair exp2, log and sin (jcg_px.cuh)
 };
 
 // ------------------------------------------------- per-cosmology tables -----
@@ -554,9 +556,36 @@ __device__ __forceinline__ double growth_scan_warp(const double* Mv, double ya, 
 // the first step has h = 0), then chi_i = Y[-1] - Y_i.  fnode: f at the
 // nodes; fmid[i]: f at the midpoint of step i (i >= 1).  Lane l holds nodes
 // 8l .. 8l + 7; the sums are associated per lane, then across lanes.
+//
+// SUFFIX: the same chi_i as the sum of the increments above i, Y[-1] - Y_i
+// without the subtraction, whose rounding (1e-12 of chi's 10^4 Mpc/h) is 1e-14
+// of a chi of 100 Mpc/h.
+template <bool SUFFIX>
 __device__ __forceinline__ void chi_scan_warp(const double* fnode, const double* fmid, const double* lna, int lane,
                                               double* out) {
   double loc[8], s = 0.0;
+  if (SUFFIX) {
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+      const int i = lane * 8 + k;
+      loc[k] = s;
+      if (i > 0) {
+        const double hh = lna[i] - lna[i - 1];
+        s += 1.0 / 6.0 * hh * (fnode[i - 1] + 2 * fmid[i] + 2 * fmid[i] + fnode[i]);
+      }
+    }
+    double x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double u = __shfl_down_sync(0xffffffffu, x, o);
+      if (lane + o < 32) x += u;
+    }
+    double off = __shfl_down_sync(0xffffffffu, x, 1);
+    if (lane == 31) off = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[lane * 8 + k] = off + loc[k];
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int i = lane * 8 + k;
@@ -794,6 +823,7 @@ __device__ __forceinline__ void ku_get_rec(const float4* rec, int& q, float& dx,
 
 void launch_tracer_kernels(const Batch& b, const ConstTables* c, cudaStream_t st);
 void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st);
+void launch_limber64(const Batch& b, const ConstTables* c, cudaStream_t st);
 // derivatives (jcg_grad.cu)
 size_t grad_workspace_bytes(const GeoHeader& h, int n_cosmo, int precision);
 void grad_run(const GeoHeader* geo, const GeoHeader& h, const double* params, int n_cosmo, int precision,

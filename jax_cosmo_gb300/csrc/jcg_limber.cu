@@ -11,9 +11,9 @@
 // nodes: the chunk's per-a rows and M_ij are staged in shared memory, every
 // thread evaluates Eisenstein-Hu x primordial x halofit at (ell, a) nodes into
 // a P tile, then the CTA contracts the P tile with M into per-thread
-// accumulators.  FP64: the reference's formula order.  FP32C: MUFU forms of the
-// same formulas (ex2/lg2/rcp/sin), per-chunk partial sums added with Kahan
-// compensation across chunks.
+// accumulators: MUFU forms of the formulas (ex2/lg2/rcp/sin), per-chunk partial
+// sums added with Kahan compensation across chunks.  This file holds the fp32c
+// form; the plain method's is jcg_limber64.cu.
 #include "jcg_internal.cuh"
 #include "jcg_fp32.cuh"
 
@@ -22,7 +22,6 @@ namespace jcg {
 constexpr int LB_THREADS = 256;
 constexpr int LB_TA = 32;   // a nodes per chunk
 constexpr int LB_MAXLT = 32;
-constexpr int LB_MAXO = (LB_MAXLT * MAXPAIR + LB_THREADS - 1) / LB_THREADS;  // 17
 
 // Per-cosmology Eisenstein & Hu constants of the FP32 node.
 // Eisenstein-Hu T(k) in FP32 (transfer.py:88-153, either type) at k, lk =
@@ -95,17 +94,6 @@ __device__ __forceinline__ float pk32_T(const EH32& e, const float* r, float k, 
   return TWO_PI2_F * (invk * invk * invk) * (d2q + d2h);
 }
 
-// Both at one node: kh = l + 1/2, lg2kh = log2(kh), invkh = 1 / kh.
-template <bool GEN>
-__device__ __forceinline__ float node32(const EH32& e, const float* r, float kh, float lg2kh,
-                                        float invkh, bool lin) {
-  const float k = kh * r[F_INVCHI];
-  const float lk = lg2kh + r[F_LG2INVCHI];
-  const float invk = invkh * r[F_CHIC];
-  const float T = eh32_T<GEN>(e, k, lk, invk);
-  return pk32_T<GEN>(e, r, k, lk, invk, ex2f(e.ns3 * lk) * (T * T), lin);
-}
-
 // T(k)^2 k^(n_s + 3) table of the fp32c Limber kernel: NTT nodes uniform in
 // log2 k over the range of one CTA's nodes, values by 4-point Lagrange
 // interpolation (error O(h^4): about 1e-7 relative for the baryon wiggles at
@@ -122,129 +110,6 @@ __device__ __forceinline__ float tt_interp(const float* tab, float lk, float lk0
          (1.f / 6.f) * (b * tm1) * tab[i + 2];
 }
 
-
-// ---------------------------------------------------------------- kernel ---
-// MAXO: accumulators per thread, >= ceil(LT * n_cls / LB_THREADS).
-template <bool FP32, int MAXO>
-__global__ void __launch_bounds__(LB_THREADS)
-    limber_kernel(Batch bt, const ConstTables* __restrict__ c, int LT) {
-  using T = typename std::conditional<FP32, float, double>::type;
-  constexpr int RW = FP32 ? NROW32 : NROW64;
-  const int item = blockIdx.y;
-  if (item >= bt.n_items) return;
-  const Item it = batch_item(bt, item);
-  const GeoHeader* geo = it.geo;
-  const int n_ell = geo->n_ell, n_cls = geo->n_cls, na = geo->na;
-  const int model = pk_model(it.physics);
-  const bool lin = model == JCG_PK_LINEAR;
-  const int l0 = blockIdx.x * LT;
-  if (l0 >= n_ell) return;
-  const int lt = min(LT, n_ell - l0);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* s = reinterpret_cast<double*>(smem_raw);    // NSCAL
-  EH32* e32 = reinterpret_cast<EH32*>(s + NSCAL);     // 1 (padded to 8 doubles)
-  double* ellv = s + NSCAL + 8;                        // LB_MAXLT: l + 1/2 (FP64 path)
-  double* lellv = ellv + LB_MAXLT;                     // LB_MAXLT: log(l + 1/2)
-  float* kh32 = reinterpret_cast<float*>(lellv + LB_MAXLT);  // 3 * LB_MAXLT floats
-  T* rowsS = reinterpret_cast<T*>(kh32 + 3 * LB_MAXLT);      // TA * RW
-  T* Ms = rowsS + LB_TA * RW;                                // TA * n_cls
-  T* Pt = Ms + LB_TA * n_cls;                                // TA * LT
-  const int tid = threadIdx.x;
-  const double* ELL = geo_ptr<double>(geo, geo->off_ell);
-  const double* EF = geo_ptr<double>(geo, geo->off_ellfac);
-  for (int i = tid; i < NSCAL; i += LB_THREADS) s[i] = it.ctab->s[i];
-  for (int l = tid; l < lt; l += LB_THREADS) {
-    const double e = ELL[l0 + l] + 0.5;
-    ellv[l] = e;
-    lellv[l] = log(e);
-    kh32[3 * l + 0] = (float)e;                               // k = kh / max(chi, 1)
-    kh32[3 * l + 1] = (float)(1.4426950408889634 * log(e));   // log2(kh)
-    kh32[3 * l + 2] = (float)(1.0 / e);                       // 1 / kh
-  }
-  __syncthreads();
-  if (FP32 && tid == 0) make_eh32(s, e32);
-  __syncthreads();
-  const double* rows64 = it.rows64;
-  const float* rows32 = it.rows32;
-  const double* kern = it.kern;
-  const int nout = lt * n_cls;
-  T acc[MAXO], comp[MAXO];
-#pragma unroll
-  for (int r = 0; r < MAXO; ++r) {
-    acc[r] = 0;
-    comp[r] = 0;
-  }
-  for (int base = 0; base < na; base += LB_TA) {
-    const int tc = min(LB_TA, na - base);
-    // stage rows
-    if (FP32) {
-      for (int i = tid; i < tc * RW; i += LB_THREADS)
-        rowsS[i] = (T)rows32[(size_t)base * NROW32 + i];
-    } else {
-      for (int i = tid; i < tc * RW; i += LB_THREADS)
-        rowsS[i] = (T)rows64[(size_t)base * NROW64 + i];
-    }
-    // M_ij(a) = u_a K_i(a) K_j(a)
-    for (int q = tid; q < tc * n_cls; q += LB_THREADS) {
-      const int t = q / n_cls, p = q - (q / n_cls) * n_cls;
-      const int n = base + t;
-      const double ki = kern[(size_t)geo->pair_i[p] * na + n];
-      const double kj = kern[(size_t)geo->pair_j[p] * na + n];
-      const double u = rows64[(size_t)n * NROW64 + R_U];
-      if (FP32)
-        Ms[t * n_cls + p] = (T)((float)ki * (float)kj * (float)u);
-      else
-        Ms[t * n_cls + p] = (T)((ki * kj) * u);
-    }
-    __syncthreads();
-    // P tile: nodes (t, l)
-    for (int q = tid; q < tc * lt; q += LB_THREADS) {
-      const int t = q / lt, l = q - (q / lt) * lt;
-      T pv;
-      if (FP32) {
-        pv = (T)node32<true>(*e32, reinterpret_cast<const float*>(rowsS) + t * NROW32, kh32[3 * l],
-                       kh32[3 * l + 1], kh32[3 * l + 2], lin);
-      } else {
-        const double* row = reinterpret_cast<const double*>(rowsS) + t * NROW64;
-        const double k = ellv[l] / fmax(row[R_CHI], 1.0);
-        pv = (T)halofit_node_lk(s, row, k, lellv[l] - row[R_LGCHIC], model);
-      }
-      Pt[t * LT + l] = pv;
-    }
-    __syncthreads();
-    // contraction
-#pragma unroll
-    for (int r = 0; r < MAXO; ++r) {
-      const int o = tid + r * LB_THREADS;
-      if (o < nout) {
-        const int l = o % lt, p = o / lt;
-        T part = 0;
-        for (int t = 0; t < tc; ++t) part += Pt[t * LT + l] * Ms[t * n_cls + p];
-        if (FP32) {
-          const T y = part - comp[r];
-          const T tt = acc[r] + y;
-          comp[r] = (tt - acc[r]) - y;
-          acc[r] = tt;
-        } else {
-          acc[r] += part;
-        }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int r = 0; r < MAXO; ++r) {
-    const int o = tid + r * LB_THREADS;
-    if (o < nout) {
-      const int l = o % lt, p = o / lt;
-      const int ell = l0 + l;
-      const double efi = EF[(size_t)geo->pair_i[p] * n_ell + ell];
-      const double efj = EF[(size_t)geo->pair_j[p] * n_ell + ell];
-      const double v = FP32 ? ((double)acc[r] - (double)comp[r]) : (double)acc[r];
-      it.cl[(size_t)p * n_ell + ell] = v * efi * efj;
-    }
-  }
-}
 
 // ------------------------------------------------------- fp32c kernel ----
 // The fp32c Limber integral with a register-blocked contraction: a work unit
@@ -468,32 +333,6 @@ static void launch_limber32_t(const Batch& b, const ConstTables* c, int lt, cuda
   limber32_kernel<MAXU, GEN><<<grid, LB_THREADS, L.total, st>>>(b, c, lt);
 }
 
-size_t limber_smem_bytes(bool fp32, int n_cls, int LT) {
-  const size_t el = fp32 ? 4 : 8;
-  const size_t rw = fp32 ? NROW32 : NROW64;
-  return (NSCAL + 8 + 2 * LB_MAXLT) * 8 + 3 * LB_MAXLT * 4 +
-         el * (LB_TA * rw + (size_t)LB_TA * n_cls + (size_t)LB_TA * LT);
-}
-
-template <bool FP32, int MAXO>
-static void launch_limber_t(const Batch& b, const ConstTables* c, int lt, size_t smem, dim3 grid,
-                            cudaStream_t st) {
-  cudaFuncSetAttribute(limber_kernel<FP32, MAXO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  limber_kernel<FP32, MAXO><<<grid, LB_THREADS, smem, st>>>(b, c, lt);
-}
-
-template <bool FP32>
-static void launch_limber_p(const Batch& b, const ConstTables* c, int lt, size_t smem, dim3 grid,
-                            cudaStream_t st) {
-  const int need = (lt * b.max_cls + LB_THREADS - 1) / LB_THREADS;
-  if (need <= 1) launch_limber_t<FP32, 1>(b, c, lt, smem, grid, st);
-  else if (need <= 2) launch_limber_t<FP32, 2>(b, c, lt, smem, grid, st);
-  else if (need <= 4) launch_limber_t<FP32, 4>(b, c, lt, smem, grid, st);
-  else if (need <= 8) launch_limber_t<FP32, 8>(b, c, lt, smem, grid, st);
-  else launch_limber_t<FP32, LB_MAXO>(b, c, lt, smem, grid, st);
-}
-
 void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st) {
   if (b.precision == JCG_FP32C) {
     // units per thread: the split path needs one, otherwise lt x ceil(n_cls / 4)
@@ -515,9 +354,7 @@ void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st
     }
     return;
   }
-  const size_t smem = limber_smem_bytes(false, b.max_cls, lt);
-  dim3 grid((b.max_ell + lt - 1) / lt, b.n_items);
-  launch_limber_p<false>(b, c, lt, smem, grid, st);
+  launch_limber64(b, c, st);
 }
 
 }  // namespace jcg

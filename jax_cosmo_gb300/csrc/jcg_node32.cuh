@@ -24,7 +24,7 @@ struct EHg {
 // one sweep; an[T_MUN] is not written (the caller skips that projection).
 __device__ __forceinline__ float node32_fb_default(const EHg& e, const float* r, float kh, float lg2kh, float invkh,
                                            float* an, float* ae) {
-  // ---- forward (same operations as node32)
+  // ---- forward (the fp32c integrand)
   const float k = kh * r[F_INVCHI];
   const float lk = lg2kh + r[F_LG2INVCHI];
   const float invk = invkh * r[F_CHIC];
@@ -301,13 +301,13 @@ __device__ __forceinline__ float pk32_fb(const EHg& e, const float* r, float k, 
   return P;
 }
 
-// P of node32 (the forward fp32c integrand) and its reverse sweep, transfer
+// P of the forward fp32c integrand and its reverse sweep, transfer
 // type "eisenhu_osc".  an[GTan] (T_CHIC..T_MUN) and ae[ETan] receive
 // dP/d(input) in the units of the stored tangents.
 template <bool GEN>
 __device__ __forceinline__ float node32_fb(const EHg& e, const float* r, float kh, float lg2kh, float invkh,
                                            float* an, float* ae, bool lin) {
-  // ---- forward (same operations as node32)
+  // ---- forward (the fp32c integrand)
   const float k = kh * r[F_INVCHI];
   const float lk = lg2kh + r[F_LG2INVCHI];
   const float invk = invkh * r[F_CHIC];

@@ -169,6 +169,17 @@ __global__ void const_ff_kernel(ConstTables* c) {
     c->sincos_ff[2 * j] = f2_of(sin(a));
     c->sincos_ff[2 * j + 1] = f2_of(cos(a));
   }
+  for (int j = tid; j < 128; j += nth) {
+    c->px.ex[j] = f2_of(exp2((j + 0.5) / 128.0));
+    c->px.sc[2 * j] = f2_of(sinpi(j / 64.0));
+    c->px.sc[2 * j + 1] = f2_of(cospi(j / 64.0));
+  }
+  for (int j = tid; j < 256; j += nth) {
+    const double r = rint(512.0 / (1.0 + (j + 0.5) / 256.0)) / 512.0;
+    c->px.rc[j] = (float)r;
+    c->px.ln[j] = f2_of(-log(r));
+    c->px.l2[j] = __double2ll_rn(-log2(r) * 144115188075855872.0);
+  }
   for (int e = tid; e < NROMB; e += nth) {
     c->romb_w_ff[e] = f2_of(c->romb_w[e]);
     c->romb_k_ff[e] = f2_of(c->romb_k[e]);
@@ -479,7 +490,7 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   }
   const int warp = t >> 5, lane = t & 31;
   if (warp == 0) {
-    chi_scan_warp(fnode, inc, c->lna_chi, lane, chis);
+    chi_scan_warp<!FAST>(fnode, inc, c->lna_chi, lane, chis);
   } else if (warp == 2) {
     // sigmasqr(8) (power.py:70-78): romb is linear in the integrand values,
     // sum_e w_e f_e with the weights of its Richardson combination
