@@ -11,6 +11,7 @@
 #include "jcg_ff.cuh"
 #include "jcg_internal.cuh"
 #include "jcg_dual.cuh"
+#include "jcg_px_node.cuh"
 
 namespace jcg {
 
@@ -221,29 +222,6 @@ __device__ void halofit_coefs_fast(const double* s, float om_m, float om_de, flo
   row[R_LGCHIC] = -0.6931471805599453 * f[F_LG2INVCHI];
 }
 
-// FP32 row of the compensated fast path from the FP64 row.
-__device__ void row32_from_row64(const double* s, const double* r, float* f) {
-  const double chic = fmax(r[R_CHI], 1.0);
-  constexpr double LOG2E = 1.4426950408889634;
-  f[F_INVCHI] = (float)(1.0 / chic);
-  f[F_CHIC] = (float)chic;
-  f[F_LG2INVCHI] = (float)(-LOG2E * r[R_LGCHIC]);
-  f[F_LG2KNL] = (float)(LOG2E * r[R_LGKNL]);
-  f[F_INVKNL] = (float)(1.0 / r[R_KNL]);
-  f[F_D2FAC] = (float)(r[R_G] * r[R_G] * s[S_PKNORM] / TWO_PI2);
-  f[F_BETAN] = (float)r[R_BETAN];
-  f[F_ALPHAN] = (float)r[R_ALPHAN];
-  f[F_AN] = (float)r[R_AN];
-  f[F_3F1] = (float)(3.0 * r[R_F1]);
-  f[F_F2] = (float)r[R_F2];
-  f[F_BN] = (float)r[R_BN];
-  f[F_LG2CF3] = (float)(LOG2E * r[R_LGCF3]);
-  f[F_3MGAMMA] = (float)(3.0 - r[R_GAMMAN]);
-  f[F_NUN] = (float)r[R_NUN];
-  f[F_MUN] = (float)r[R_MUN];
-  for (int i = NROW32_USED; i < NROW32; ++i) f[i] = 0.f;
-}
-
 // chi and growth at a from the tables (background.py:242, 488) with the
 // segment chosen by the reference's rule and the precomputed chi slopes.
 __device__ __forceinline__ double chi_at(const CosmoTab* ct, const ConstTables* c, double a, int2 seg) {
@@ -252,16 +230,13 @@ __device__ __forceinline__ double chi_at(const CosmoTab* ct, const ConstTables* 
 }
 
 constexpr int HF_WARPS = 8;
-// Limber nodes per CTA: the fp32c rows keep every thread busy in the
-// thread-per-node phases (256 nodes); the float64 rows, whose warp-per-node
-// moments dominate, use 64
-__host__ __device__ constexpr int hf_nodes_per_block(bool fast) { return fast ? 256 : 64; }
+constexpr int HF_NODES = 256;  // fp32c: Limber nodes per CTA (every thread busy in the thread-per-node phases)
 
-// Root find of one node by one thread: c = #{j : sig_j g2 > 1} by bisection
-// (the sequence is strictly decreasing), then the argmin among c - 1, c with
-// the first index on ties -- the same index as argmin((1 - sig g2)^2).
-__device__ __forceinline__ double root_knl_thread(const double* sig, double g2,
-                                                  const ConstTables* __restrict__ c) {
+// argmin_j (1 - sig_j g2)^2 with the first index on ties, by one thread: c =
+// #{j : sig_j g2 > 1} by bisection (the sequence is strictly decreasing), then
+// the nearer of c - 1, c; and the other end of the segment on the side of
+// sign(clip(1, v_1, v_{n-2}) - v_ind) (scipy/interpolate.py:47-57).
+__device__ __forceinline__ void root_segment(const double* sig, double g2, int& ind, int& j2) {
   int lo = 0, hi = NRT;  // invariant: v_j > 1 for j < lo, v_j <= 1 for j >= hi
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
@@ -279,17 +254,9 @@ __device__ __forceinline__ double root_knl_thread(const double* sig, double g2,
       best = cc - 1;
     }
   }
-  const int ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-  const double xp_ind = sig[ind] * g2;
-  const double lo_v = sig[1] * g2, hi_v = sig[NRT - 2] * g2;
-  const double xc = fmin(fmax(1.0, lo_v), hi_v);  // clip(x, xp[1], xp[-2])
-  const int sgn = (xc - xp_ind >= 0.0) ? 1 : -1;
-  const int j2 = ind + sgn;
-  const double slope = (c->logr[j2] - c->logr[ind]) / (sig[j2] * g2 - xp_ind);
-  const double b = c->logr[ind] - slope * xp_ind;
-  const double root = slope * 1.0 + b;
-  const double R = fmax(exp(root), 1e-6);  // power.py:113-115
-  return 1.0 / R;                          // power.py:118
+  ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
+  const double xc = fmin(fmax(1.0, sig[1] * g2), sig[NRT - 2] * g2);  // clip(x, xp[1], xp[-2])
+  j2 = ind + ((xc - sig[ind] * g2 >= 0.0) ? 1 : -1);
 }
 
 // fp32c: the same root find with the interpolation (power.py:112-115) in
@@ -298,53 +265,32 @@ __device__ __forceinline__ double root_knl_thread(const double* sig, double g2,
 // the pair quotient and exp.  Returns R = 1 / k_nl.
 __device__ __forceinline__ FF root_R_ff(const double* sig, double g2, const ConstTables* __restrict__ c,
                                         const float2* e2) {
-  int lo = 0, hi = NRT;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (sig[mid] * g2 > 1.0) lo = mid + 1;
-    else hi = mid;
-  }
-  const int cc = lo;
-  int best = cc < NRT ? cc : NRT - 1;
-  if (cc >= 1) {
-    const double dlo = 1.0 - sig[cc - 1] * g2;
-    if (cc < NRT) {
-      const double dhi = 1.0 - sig[cc] * g2;
-      best = (dlo * dlo <= dhi * dhi) ? cc - 1 : cc;
-    } else {
-      best = cc - 1;
-    }
-  }
-  const int ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
+  int ind, j2;
+  root_segment(sig, g2, ind, j2);
   const double xp_ind = sig[ind] * g2;
-  const double lo_v = sig[1] * g2, hi_v = sig[NRT - 2] * g2;
-  const double xc = fmin(fmax(1.0, lo_v), hi_v);
-  const int j2 = ind + ((xc - xp_ind >= 0.0) ? 1 : -1);
   const FF slope = ff_of(c->logr[j2] - c->logr[ind]) / ff_of(sig[j2] * g2 - xp_ind);
   const FF root = ff_of(c->logr[ind]) + slope * ff_of(1.0 - xp_ind);
   const FF R = ff_exp(root, e2);
   return R.hi < 1e-6f ? ff_of(1e-6) : R;  // power.py:115
 }
 
-// Three phases per block of Limber nodes:
-//  1a thread per node: growth, chi, root find, k_nl; FAST: the exp index
-//     range and the Taylor part of the moments;
+// The fp32c rows, three phases per block of Limber nodes:
+//  1a thread per node: growth, chi, root find, k_nl, the exp index range and
+//     the Taylor part of the moments;
 //  1b warp per node: the exp part of the moments (power.py:121-136);
 //  2  thread per node: n_eff, C and the takahashi2012 coefficients.
-// A block takes 64 nodes of one cosmology (float64), or 256 consecutive
-// nodes of the batch's flat (cosmology, node) index (fp32c, one geometry,
-// at least 256 nodes per cosmology: each block spans at most two
-// cosmologies, whose tables it holds side by side, and no block runs short),
-// or 256 nodes of one cosmology (fp32c otherwise).
+// A block takes 256 consecutive nodes of the batch's flat (cosmology, node)
+// index (one geometry, at least 256 nodes per cosmology: each block spans at
+// most two cosmologies, whose tables it holds side by side, and no block runs
+// short), or 256 nodes of one cosmology (otherwise).
 __host__ __device__ inline bool hf_flat(const Batch& b) {
-  return b.precision == JCG_FP32C && !b.listed && b.max_na >= hf_nodes_per_block(true);
+  return !b.listed && b.max_na >= HF_NODES;
 }
-template <bool FAST>
-__global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
+__global__ void __launch_bounds__(HF_WARPS * 32, 6)
     halofit_rows_kernel(Batch bt, const ConstTables* __restrict__ c) {
-  constexpr int NB = hf_nodes_per_block(FAST);
-  constexpr int NSL = FAST ? 2 : 1;  // cosmologies per block at most
-  const bool flat = FAST && hf_flat(bt);
+  constexpr int NB = HF_NODES;
+  constexpr int NSL = 2;  // cosmologies per block at most
+  const bool flat = hf_flat(bt);
   int item0, n0, cnt, nsl;
   if (flat) {
     const long long f0 = (long long)blockIdx.x * NB, nf = (long long)bt.n_items * bt.max_na;
@@ -368,29 +314,22 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
   const int na = geo->na;
   const int model = pk_model(itA.physics);
   __shared__ double sigS[NSL][NRT];
-  __shared__ double pk3[FAST ? 1 : NKH];
   __shared__ double sS[NSL][NSCAL];
-  __shared__ double knl_s[NB], inv_s[NB], g_s[NB], chi_s[NB], t1_s[NB], t2_s[NB], s1_s[NB], s2_s[NB];
+  __shared__ double knl_s[NB], inv_s[NB], g_s[NB], chi_s[NB], t1_s[NB], t2_s[NB];
   __shared__ int ilo_s[NB], ihi_s[NB];
   __shared__ float iv2h_s[NB], iv2l_s[NB], f1_s[NB], f2_s[NB];
-  __shared__ float wpfS[NSL][FAST ? NKH : 1], k2h[FAST ? NKH + 1 : 1], k2l[FAST ? NKH + 1 : 1];
-  __shared__ float2 e2s[FAST ? 64 : 1];
-  if (FAST)
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) e2s[i] = c->exp2_ff[i];
+  __shared__ float wpfS[NSL][NKH], k2h[NKH + 1], k2l[NKH + 1];
+  __shared__ float2 e2s[64];
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) e2s[i] = c->exp2_ff[i];
   for (int k = 0; k < nsl; ++k) {
     const CosmoTab* ctk = k ? itB.ctab : itA.ctab;
     for (int i = threadIdx.x; i < NRT; i += blockDim.x) sigS[k][i] = ctk->sig[i];
     for (int i = threadIdx.x; i < NSCAL; i += blockDim.x) sS[k][i] = ctk->s[i];
-    if (FAST)
-      for (int i = threadIdx.x; i < NKH; i += blockDim.x) wpfS[k][i] = ctk->wpk3f[i];
+    for (int i = threadIdx.x; i < NKH; i += blockDim.x) wpfS[k][i] = ctk->wpk3f[i];
   }
-  if (FAST) {
-    for (int i = threadIdx.x; i < NKH + 1; i += blockDim.x) {
-      k2h[i] = c->kh2_hi[i];
-      k2l[i] = c->kh2_lo[i];
-    }
-  } else {
-    for (int i = threadIdx.x; i < NKH; i += blockDim.x) pk3[i] = itA.ctab->pk3[i];
+  for (int i = threadIdx.x; i < NKH + 1; i += blockDim.x) {
+    k2h[i] = c->kh2_hi[i];
+    k2l[i] = c->kh2_lo[i];
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -407,22 +346,13 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
     const double* sig = sigS[slt];
     const CosmoTab* ct = slt ? itB.ctab : itA.ctab;
     const double a = A[n];
-    double g, knl, inv;
-    FF iv2;
-    if (FAST) {
-      // growth by the segment's node spacing reciprocal (no float64 division)
-      const int2 sg = unpack_seg(SG[n]);
-      const double sl = (ct->g[sg.y] - ct->g[sg.x]) * c->grow_ida[min(sg.x, sg.y)] * (sg.y > sg.x ? 1.0 : -1.0);
-      g = clip_lohi(ct->g[sg.x] + sl * (a - c->atab_grow[sg.x]), 0.0, 1.0);
-      const FF R = root_R_ff(sig, g * g, c, e2s);
-      inv = ffd(R);
-      knl = ffd(ff_rcp(R));
-      iv2 = ff_sqr(R);
-    } else {
-      g = clip_lohi(interp_eval(a, c->atab_grow, ct->g, unpack_seg(SG[n])), 0.0, 1.0);
-      knl = root_knl_thread(sig, g * g, c);
-      inv = 1.0 / knl;  // y = k * (1 / k_nl)
-    }
+    // growth by the segment's node spacing reciprocal (no float64 division)
+    const int2 sg = unpack_seg(SG[n]);
+    const double sl = (ct->g[sg.y] - ct->g[sg.x]) * c->grow_ida[min(sg.x, sg.y)] * (sg.y > sg.x ? 1.0 : -1.0);
+    const double g = clip_lohi(ct->g[sg.x] + sl * (a - c->atab_grow[sg.x]), 0.0, 1.0);
+    const FF R = root_R_ff(sig, g * g, c, e2s);
+    const double inv = ffd(R), knl = ffd(ff_rcp(R));
+    const FF iv2 = ff_sqr(R);
     g_s[t] = g;
     knl_s[t] = knl;
     inv_s[t] = inv;
@@ -431,7 +361,7 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
     double t1 = 0.0, t2 = 0.0;
     if (model == JCG_PK_LINEAR) {
       ihi = -1;  // linear_matter_power: the halofit moments are not used
-    } else if (FAST) {
+    } else {
       // exp only for y^2 in [Y2_TAYLOR, Y2_SKIP] (the split point only needs
       // to be consistent, so it is found in FP32); y^2 = kh^2 inv^2 with
       // inv^2 as a float pair for the FP32 terms
@@ -475,51 +405,30 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
   __syncthreads();
   // phase 1b
   for (int t = warp; t < cnt; t += HF_WARPS) {
-    const double inv = inv_s[t];
     const float* wpf = wpfS[slot_of(t)];
-    double s1 = 0.0, s2 = 0.0;
-    if (FAST) {
-      // FP32 terms: y^2 = kh^2 inv^2 as a float pair (hi p, lo e), exp(-y^2)
-      // from the pair, weights w pk3 rounded once to float
-      const float ih = iv2h_s[t], il = iv2l_s[t];
-      float f1 = 0.f, f2 = 0.f;
-      for (int i = ilo_s[t] + lane; i <= ihi_s[t]; i += 32) {
-        const float kh = k2h[i];
-        const float p = kh * ih;
-        float e = fmaf(kh, ih, -p);
-        e = fmaf(kh, il, e);
-        e = fmaf(k2l[i], ih, e);
-        const float r = wpf[i] * exp_neg_pair(p, e);
-        const float y2 = p + e;
-        f1 = fmaf(2.f * r, y2, f1);
-        f2 = fmaf(4.f * r, y2 * ((1.f - p) - e), f2);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-        f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-      }
-      if (lane == 0) {
-        f1_s[t] = f1;
-        f2_s[t] = f2;
-      }
-    } else {
-      const double g2 = g_s[t] * g_s[t];
-      for (int i = lane; i <= ihi_s[t]; i += 32) {
-        const double y = c->kh[i] * inv;
-        const double y2 = y * y;
-        const double res = pk3[i] * exp(-y2) * g2 / TWO_PI2;
-        s1 += c->simpson_kh[i] * (2 * res * y2);
-        s2 += c->simpson_kh[i] * (4 * res * (y2 - y2 * y2));
-      }
+    // FP32 terms: y^2 = kh^2 inv^2 as a float pair (hi p, lo e), exp(-y^2)
+    // from the pair, weights w pk3 rounded once to float
+    const float ih = iv2h_s[t], il = iv2l_s[t];
+    float f1 = 0.f, f2 = 0.f;
+    for (int i = ilo_s[t] + lane; i <= ihi_s[t]; i += 32) {
+      const float kh = k2h[i];
+      const float p = kh * ih;
+      float e = fmaf(kh, ih, -p);
+      e = fmaf(kh, il, e);
+      e = fmaf(k2l[i], ih, e);
+      const float r = wpf[i] * exp_neg_pair(p, e);
+      const float y2 = p + e;
+      f1 = fmaf(2.f * r, y2, f1);
+      f2 = fmaf(4.f * r, y2 * ((1.f - p) - e), f2);
     }
-    if (!FAST) {
-      s1 = warp_sum(s1);
-      s2 = warp_sum(s2);
-      if (lane == 0) {
-        s1_s[t] = s1;
-        s2_s[t] = s2;
-      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      f1 += __shfl_xor_sync(0xffffffffu, f1, o);
+      f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+    }
+    if (lane == 0) {
+      f1_s[t] = f1;
+      f2_s[t] = f2;
     }
   }
   __syncthreads();
@@ -531,12 +440,9 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
     float* const rows32 = slt ? itB.rows32 : itA.rows32;
     float* const u32 = slt ? itB.u32 : itA.u32;
     const double a = A[n];
-    double s1 = FAST ? (double)f1_s[t] : s1_s[t], s2 = FAST ? (double)f2_s[t] : s2_s[t];
-    if (FAST) {
-      const double g2 = g_s[t] * g_s[t] * (1.0 / TWO_PI2);
-      s1 = (s1 + 2.0 * t1_s[t]) * g2;
-      s2 = (s2 + 4.0 * t2_s[t]) * g2;
-    }
+    const double g2 = g_s[t] * g_s[t] * (1.0 / TWO_PI2);
+    const double s1 = ((double)f1_s[t] + 2.0 * t1_s[t]) * g2;
+    const double s2 = ((double)f2_s[t] + 4.0 * t2_s[t]) * g2;
     HfParams hp;
     hp.knl = knl_s[t];
     hp.neff = s1 - 3.0;  // power.py:138-139
@@ -547,61 +453,251 @@ __global__ void __launch_bounds__(HF_WARPS * 32, FAST ? 6 : 1)
     row[R_CHI] = chiv;
     row[R_G] = g_s[t];
     float f[NROW32];
-    if (FAST) {
-      // background in FP32 (background.py:122-126, 168, 196, 270-294):
-      // E^2(a), Omega_m(a), Omega_de(a), w(a), dchi/da
-      const float af = (float)a, ia = rcpf(af), ia2 = ia * ia;
-      const float w0 = (float)s[S_W0], wa = (float)s[S_WA];
-      const float fde = -3.f * (1.f + w0 + wa) * (LN2_F * lg2f(af)) + 3.f * wa * (af - 1.f);
-      const float ef = fde == 0.f ? 1.f : ex2f(fde * LOG2E_F);
-      const float om3 = (float)s[S_OMEGA_M] * (ia2 * ia), ode = (float)s[S_OMEGA_DE] * ef;
-      const float e2 = om3 + (float)s[S_OMEGA_K] * ia2 + ode;
-      const float ie2 = rcpf(e2);
-      const float omm = om3 * ie2, omde = ode * ie2, wv = w0 + (1.f - af) * wa;
-      halofit_coefs_fast(s, omm, omde, wv, hp, chiv, g_s[t], row, f, model);
-      const float dchi = (float)RH * ia2 * rsqrtf(e2);
-      const float chic = fmaxf((float)chiv, 1.f);
-      row[R_DCHI] = dchi;
-      const float uf = (float)WS[n] * dchi * rcpf(chic * chic) * (float)(1.0 / C2);
-      row[R_U] = (double)uf;
-      if (u32) u32[n] = uf;  // the Limber kernel's float copy
-    } else {
-      const double lna = log(a);
-      const Bg bg = make_bg(s);
-      halofit_coefs(bg, a, lna, hp, row, model);
-      row[R_LGCHIC] = log(fmax(chiv, 1.0));
-      const double dchi = bg_dchioverda_l(bg, a, lna);
-      row[R_DCHI] = dchi;
-      row[R_U] = WS[n] * dchi / fmax(chiv * chiv, 1.0) / C2;
-    }
+    // background in FP32 (background.py:122-126, 168, 196, 270-294):
+    // E^2(a), Omega_m(a), Omega_de(a), w(a), dchi/da
+    const float af = (float)a, ia = rcpf(af), ia2 = ia * ia;
+    const float w0 = (float)s[S_W0], wa = (float)s[S_WA];
+    const float fde = -3.f * (1.f + w0 + wa) * (LN2_F * lg2f(af)) + 3.f * wa * (af - 1.f);
+    const float ef = fde == 0.f ? 1.f : ex2f(fde * LOG2E_F);
+    const float om3 = (float)s[S_OMEGA_M] * (ia2 * ia), ode = (float)s[S_OMEGA_DE] * ef;
+    const float e2 = om3 + (float)s[S_OMEGA_K] * ia2 + ode;
+    const float ie2 = rcpf(e2);
+    const float omm = om3 * ie2, omde = ode * ie2, wv = w0 + (1.f - af) * wa;
+    halofit_coefs_fast(s, omm, omde, wv, hp, chiv, g_s[t], row, f, model);
+    const float dchi = (float)RH * ia2 * rsqrtf(e2);
+    const float chic = fmaxf((float)chiv, 1.f);
+    row[R_DCHI] = dchi;
+    const float uf = (float)WS[n] * dchi * rcpf(chic * chic) * (float)(1.0 / C2);
+    row[R_U] = (double)uf;
+    if (u32) u32[n] = uf;  // the Limber kernel's float copy
     if (rows64) {
+      // the Limber weight and the halofit parameters (the rest of the
+      // integrand's inputs are in the FP32 row)
       double* dst = rows64 + (size_t)n * NROW64;
-      if (FAST) {
-        // fp32c: the Limber weight and the halofit parameters (the rest of
-        // the integrand's inputs are in the FP32 row)
-        constexpr int keep[] = {R_CHI, R_G, R_KNL, R_NEFF, R_C, R_DCHI, R_U};
+      constexpr int keep[] = {R_CHI, R_G, R_KNL, R_NEFF, R_C, R_DCHI, R_U};
 #pragma unroll
-        for (int q = 0; q < 7; ++q) dst[keep[q]] = row[keep[q]];
-      } else {
-        for (int i = 0; i < NROW64; ++i) dst[i] = row[i];
-      }
+      for (int q = 0; q < 7; ++q) dst[keep[q]] = row[keep[q]];
     }
     if (rows32) {
-      if (!FAST) row32_from_row64(s, row, f);
       float* dst = rows32 + (size_t)n * NROW32;
       for (int i = 0; i < NROW32; ++i) dst[i] = f[i];
     }
   }
 }
 
+// The float64 rows, float64-class numbers on the FP32 pipe where the work is
+// (jcg_px.cuh).  Bound: issue.  The moments (power.py:121-136) take up to 257
+// exponentials per node, each 35 FP64 operations in float64 (9,000 per node, on
+// a pipe of 1/64 rate); a term in pairs is about 130 FP32 and integer
+// instructions.  Terms with y^2 > 60 are below 1e-20 of the sums and end the
+// loop (lanes walk k upwards).  The root find's decisions stay in float64.
+// Phases: a thread per node (growth, chi, root find), a warp per node (the
+// moments), a thread per node (coefficients, Limber weight; exponentials and
+// logarithms by the pair functions, sums in float64: 230 FP64 operations where
+// float64 functions made it 600).
+//   4096 cosmologies x 513 nodes: 52.3 -> 3.5 ms; one cosmology: 241 -> 17 us.
+constexpr int H64_NODES = 64;
+
+// exp(v) and log of positive v by the pair functions, as doubles
+__device__ __forceinline__ double px_expd(double v, const PxTab& T) {
+  return px_join(px_exp2(__double2ll_rn(v * (D_LOG2E * 9007199254740992.0)), T));
+}
+
+// halofit coefficients (power.py:177-244) into a row, as halofit_coefs
+__device__ void halofit_coefs64(double om_m, double om_de, double w, const HfParams& hp, double* row, int model,
+                                const PxTab& T) {
+  const double n = hp.neff, C = hp.C;
+  row[R_KNL] = hp.knl;
+  row[R_NEFF] = n;
+  row[R_C] = C;
+  row[R_OMM] = om_m;
+  row[R_OMDE] = om_de;
+  row[R_W] = w;
+  if (model != JCG_PK_TAKAHASHI2012) {
+    const HfCoef<double> h = hf_coefs<double>(model, n, C, om_m, om_de, w);
+    row[R_AN] = h.an, row[R_BN] = h.bn, row[R_CN] = h.cn, row[R_GAMMAN] = h.gam, row[R_ALPHAN] = h.alpha;
+    row[R_BETAN] = h.beta, row[R_NUN] = h.nu, row[R_MUN] = h.mu, row[R_F1] = h.f1, row[R_F2] = h.f2;
+    row[R_F3] = h.f3, row[R_LGCF3] = h.lcf3;
+    return;
+  }
+  constexpr double L10 = 2.302585092994046;
+  const double dw = om_de * (1.0 + w);
+  const double e_an = 1.5222 + n * (2.8553 + n * (2.3706 + n * (0.9903 + n * 0.2250))) - 0.6038 * C + 0.1749 * dw;
+  const double e_bn = -0.5642 + n * (0.5864 + n * 0.5716) - 1.5474 * C + 0.2279 * dw;
+  const double e_cn = 0.3698 + n * (2.0404 + n * 0.8161) + 0.5869 * C;
+  row[R_AN] = px_expd(L10 * e_an, T);
+  row[R_BN] = px_expd(L10 * e_bn, T);
+  row[R_CN] = px_expd(L10 * e_cn, T);
+  row[R_NUN] = px_expd(L10 * (5.2105 + 3.6902 * n), T);
+  row[R_GAMMAN] = 0.1971 - 0.0843 * n + 0.8460 * C;
+  row[R_ALPHAN] = fabs(6.0835 + n * (1.3373 - n * 0.1959) - 5.5274 * C);
+  row[R_BETAN] = 2.0379 + n * (-0.7354 + n * (0.3157 + n * (1.2490 + n * 0.3980))) - 0.1682 * C;
+  row[R_MUN] = 0.0;
+  // Omega_m^e, e = -0.0307, -0.0585, 0.0743, which scale exponents of P(k):
+  // e^x in float64 by its Taylor polynomial for |x| < 0.25 (Omega_m > 0.035)
+  const double lom = (double)px_log2_d(om_m, T) * (0.69314718055994530942 / 144115188075855872.0);
+  const double ex[3] = {-0.0307 * lom, -0.0585 * lom, 0.0743 * lom};
+  double f[3];
+  const bool small = om_m > 0.035 && om_m < 28.0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double x = ex[q];
+    double p = 1.0 / 479001600.0;
+    p = fma(p, x, 1.0 / 39916800.0);
+    p = fma(p, x, 1.0 / 3628800.0);
+    p = fma(p, x, 1.0 / 362880.0);
+    p = fma(p, x, 1.0 / 40320.0);
+    p = fma(p, x, 1.0 / 5040.0);
+    p = fma(p, x, 1.0 / 720.0);
+    p = fma(p, x, 1.0 / 120.0);
+    p = fma(p, x, 1.0 / 24.0);
+    p = fma(p, x, 1.0 / 6.0);
+    p = fma(p, x, 0.5);
+    p = fma(p, x, 1.0);
+    f[q] = fma(p, x, 1.0);
+  }
+  if (!small) {
+    const double l = log(om_m);
+    f[0] = exp(-0.0307 * l), f[1] = exp(-0.0585 * l), f[2] = exp(0.0743 * l);
+  }
+  row[R_F1] = f[0];
+  row[R_F2] = f[1];
+  row[R_F3] = f[2];
+  row[R_LGCF3] = L10 * e_cn + (small ? ex[2] : log(f[2]));
+}
+
+__global__ void __launch_bounds__(HF_WARPS * 32, 3)
+    halofit_rows64_kernel(Batch bt, const ConstTables* __restrict__ c, int nb) {
+  const int item = blockIdx.y;
+  const Item it = batch_item(bt, item);
+  const GeoHeader* geo = it.geo;
+  const int na = geo->na, n0 = blockIdx.x * nb;
+  if (n0 >= na) return;
+  const int cnt = min(na - n0, nb);
+  const int model = pk_model(it.physics);
+  const CosmoTab* ct = it.ctab;
+  __shared__ __align__(16) PxTab T;
+  __shared__ double sig[NRT], s[NSCAL];
+  __shared__ float2 wpk[NKH], kh2[NKH];
+  __shared__ double knl_s[H64_NODES], inv_s[H64_NODES], lgk_s[H64_NODES], g_s[H64_NODES], chi_s[H64_NODES], s1_s[H64_NODES],
+      s2_s[H64_NODES];
+  __shared__ int wide;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < (int)(sizeof(PxTab) / 16); i += HF_WARPS * 32)
+    reinterpret_cast<uint4*>(&T)[i] = reinterpret_cast<const uint4*>(&c->px)[i];
+  for (int i = tid; i < NRT; i += HF_WARPS * 32) sig[i] = ct->sig[i];
+  for (int i = tid; i < NSCAL; i += HF_WARPS * 32) s[i] = ct->s[i];
+  if (tid == 0) wide = 0;
+  __syncthreads();
+  for (int i = tid; i < NKH; i += HF_WARPS * 32) {
+    const float2 w = ct->rtay[0][i];  // w_i P(k_i) k_i^3 / (2 pi^2), written by the float64 table stage
+    wpk[i] = w;
+    kh2[i] = make_float2(c->kh2_hi[i], c->kh2_lo[i]);
+    if (!(w.x > 1e-28f && w.x < 1e28f)) wide = 1;  // outside what the pairs below hold: float64 terms
+  }
+  const double* A = geo_ptr<double>(geo, geo->off_a);
+  const double* WS = geo_ptr<double>(geo, geo->off_wsimp);
+  const int64_t* SC = geo_ptr<int64_t>(geo, geo->off_seg_chi);
+  const int64_t* SG = geo_ptr<int64_t>(geo, geo->off_seg_grow);
+  // growth, chi and the root find (power.py:96-118)
+  for (int t = tid; t < cnt; t += HF_WARPS * 32) {
+    const int n = n0 + t;
+    const double a = A[n];
+    const int2 sg = unpack_seg(SG[n]);
+    const double sl = (ct->g[sg.y] - ct->g[sg.x]) * c->grow_ida[min(sg.x, sg.y)] * (sg.y > sg.x ? 1.0 : -1.0);
+    const double g = clip_lohi(ct->g[sg.x] + sl * (a - c->atab_grow[sg.x]), 0.0, 1.0);
+    const double g2 = g * g;
+    int ind, j2;
+    root_segment(sig, g2, ind, j2);
+    const double xp = sig[ind] * g2;
+    double root = c->logr[ind] + (c->logr[j2] - c->logr[ind]) / (sig[j2] * g2 - xp) * (1.0 - xp);
+    double R = exp(root);
+    if (!(R >= 1e-6)) R = R < 1e-6 ? 1e-6 : R, root = log(R);  // power.py:113-115
+    g_s[t] = g;
+    inv_s[t] = R;
+    knl_s[t] = 1.0 / R;
+    lgk_s[t] = -root;
+    chi_s[t] = chi_at(ct, c, a, unpack_seg(SC[n]));
+    if (!(R < 1e6)) wide = 1;
+  }
+  __syncthreads();
+  // the moments
+  if (model != JCG_PK_LINEAR) {
+    for (int t = warp; t < cnt; t += HF_WARPS) {
+      double s1, s2;
+      const double R = inv_s[t];
+      if (!wide) {
+        const FF R2 = px_split(R * R);
+        FF a1{0.f, 0.f}, a2{0.f, 0.f};  // at most 9 terms per lane
+        for (int i = lane; i < NKH; i += 32) {
+          const FF y2 = px_mul(R2, px_f2(kh2[i]));
+          if (y2.hi > 60.f) break;
+          const FF e = px_exp2(-px_fix53(px_mul(y2, pxc(D_LOG2E))), T);
+          const FF r = px_mul(px_mul(px_f2(wpk[i]), e), y2);
+          a1 = px_add(a1, r);
+          a2 = px_add(a2, px_mul(r, px_1p(FF{-y2.hi, -y2.lo})));
+        }
+        __syncwarp();
+        s1 = 2.0 * warp_sum(px_join(a1));
+        s2 = 4.0 * warp_sum(px_join(a2));
+      } else {
+        s1 = s2 = 0.0;
+        for (int i = lane; i < NKH; i += 32) {
+          const double y = c->kh[i] * R, y2 = y * y;
+          const double r = ct->pk3[i] * exp(-y2) / TWO_PI2;
+          s1 += c->simpson_kh[i] * (2 * r * y2);
+          s2 += c->simpson_kh[i] * (4 * r * (y2 - y2 * y2));
+        }
+        s1 = warp_sum(s1);
+        s2 = warp_sum(s2);
+      }
+      if (lane == 0) s1_s[t] = s1, s2_s[t] = s2;
+    }
+  }
+  __syncthreads();
+  // coefficients and the Limber weight
+  for (int t = tid; t < cnt; t += HF_WARPS * 32) {
+    const int n = n0 + t;
+    const double a = A[n], g2 = g_s[t] * g_s[t];
+    double row[NROW64];
+    for (int i = 0; i < NROW64; ++i) row[i] = 0.0;
+    // background (background.py:122-126, 168, 196, 270-294)
+    const double ia = px_ddiv(1.0, a, px_rcp(px_hi(a)));
+    const double lna = (double)px_log2_d(a, T) * (0.69314718055994530942 / 144115188075855872.0);
+    const double fde = -3.0 * (1.0 + s[S_W0] + s[S_WA]) * lna + 3.0 * s[S_WA] * (a - 1.0);
+    const double ef = fde == 0.0 ? 1.0 : exp(fde);
+    const double ia2 = ia * ia, om3 = s[S_OMEGA_M] * (ia2 * ia), ode = s[S_OMEGA_DE] * ef;
+    const double e2 = om3 + s[S_OMEGA_K] * ia2 + ode;
+    const double ie2 = 1.0 / e2;
+    const double chi = chi_s[t], dchi = RH * ia2 * rsqrt(e2);
+    HfParams hp;
+    hp.knl = knl_s[t];
+    const double s1 = model == JCG_PK_LINEAR ? 0.0 : s1_s[t] * g2;
+    hp.neff = s1 - 3.0;  // power.py:138-139
+    hp.C = model == JCG_PK_LINEAR ? 0.0 : s1 * s1 + s2_s[t] * g2;
+    halofit_coefs64(om3 * ie2, ode * ie2, s[S_W0] + (1.0 - a) * s[S_WA], hp, row, model, T);
+    row[R_CHI] = chi;
+    row[R_G] = g_s[t];
+    row[R_LGKNL] = lgk_s[t];
+    row[R_LGCHIC] = log(fmax(chi, 1.0));
+    row[R_DCHI] = dchi;
+    row[R_U] = WS[n] * dchi / fmax(chi * chi, 1.0) * (1.0 / C2);
+    double* dst = it.rows64 + (size_t)n * NROW64;
+    for (int i = 0; i < NROW64; ++i) dst[i] = row[i];
+  }
+}
+
 void launch_halofit_rows(const Batch& b, const ConstTables* c, cudaStream_t st) {
-  const int nb = hf_nodes_per_block(b.precision == JCG_FP32C);
-  dim3 grid((b.max_na + nb - 1) / nb, b.n_items);
-  if (hf_flat(b)) grid = dim3((unsigned)(((long long)b.n_items * b.max_na + nb - 1) / nb), 1);
-  if (b.precision == JCG_FP32C)
-    halofit_rows_kernel<true><<<grid, HF_WARPS * 32, 0, st>>>(b, c);
-  else
-    halofit_rows_kernel<false><<<grid, HF_WARPS * 32, 0, st>>>(b, c);
+  if (b.precision == JCG_FP32C) {
+    dim3 grid((b.max_na + HF_NODES - 1) / HF_NODES, b.n_items);
+    if (hf_flat(b)) grid = dim3((unsigned)(((long long)b.n_items * b.max_na + HF_NODES - 1) / HF_NODES), 1);
+    halofit_rows_kernel<<<grid, HF_WARPS * 32, 0, st>>>(b, c);
+    return;
+  }
+  // few CTAs: fewer nodes each, so that the batch spreads over the SMs
+  int nb = H64_NODES;
+  while (nb > 8 && (long long)b.n_items * ((b.max_na + nb - 1) / nb) < 2 * device_sm_count()) nb >>= 1;
+  halofit_rows64_kernel<<<dim3((b.max_na + nb - 1) / nb, b.n_items), HF_WARPS * 32, 0, st>>>(b, c, nb);
 }
 
 // ------------------------------------------------------ pointwise queries ---

@@ -155,7 +155,8 @@ struct CosmoTab {
   float wpk3f[NKH + 15];   // simpson_kh[i] * pk3[i], float (fp32c halofit moments); padded to 64 bytes
   // fp32c: the small-y part of the halofit moments as a Taylor series in y^2.
   // Float pairs R_m[i] = c_m Q_m[i], c_m = (-1)^m / m!,
-  // Q_m[i] = sum_{k < i} w_k P(k_k) k_k^3 (k_k / k_i)^(2(m+1)), m < NTAYLOR
+  // Q_m[i] = sum_{k < i} w_k P(k_k) k_k^3 (k_k / k_i)^(2(m+1)), m < NTAYLOR.
+  // float64 tables: rtay[0][i] = w_i P(k_i) k_i^3 / (2 pi^2) as a pair
   float2 rtay[NTAYLOR][NKH + 1];
   EH32 eh32;               // fp32c Limber integrand's transfer inputs (from s)
   double pad[PAD_CT];
@@ -822,6 +823,7 @@ __device__ __forceinline__ void ku_get_rec(const float4* rec, int& q, float& dx,
 }
 
 void launch_tracer_kernels(const Batch& b, const ConstTables* c, cudaStream_t st);
+void launch_tracer64(const Batch& b, const ConstTables* c, cudaStream_t st);
 void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st);
 void launch_limber64(const Batch& b, const ConstTables* c, cudaStream_t st);
 // derivatives (jcg_grad.cu)

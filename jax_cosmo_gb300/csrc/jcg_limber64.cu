@@ -286,9 +286,9 @@ __global__ void __launch_bounds__(PX_THREADS, 2)
     __syncthreads();
     for (int u = tid; u < units; u += PX_THREADS) {
       const int pg = u / lt, l = u - pg * lt;
-      float hs[4], ls[4], xs[4];
+      F3 sum[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) hs[j] = ls[j] = xs[j] = 0.f;
+      for (int j = 0; j < 4; ++j) sum[j] = F3{0.f, 0.f, 0.f};
       for (int t0 = 0; t0 < nb; t0 += PX_RUN) {
         float ah[4], al[4];
 #pragma unroll
@@ -304,23 +304,13 @@ __global__ void __launch_bounds__(PX_THREADS, 2)
           ff_acc_prod(ah[3], al[3], P, make_float2(m23.z, m23.w));
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // three-float total: the roundings of the high and of the middle part
-          // are carried on
-          const FF a = px_norm(ah[j], al[j]);
-          const FF w = px_two_sum(hs[j], a.hi);
-          const FF m = px_two_sum(ls[j], w.lo);
-          const FF n = px_two_sum(m.hi, a.lo);
-          hs[j] = w.hi;
-          ls[j] = n.hi;
-          xs[j] += m.lo + n.lo;
-        }
+        for (int j = 0; j < 4; ++j) px_acc3(sum[j], px_norm(ah[j], al[j]));
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int p = pg * 4 + j;
         const int sh = esc[p] - 1023, h = sh >> 1;
-        const double part = (((double)xs[j] + (double)ls[j]) + (double)hs[j]) * __hiloint2double((1023 + h) << 20, 0) *
+        const double part = px_d3(sum[j]) * __hiloint2double((1023 + h) << 20, 0) *
                             __hiloint2double((1023 + sh - h) << 20, 0);
         double* w = dst + (size_t)l * ncp + p;
         *w = first ? part : *w + part;

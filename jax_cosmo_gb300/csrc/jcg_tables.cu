@@ -549,7 +549,10 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   // with the Simpson weights and 1 / (2 pi^2) folded into the k-node factor:
   // one FMA per (k, R) term
   if (!FAST) {
-    for (int i = t; i < NKH; i += blockDim.x) pq[i] = c->simpson_kh[i] * (pk3[i] / (2.0 * (PI * PI)));
+    for (int i = t; i < NKH; i += blockDim.x) {
+      pq[i] = c->simpson_kh[i] * (pk3[i] / (2.0 * (PI * PI)));
+      it.ctab->rtay[0][i] = f2_of(pq[i]);  // as a pair, for the moments of the float64 rows
+    }
     __syncthreads();
   }
   CosmoTab* out = it.ctab;
