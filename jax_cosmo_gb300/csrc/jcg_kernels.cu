@@ -11,9 +11,9 @@
 // NumberCounts (probes.py:77-99, 260-272): n_i(z) * b * H(z2a(z)).
 // The ell factor of WeakLensing (probes.py:73) is applied in the Limber stage.
 //
-// FP64 (plain): float64 throughout.  FP32 (fp32c): the lensing integrand in
-// float32 (chi' from the float table, reciprocal by MUFU), the result scaled
-// in float64.
+// This file holds the fp32c form: the lensing integrand in float32 (chi' from
+// the float table, reciprocal by MUFU), the result scaled in float64.  The plain
+// method's kernels are in jcg_tracer64.cu.
 #include "jcg_internal.cuh"
 
 namespace jcg {
@@ -27,10 +27,9 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-template <bool FP32>
 __global__ void __launch_bounds__(TK_WARPS * 32)
     tracer_kernels_kernel(Batch bt, const ConstTables* __restrict__ c) {
-  using T = typename std::conditional<FP32, float, double>::type;
+  using T = float;
   const int item = blockIdx.y;
   if (item >= bt.n_items) return;
   const Item it = batch_item(bt, item);
@@ -40,18 +39,11 @@ __global__ void __launch_bounds__(TK_WARPS * 32)
   if (n0 >= na) return;
   __shared__ T chi[NCHI];
   __shared__ T slope[NCHI];
-  __shared__ double atab[NCHI];
   __shared__ double s[NSCAL];
   const CosmoTab* ct = it.ctab;
   for (int i = threadIdx.x; i < NCHI; i += blockDim.x) {
-    if (FP32) {
-      chi[i] = (T)ct->chi32[i];
-      slope[i] = (T)ct->slope32[i];
-    } else {
-      chi[i] = (T)ct->chi[i];
-      slope[i] = (T)ct->chi_slope[i];
-    }
-    atab[i] = c->atab_chi[i];
+    chi[i] = (T)ct->chi32[i];
+    slope[i] = (T)ct->slope32[i];
   }
   for (int i = threadIdx.x; i < NSCAL; i += blockDim.x) s[i] = ct->s[i];
   __syncthreads();
@@ -59,7 +51,6 @@ __global__ void __launch_bounds__(TK_WARPS * 32)
   const int n_tr = geo->n_tr;
   const double* Z = geo_ptr<double>(geo, geo->off_z);
   const double* AWL = geo_ptr<double>(geo, geo->off_awl);
-  const int64_t* SW = geo_ptr<int64_t>(geo, geo->off_seg_chiwl);
   const int32_t* QWL = geo_ptr<int32_t>(geo, geo->off_qwl32);
   const float* DXWL = geo_ptr<float>(geo, geo->off_dxwl32);
   const double* NZL = geo_ptr<double>(geo, geo->off_nzl);
@@ -68,45 +59,24 @@ __global__ void __launch_bounds__(TK_WARPS * 32)
   const int n_end = min(na, n0 + TK_NODES_PER_BLOCK);
   for (int n = n0 + warp; n < n_end; n += TK_WARPS) {
     const double awl = AWL[n];
-    T chi_wl;
-    if (FP32) {
-      const int q = QWL[n];
-      chi_wl = fmaxf((float)chi[q & 0xffff] + (float)slope[q >> 16] * DXWL[n], 0.f);
-    } else {
-      const int2 sg = unpack_seg(SW[n]);
-      chi_wl = fmax((double)chi[sg.x] + (double)slope[min(sg.x, sg.y)] * (awl - atab[sg.x]), 0.0);
-    }
+    const int qw = QWL[n];
+    const T chi_wl = fmaxf((float)chi[qw & 0xffff] + (float)slope[qw >> 16] * DXWL[n], 0.f);
     T acc[MAXTR];
 #pragma unroll
     for (int t = 0; t < MAXTR; ++t) acc[t] = 0;
     for (int g = 0; g < geo->n_groups; ++g) {
       const size_t row = (size_t)n * NZP;
-      const double* AP = geo_ptr<double>(geo, geo->off_ap[g]) + row;
-      const int64_t* SP = geo_ptr<int64_t>(geo, geo->off_segp[g]) + row;
       const int32_t* Q32 = geo_ptr<int32_t>(geo, geo->off_q32[g]) + row;
       const float* DX32 = geo_ptr<float>(geo, geo->off_dx32[g]) + row;
       for (int j = lane; j < NZP; j += 32) {
-        T ratio;
-        if (FP32) {
-          const int q = Q32[j];
-          const float chip = fmaxf((float)chi[q & 0xffff] + (float)slope[q >> 16] * DX32[j], 0.f);
-          ratio = fmaxf(chip - (float)chi_wl, 0.f) * rcp_approx(fmaxf(chip, 1.f));
-        } else {
-          const int2 sg = unpack_seg(SP[j]);
-          const double chip =
-              fmax((double)chi[sg.x] + (double)slope[min(sg.x, sg.y)] * (AP[j] - atab[sg.x]), 0.0);
-          ratio = fmax(chip - (double)chi_wl, 0.0) / fmax(chip, 1.0);
-        }
+        const int q = Q32[j];
+        const float chip = fmaxf((float)chi[q & 0xffff] + (float)slope[q >> 16] * DX32[j], 0.f);
+        const T ratio = fmaxf(chip - (float)chi_wl, 0.f) * rcp_approx(fmaxf(chip, 1.f));
 #pragma unroll
         for (int t = 0; t < MAXTR; ++t) {
           if (t < n_tr && geo->kind[t] == JCG_TRACER_WL && geo->group[t] == g) {
-            if (FP32) {
-              const float* W = geo_ptr<float>(geo, geo->off_W32[t]) + row;
-              acc[t] += (T)W[j] * ratio;
-            } else {
-              const double* W = geo_ptr<double>(geo, geo->off_W[t]) + row;
-              acc[t] += (T)W[j] * ratio;
-            }
+            const float* W = geo_ptr<float>(geo, geo->off_W32[t]) + row;
+            acc[t] += (T)W[j] * ratio;
           }
         }
       }
@@ -301,7 +271,11 @@ static void launch_tu(const Batch& b, const ConstTables* c, cudaStream_t st) {
 }
 
 void launch_tracer_kernels(const Batch& b, const ConstTables* c, cudaStream_t st) {
-  if (b.precision == JCG_FP32C && !b.listed && !b.special_bias && !b.has_delta && b.n_wl_groups == 1 && b.n_wl >= 1 &&
+  if (b.precision != JCG_FP32C) {
+    launch_tracer64(b, c, st);
+    return;
+  }
+  if (!b.listed && !b.special_bias && !b.has_delta && b.n_wl_groups == 1 && b.n_wl >= 1 &&
       b.n_wl <= 8) {
     switch (b.n_wl) {
       case 1: launch_tu<1>(b, c, st); return;
@@ -315,10 +289,7 @@ void launch_tracer_kernels(const Batch& b, const ConstTables* c, cudaStream_t st
     }
   }
   dim3 grid((b.max_na + TK_NODES_PER_BLOCK - 1) / TK_NODES_PER_BLOCK, b.n_items);
-  if (b.precision == JCG_FP32C)
-    tracer_kernels_kernel<true><<<grid, TK_WARPS * 32, 0, st>>>(b, c);
-  else
-    tracer_kernels_kernel<false><<<grid, TK_WARPS * 32, 0, st>>>(b, c);
+  tracer_kernels_kernel<<<grid, TK_WARPS * 32, 0, st>>>(b, c);
 }
 
 }  // namespace jcg
