@@ -26,13 +26,11 @@ namespace jcg {
 // value as a float pair, 8 FP32 tangents: the fp32c table stages (jcg_dualff.cuh)
 typedef DualFF<NDIR> FF8;
 
-// Tables of one cosmology with tangents.  Lanes: dir = tid & 7, item = tid >> 3.
-// F32T (fp32c Jacobian): the per-node evaluations (ODE right-hand sides,
-// Eisenstein-Hu at the Romberg and halofit k nodes) run one node per thread in
-// DualF<8> -- value in FP64, tangents in FP32 -- instead of one direction per
-// lane; the sigma^2(R) tangents are FP32 sums; float copies of the chi and
-// P(k) k^3 tangent tables are written for the FP32 stages.  The sequential
-// scans (chi prefix sum, growth RK4, Romberg) stay FP64 Dual<1>.
+// fp32c tables of one cosmology with tangents (the float64 form: jcg_grad64.cu).
+// The per-node evaluations (ODE right-hand sides, Eisenstein-Hu at the Romberg
+// and halofit k nodes) run one node per thread in grad_nodes_kernel; the
+// sigma^2(R) tangents are FP32 sums; float copies of the chi and P(k) k^3
+// tangent tables are written for the FP32 stages.
 // fp32c node arrays, packed: [n] float-pair values (float2), then
 // [NDIR][n] float tangents (5 n doubles of storage); written by
 // grad_nodes_kernel, read by grad_tables_kernel, no float64 conversion on
@@ -98,23 +96,19 @@ __device__ __forceinline__ void chi_scan_ff(const double* fnode, const double* f
   for (int k = 0; k < 8; ++k) v[k] = tot - (off + loc[k]);
 }
 
-// NW: some item may use the transfer type "eisenhu"
-template <bool F32T, bool NW>
-__global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+__global__ void __launch_bounds__(128, 4) grad_tables_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
   const int item = blockIdx.x;
   if (item >= gb.n_items) return;
   extern __shared__ __align__(16) double sm[];
   double* sv = sm;                      // NSCAL
   double* sd = sv + NSCAL;              // [NDIR][NSCAL]
-  // FP64: [NDIR+1][n] doubles per array; fp32c: the packed layout of
-  // grad_nodes_kernel (GNODE_* offsets)
-  double* fn = sd + NDIR * NSCAL;       // f at the chi nodes
-  double* fm = fn + (F32T ? GNODE_FM : (NDIR + 1) * NCHI);  // f at the chi midpoints
-  double* qr = fn + (F32T ? GNODE_QR : 2 * (NDIR + 1) * NCHI);  // qa, ra, qm, rm
-  double* fr = fn + (F32T ? GNODE_FR : 2 * (NDIR + 1) * NCHI + 4 * (NDIR + 1) * NGROW);  // Romberg integrand
-  double* g1s = F32T ? fn + GNODE_U : fr + (NDIR + 1) * NROMB;  // [NDIR+1]
-  double* pq = qr;                            // FP64: [NDIR+1][NKH], after the growth RK4
-  const int t = threadIdx.x, dir = t & 7, it = t >> 3;
+  // the packed layout of grad_nodes_kernel (GNODE_* offsets)
+  double* fn = sd + NDIR * NSCAL;  // f at the chi nodes
+  double* fm = fn + GNODE_FM;      // f at the chi midpoints
+  double* qr = fn + GNODE_QR;      // qa, ra, qm, rm
+  double* fr = fn + GNODE_FR;      // Romberg integrand
+  double* g1s = fn + GNODE_U;      // [NDIR+1]
+  const int t = threadIdx.x, dir = t & 7;
   const GradItem gi = grad_item(gb, item);
   TabD* out = gi.tab;
   // the chi and growth tables go straight to the output (read back after a barrier)
@@ -122,56 +116,7 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
   for (int i = t; i < NSCAL; i += blockDim.x) sv[i] = out->sv[i];
   for (int i = t; i < NDIR * NSCAL; i += blockDim.x) sd[i] = out->sd[i / NSCAL][i % NSCAL];
   __syncthreads();
-  D1 sD[NSCAL];
-  for (int i = 0; i < NSCAL; ++i) sD[i] = mk1(sv[i], sd[dir * NSCAL + i]);
-  const BgT<D1> bg = make_bgT(sD);
-  auto put = [&](double* arr, int stride, int e, const D1& x) {
-    if (dir == 0) arr[e] = x.v;
-    arr[(1 + dir) * stride + e] = x.d[0];
-  };
-  auto putf = [&](double* arr, int stride, int e, const auto& x) {
-    arr[e] = val(x);
-#pragma unroll
-    for (int d = 0; d < NDIR; ++d) arr[(1 + d) * stride + e] = x.d[d];
-  };
-  if (!F32T) {
-    // chi RK4 right-hand side at nodes and midpoints (background.py:227-231)
-    for (int e = it; e < 2 * NCHI; e += 32) {
-      if (e < NCHI) {
-        put(fn, NCHI, e, dchi_dlnaT(bg, c->lna_chi[e]));
-      } else if (e > NCHI) {
-        const int i = e - NCHI;
-        const double t0 = c->lna_chi[i - 1], t1 = c->lna_chi[i];
-        put(fm, NCHI, i, dchi_dlnaT(bg, t0 + (t1 - t0) / 2));
-      }
-    }
-    // growth ODE coefficients (background.py:96-106)
-    for (int e = it; e < 2 * NGROW; e += 32) {
-      D1 q, r;
-      if (e < NGROW) {
-        growth_qrT(bg, c->atab_grow[e], q, r);
-        put(qr + 0 * (NDIR + 1) * NGROW, NGROW, e, q);
-        put(qr + 1 * (NDIR + 1) * NGROW, NGROW, e, r);
-      } else if (e > NGROW) {
-        const int i = e - NGROW;
-        const double x = c->atab_grow[i], xp = c->atab_grow[i - 1];
-        growth_qrT(bg, xp + (x - xp) / 2, q, r);
-        put(qr + 2 * (NDIR + 1) * NGROW, NGROW, i, q);
-        put(qr + 3 * (NDIR + 1) * NGROW, NGROW, i, r);
-      }
-    }
-    // sigmasqr(8) integrand at the romb nodes (power.py:70-75)
-    for (int e = it; e < NROMB; e += 32) {
-      const double logk = c->romb_logk[e];
-      const double k = exp(logk);
-      const double x = k * 8.0;
-      const double wf = 3.0 * (sin(x) - x * cos(x)) / (x * x * x);
-      const D1 T = eh_transferT<NW>(sD, k, logk);
-      const D1 pk = (T * T) * xexp(sD[S_NS] * logk);
-      const double kw = k * wf;
-      put(fr, NROMB, e, k * (kw * kw) * pk);
-    }
-  } else {
+  {
     // node values from grad_nodes_kernel: the same packed layout as fn .. fr here;
     // 16-byte copies, eight in flight per thread
     static_assert((9 * NSCAL) % 2 == 0 && GNODE_STRIDE % 2 == 0, "16-byte aligned node copy");
@@ -195,8 +140,8 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
   }
   __syncthreads();
   const int warp = t >> 5, lane = t & 31;
-  if (F32T) {
-    // fp32c: the three sequential scans as parallel scans (128 threads).
+  {
+    // the three sequential scans as parallel scans (128 threads).
     // Growth: one RK4 step is linear in y = (D, dD/da), y_i = M_i y_{i-1};
     // thread i forms M_i (FP64) and its tangents dM_i (FP32) by running the
     // step on the unit vectors in DualF<8>.
@@ -347,91 +292,9 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
         out->gdF[i][d] = gdv;  // the row stage's copy
       }
     }
-  } else if (lane < NDIR) {
-    const int d = lane;
-    auto gv = [&](const double* arr, int stride, int e) { return mk1(arr[e], arr[(1 + d) * stride + e]); };
-    if (warp == 0) {
-      // chi prefix sum (scipy/ode.py:21 first step h = 0), then chi[-1] - chi
-      D1 y = mk1(0.0, 0.0);
-      D1 ys[NCHI];
-      ys[0] = y;
-      for (int i = 1; i < NCHI; ++i) {
-        const double hh = c->lna_chi[i] - c->lna_chi[i - 1];
-        const D1 fmv = gv(fm, NCHI, i);
-        y = y + 1.0 / 6.0 * hh * (gv(fn, NCHI, i - 1) + 2 * fmv + 2 * fmv + gv(fn, NCHI, i));
-        ys[i] = y;
-      }
-      for (int i = 0; i < NCHI; ++i) {
-        const D1 v = ys[NCHI - 1] - ys[i];
-        if (d == 0) out->chiv[i] = v.v;
-        out->chid[d][i] = v.d[0];
-      }
-    } else if (warp == 1) {
-      // growth RK4 in a (background.py:108-111)
-      const double* QA = qr;
-      const double* RA = qr + (NDIR + 1) * NGROW;
-      const double* QM = qr + 2 * (NDIR + 1) * NGROW;
-      const double* RM = qr + 3 * (NDIR + 1) * NGROW;
-      D1 y0 = mk1(c->atab_grow[0], 0.0), y1 = mk1(1.0, 0.0);
-      D1 ys[NGROW];
-      ys[0] = y0;
-      for (int i = 1; i < NGROW; ++i) {
-        const double hh = c->atab_grow[i] - c->atab_grow[i - 1];
-        const D1 qa0 = gv(QA, NGROW, i - 1), ra0 = gv(RA, NGROW, i - 1);
-        const D1 qm = gv(QM, NGROW, i), rm = gv(RM, NGROW, i);
-        const D1 qa1 = gv(QA, NGROW, i), ra1 = gv(RA, NGROW, i);
-        const D1 k1a = y1, k1b = -qa0 * y1 + ra0 * y0;
-        const D1 y0b = y0 + hh * k1a / 2, y1b = y1 + hh * k1b / 2;
-        const D1 k2a = y1b, k2b = -qm * y1b + rm * y0b;
-        const D1 y0c = y0 + hh * k2a / 2, y1c = y1 + hh * k2b / 2;
-        const D1 k3a = y1c, k3b = -qm * y1c + rm * y0c;
-        const D1 y0d = y0 + hh * k3a, y1d = y1 + hh * k3b;
-        const D1 k4a = y1d, k4b = -qa1 * y1d + ra1 * y0d;
-        y0 = y0 + 1.0 / 6.0 * hh * (k1a + 2 * k2a + 2 * k3a + k4a);
-        y1 = y1 + 1.0 / 6.0 * hh * (k1b + 2 * k2b + 2 * k3b + k4b);
-        ys[i] = y0;
-      }
-      for (int i = 0; i < NGROW; ++i) {
-        const D1 v = ys[i] / y0;
-        if (d == 0) out->gv[i] = v.v;
-        out->gd[d][i] = v.d[0];
-      }
-    } else if (warp == 2) {
-      // romb combination (scipy/integrate.py:131-159), divmax = 7
-      const double a = -4.0, b = 3.0, intrange = b - a;
-      D1 ordsum = 0.5 * (gv(fr, NROMB, 0) + gv(fr, NROMB, 1));
-      D1 state[8];
-      for (int i = 0; i < 8; ++i) state[i] = intrange * ordsum;
-      int pos = 2;
-      for (int lev = 1; lev <= 7; ++lev) {
-        const int n = 1 << lev, numtosum = n / 2;
-        D1 sum = mk1(0.0, 0.0);
-        for (int m = 0; m < numtosum; ++m) sum = sum + gv(fr, NROMB, pos + m);
-        pos += numtosum;
-        ordsum = ordsum + sum;
-        D1 x = intrange * ordsum / (double)n;
-        D1 ns[8];
-        ns[0] = x;
-        for (int kk = 0; kk < 7; ++kk) {
-          const double tmp = ldexp(1.0, 2 * (kk + 1));
-          x = (tmp * x - state[kk]) / (tmp - 1.0);
-          ns[kk + 1] = x;
-        }
-        for (int i = 0; i < 8; ++i) state[i] = ns[i];
-      }
-      const D1 sig8 = 1.0 / (2.0 * (PI * PI)) * state[7];
-      const D1 s8 = mk1(sv[S_SIGMA8], sd[d * NSCAL + S_SIGMA8]);
-      const D1 pkn = (s8 * s8) / sig8;
-      if (d == 0) {
-        sv[S_SIGMASQR8] = sig8.v;
-        sv[S_PKNORM] = pkn.v;
-      }
-      sd[d * NSCAL + S_SIGMASQR8] = sig8.d[0];
-      sd[d * NSCAL + S_PKNORM] = pkn.d[0];
-    }
   }
   __syncthreads();
-  if (F32T && t < NDIR) {
+  if (t < NDIR) {
     // P(k) normalisation sigma8^2 / sigmasqr(8) (power.py:47)
     const D1 s8 = mk1(sv[S_SIGMA8], sd[dir * NSCAL + S_SIGMA8]);
     const D1 pkn = (s8 * s8) / mk1(sv[S_SIGMASQR8], sd[dir * NSCAL + S_SIGMASQR8]);
@@ -448,18 +311,8 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
     g1s[1 + dir] = g1.d[0];
   }
   __syncthreads();
-  for (int i = 0; i < NSCAL; ++i) sD[i] = mk1(sv[i], sd[dir * NSCAL + i]);
-  const D1 g1 = mk1(g1s[0], g1s[1 + dir]);
-  // P(k_i, a = 1) k_i^3 and pk3 / (2 pi^2) on the halofit grid
-  if (!F32T) {
-    for (int e = it; e < NKH; e += 32) {
-      const double k = c->kh[e];
-      const D1 p3 = pk_linearT<NW>(sD, k, c->logk[e], g1) * c->kh3[e];
-      if (dir == 0) out->pk3v[e] = p3.v;
-      out->pk3d[dir][e] = p3.d[0];
-      put(pq, NKH, e, p3 / (2.0 * (PI * PI)));
-    }
-  } else {
+  // P(k_i, a = 1) k_i^3 on the halofit grid
+  {
     // the node values exp(n_s ln k) T(k)^2 from grad_nodes_kernel, in
     // pk_linearT's order: ((u g^2) pknorm), then k^3
     const FF8 g1f = ff8_of(g1s[0], g1s + 1, 1);
@@ -475,7 +328,7 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
       pd[1] = make_float4(p3.d[4], p3.d[5], p3.d[6], p3.d[7]);
     }
   }
-  if (F32T && t < NDIR + 1) {
+  if (t < NDIR + 1) {
     // the Limber kernels' FP32 Eisenstein-Hu inputs and their tangents,
     // once per cosmology: t 0 the values, t 1..8 direction t - 1
     const int d = t - 1;
@@ -523,25 +376,11 @@ __global__ void __launch_bounds__(F32T ? 128 : 256, F32T ? 4 : 1) grad_tables_ke
   }
   __syncthreads();
   // fp32c: the Taylor tables and sigma^2(R) follow in grad_moments32_kernel
-  const double dx = (c->logk[NKH - 1] - c->logk[0]) / 256;
-  for (int e = F32T ? (NDIR + 1) * NRT : t; e < (NDIR + 1) * NRT; e += blockDim.x) {
-    const int comp = e / NRT, j = e % NRT;
-    const double* w = pq + comp * NKH;
-    double acc = 0.0;
-    for (int m = 0; m < 128; ++m) {
-      const double y0 = w[2 * m] * c->E[(2 * m) * NRT + j];
-      const double y1 = w[2 * m + 1] * c->E[(2 * m + 1) * NRT + j];
-      const double y2 = w[2 * m + 2] * c->E[(2 * m + 2) * NRT + j];
-      acc += y0 + 4 * y1 + y2;
-    }
-    if (comp == 0) out->sigv[j] = dx / 3 * acc;
-    else out->sigd[comp - 1][j] = dx / 3 * acc;
-  }
   for (int i = t; i < NSCAL; i += blockDim.x) {
     out->sv[i] = sv[i];
     for (int d = 0; d < NDIR; ++d) out->sd[d][i] = sd[d * NSCAL + i];
   }
-  if (F32T) {
+  {
     // float-pair copies for the row stage
     for (int i = t; i < NSCAL; i += blockDim.x) {
       const FF v = ff_of(sv[i]);
@@ -650,11 +489,7 @@ __global__ void __launch_bounds__(NRT) grad_moments32_kernel(GradBatch gb, const
   }
 }
 
-size_t grad_tables_smem(bool f32t) {
-  static_assert(4 * NGROW >= NKH, "P(k) k^3 staging aliases the growth coefficients");
-  if (f32t) return sizeof(double) * (NSCAL * (1 + NDIR) + GNODE_U + NDIR + 1);
-  return sizeof(double) * (NSCAL * (1 + NDIR) + (NDIR + 1) * (2 * NCHI + 4 * NGROW + NROMB + 1));
-}
+size_t grad_tables_smem() { return sizeof(double) * (NSCAL * (1 + NDIR) + GNODE_U + NDIR + 1); }
 
 // ----------------------------------------------------------- dual rows -----
 // FP64 Jacobian rows.  One warp per 4 Limber nodes: lane = 8 * node slot +
@@ -2001,7 +1836,6 @@ __global__ void __launch_bounds__(32 * NDIR) grad_growth_gamma_kernel(GradBatch 
 }
 
 void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t st, unsigned stages) {
-  const size_t smt = grad_tables_smem(gb.precision == JCG_FP32C);
   if (stages & GS_TABLES) {
   if (gb.n_items <= GNODE_MAX_ITEMS)
     grad_scalars_warp_kernel<<<gb.n_items, 16 * NDIR, 0, st>>>(gb);
@@ -2015,20 +1849,13 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
     grad_nodes_kernel<2><<<dim3((NROMB + NKH + 127) / 128, gb.n_items), 128, 0, st>>>(gb, c);
   }
   if (gb.precision == JCG_FP32C) {
-    if (tf_nowiggle(gb.physics_or)) {
-      cudaFuncSetAttribute(grad_tables_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
-      cudaFuncSetAttribute(grad_tables_kernel<true, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared);  // four CTAs per SM
-      grad_tables_kernel<true, true><<<gb.n_items, 128, smt, st>>>(gb, c);
-    } else {
-      cudaFuncSetAttribute(grad_tables_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
-      cudaFuncSetAttribute(grad_tables_kernel<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared);  // four CTAs per SM
-      grad_tables_kernel<true, false><<<gb.n_items, 128, smt, st>>>(gb, c);
-    }
+    const size_t smt = grad_tables_smem();
+    cudaFuncSetAttribute(grad_tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
+    cudaFuncSetAttribute(grad_tables_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         (int)cudaSharedmemCarveoutMaxShared);  // four CTAs per SM
+    grad_tables_kernel<<<gb.n_items, 128, smt, st>>>(gb, c);
   } else {
-    cudaFuncSetAttribute(grad_tables_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
-    grad_tables_kernel<false, true><<<gb.n_items, 256, smt, st>>>(gb, c);
+    launch_grad_tables64(gb, c, st);
   }
   if (gb.precision == JCG_FP32C) grad_moments32_kernel<<<gb.n_items, NRT, 0, st>>>(gb, c);
   if (growth_gamma(gb.physics_or)) grad_growth_gamma_kernel<<<gb.n_items, 32 * NDIR, 0, st>>>(gb, c);

@@ -290,6 +290,8 @@ static __device__ __noinline__ void bias_term_d1(const TabD* tb, const ConstTabl
 // the product kernel, the reverse lensing kernel with the gradient sum
 enum GradStage : unsigned { GS_TABLES = 1, GS_ROWS = 2, GS_KERNELS = 4, GS_PRODUCT = 8, GS_REVERSE = 16, GS_ALL = 31 };
 
+// FP64 tables with tangents (jcg_grad64.cu)
+void launch_grad_tables64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 // FP32 compensated stages (jcg_grad32.cu)
 void launch_grad_kern32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 void launch_grad_limber32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
