@@ -504,10 +504,11 @@ size_t grad_tables_smem() { return sizeof(double) * (NSCAL * (1 + NDIR) + GNODE_
 //     every term with y^2 <= 60 (the rest is below 1e-20 of the sums);
 //   epilogue (per lane, Dual<1>): n_eff, C, takahashi2012 coefficients, the
 //     Limber weight; rows out.
-__global__ void __launch_bounds__(256) grad_rows_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+__global__ void __launch_bounds__(256) grad_rows_kernel(GradBatch gb, const ConstTables* __restrict__ c, int only_wide) {
   const int item = blockIdx.y;
   if (item >= gb.n_items) return;
   const GradItem gi = grad_item(gb, item);
+  if (only_wide && !gi.tab->wide) return;
   const GeoHeader* geo = gi.geo;
   const int na = geo->na;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1138,10 +1139,11 @@ __global__ void __launch_bounds__(GR32_THREADS, 2) grad_rows32_kernel(GradBatch 
 // ------------------------------------------------------ dual radial kernels -
 // One warp per node: chi_wl and H on lanes 0-7, the lensing integrand over 32
 // lanes in Dual<8> (probes.py:44-51), four tracers per pass.
-__global__ void __launch_bounds__(256) grad_kern_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+__global__ void __launch_bounds__(256) grad_kern_kernel(GradBatch gb, const ConstTables* __restrict__ c, int only_wide) {
   const int item = blockIdx.y;
   if (item >= gb.n_items) return;
   const GradItem gi = grad_item(gb, item);
+  if (only_wide && !gi.tab->wide) return;
   const GeoHeader* geo = gi.geo;
   const int na = geo->na, n_tr = geo->n_tr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1441,12 +1443,14 @@ constexpr int GL_TA = 16;     // a nodes per chunk
 constexpr int GL_THREADS = 256;
 constexpr int GL_MAXO = 17;   // accumulators per thread
 
-// One CTA per (l tile, a split, cosmology): C_ell and dC_ell/dtheta partial sums.
+// One CTA per (l tile, a split, cosmology): C_ell and dC_ell/dtheta partial
+// sums, for the cosmologies whose numbers leave the range of float pairs.
 __global__ void __launch_bounds__(GL_THREADS)
     grad_limber_kernel(GradBatch gb, const ConstTables* __restrict__ c, int LT) {
   const int item = blockIdx.z, split = blockIdx.y;
   if (item >= gb.n_items) return;
   const GradItem gi = grad_item(gb, item);
+  if (!gi.tab->wide) return;
   const GeoHeader* geo = gi.geo;
   const int n_ell = geo->n_ell, n_cls = geo->n_cls, na = geo->na;
   const bool lin = pk_model(geo->physics) == JCG_PK_LINEAR;
@@ -1867,7 +1871,7 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
       grad_rows32_kernel<<<grw, GR32_THREADS, 0, st>>>(gb, c);
     } else {
       dim3 grw((gb.na + 31) / 32, gb.n_items);
-      grad_rows_kernel<<<grw, 256, 0, st>>>(gb, c);
+      grad_rows_kernel<<<grw, 256, 0, st>>>(gb, c, 0);
     }
   }
   if (stages & GS_KERNELS) {
@@ -1875,7 +1879,7 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
       launch_grad_kern32(gb, c, st);
     } else {
       dim3 gr((gb.na + 7) / 8, gb.n_items);
-      grad_kern_kernel<<<gr, 256, 0, st>>>(gb, c);
+      grad_kern_kernel<<<gr, 256, 0, st>>>(gb, c, 0);
     }
   }
 }
@@ -1885,6 +1889,10 @@ void launch_grad(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
   if (gb.precision == JCG_FP32C) {
     launch_grad_limber32(gb, c, st);
   } else {
+    launch_grad_limber64(gb, c, st);
+    // cosmologies out of the pairs' range: rows, kernels and integral in float64
+    grad_rows_kernel<<<dim3((gb.na + 31) / 32, gb.n_items), 256, 0, st>>>(gb, c, 1);
+    grad_kern_kernel<<<dim3((gb.na + 7) / 8, gb.n_items), 256, 0, st>>>(gb, c, 1);
     const int lt = grad_limber_tile(gb.n_ell, gb.n_cls);
     const size_t sml = grad_limber_smem(gb.n_cls, lt);
     cudaFuncSetAttribute(grad_limber_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sml);
@@ -1907,11 +1915,16 @@ namespace jcg {
 // ell tile and a-chunk of the Limber Jacobian kernel of each precision
 int grad_tile(int precision, int n_ell, int n_cls) {
   if (precision == JCG_FP32C) return grad_limber32_tile(n_ell, n_cls);
-  return grad_limber_tile(n_ell, n_cls);
+  int lt, ta;
+  grad_limber64_tile(n_ell, n_cls, &lt, &ta);
+  return lt;
 }
 
 static int grad_chunk(int precision, int n_cls) {
-  return precision == JCG_FP32C ? grad_limber32_chunk(n_cls) : GL_TA;
+  if (precision == JCG_FP32C) return grad_limber32_chunk(n_cls);
+  int lt, ta;
+  grad_limber64_tile(1, n_cls, &lt, &ta);
+  return ta;
 }
 
 // a-splits of the Limber Jacobian: enough CTAs to fill the GPU for small batches

@@ -54,7 +54,8 @@ struct TabD {
   double sigd[NDIR][NRT];
   double pk3v[NKH];
   double pk3d[NDIR][NKH];
-  double pad[7];
+  int wide;  // FP64: 1 where the Limber integral's numbers leave the range of float pairs
+  int padi[13];
   // fp32c Jacobian only: float copies for the FP32 stages
   float c32[NDIR + 1][NCHI];   // chi (row 0) and its tangents
   float s32[NDIR + 1][NCHI];   // segment slopes (chi[i+1] - chi[i]) / (a[i+1] - a[i]) and tangents
@@ -292,6 +293,9 @@ enum GradStage : unsigned { GS_TABLES = 1, GS_ROWS = 2, GS_KERNELS = 4, GS_PRODU
 
 // FP64 tables with tangents (jcg_grad64.cu)
 void launch_grad_tables64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
+// FP64 Limber integral with tangents in float pairs (jcg_gradlim64.cu)
+void launch_grad_limber64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
+void grad_limber64_tile(int n_ell, int n_cls, int* lt, int* ta);
 // FP32 compensated stages (jcg_grad32.cu)
 void launch_grad_kern32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 void launch_grad_limber32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, c
   double* qr = fm + (NDIR + 1) * NCHI;       // [4][NDIR + 1][NGROW] growth coefficients qa, ra, qm, rm
   double* yv = qr + 4 * (NDIR + 1) * NGROW;  // [NGROW][2] growth solution
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) tb->wide = 0;
   for (int i = t; i < NSCAL; i += BG64_THREADS) s[i] = tb->sv[i];
   for (int i = t; i < NDIR * NSCAL; i += BG64_THREADS) sd[i] = tb->sd[i / NSCAL][i % NSCAL];
   __syncthreads();

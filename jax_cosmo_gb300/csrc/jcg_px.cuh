@@ -106,6 +106,13 @@ PX_FN FF px_split(double v) {
   const float hi = px_asf((((h - 0x38000000u) << 3) | (l >> 29)) + ((l >> 28) & 1u));  // to nearest
   return FF{hi, (float)((int)(l << 3) >> 3) * px_asf(((h >> 20) - 948u) << 23)};
 }
+PX_FN bool px_tiny(double v) {  // v >= 0 below what px_split takes
+#ifdef __CUDA_ARCH__
+  return __double2hiint(v) < ((1023 - 70) << 20);
+#else
+  return v < 8.470329472543003e-22;
+#endif
+}
 PX_FN double px_widen(float v) {  // normal v (0 becomes 2^-127)
   const uint32_t u = px_asu(v), h = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u), l = u << 29;
 #ifdef __CUDA_ARCH__
@@ -246,6 +253,16 @@ PX_FN long long px_fix53(float v) {
 }
 PX_FN long long px_fix53(FF v) { return px_fix53(v.hi) + px_fix53(v.lo); }
 
+// a fixed point number of 2^-60 units (a logarithm of 2^-57 units: 8 times its
+// value) as a pair, from its three pieces of 24, 24 and 16 bits
+PX_FN FF px_unfix60(long long v) {
+  const float a = (float)(int)(v >> 40) * 9.5367431640625e-07f;                                 // 2^-20
+  const float b = (float)(int)((v >> 16) & 0xffffff) * 5.684341886080802e-14f;                  // 2^-44
+  const float c = (float)(int)(v & 0xffff) * 8.673617379884035e-19f;                            // 2^-60
+  const FF n = px_norm(a, b);
+  return px_norm(n.hi, n.lo + c);
+}
+
 // 2^Y, Y in 2^-53 units; 0 below 2^-120, infinite from 2^127 on
 PX_FN FF px_exp2(long long Y, const PxTab& T) {
   const int hi = (int)(Y >> 32);
@@ -371,8 +388,9 @@ PX_FN long long px_log2_d(double x, const PxTab& T) {
   return ((long long)e << 57) + T.l2[j] + f;
 }
 
-// sin(pi u), 0 <= u < 2^17
-PX_FN FF px_sinpi(FF u, const PxTab& T) {
+// sin(pi u), 0 <= u < 2^17; COS: and cos(pi u)
+template <bool COS>
+PX_FN FF px_sincospi(FF u, const PxTab& T, FF* co) {
   const float n = rintf(u.hi * 64.f);
   const float d0 = fmaf(n, -0.015625f, u.hi);  // exact, 0 or larger than u.lo
   const float d = d0 + u.lo, dl = (d0 - d) + u.lo;
@@ -396,9 +414,16 @@ PX_FN FF px_sinpi(FF u, const PxTab& T) {
   const float kl = fmaf(-0.5f, pe, (p * p) * fmaf(p, -1.3888889e-3f, 4.1666668e-2f));
   const float2 sj = T.sc[2 * j], cj = T.sc[2 * j + 1];
   // sj + sj (cos z - 1) + cj sin z
-  const FF m1 = px_mul(FF{cj.x, cj.y}, px_norm(s, sl));
-  const FF m2 = px_mul(FF{sj.x, sj.y}, px_norm(k, kl));
+  const FF sz = px_norm(s, sl), cz = px_norm(k, kl);
+  const FF m1 = px_mul(FF{cj.x, cj.y}, sz);
+  const FF m2 = px_mul(FF{sj.x, sj.y}, cz);
+  if (COS) {
+    const FF n1 = px_mul(FF{-sj.x, -sj.y}, sz);
+    const FF n2 = px_mul(FF{cj.x, cj.y}, cz);
+    *co = px_add(px_add(n1, n2), FF{cj.x, cj.y});
+  }
   return px_add(px_add(m1, m2), FF{sj.x, sj.y});
 }
+PX_FN FF px_sinpi(FF u, const PxTab& T) { return px_sincospi<false>(u, T, nullptr); }
 
 }  // namespace jcg

@@ -102,6 +102,7 @@ PX_FN FF px_node(const PxCos& c, const PxTab& T, const long long* row, double kh
   else t = px_eh_osc(c, T, kd, k, k2, lk);
   const double d2 = px_join(px_exp2(px_mulhi(c.ns3, lk) + row[PR_LD], T)) * (t * t);
   const FF d2l = px_split(d2);
+  if (px_tiny(d2)) return FF{0.f, 0.f};  // the caller takes float64
   if (GEN && lin) return d2l;
   const FF y = px_split(kh * rd[PR_IYK]);
   const long long ly = l2kh - row[PR_L2Y];
