@@ -1136,120 +1136,6 @@ __global__ void __launch_bounds__(GR32_THREADS, 2) grad_rows32_kernel(GradBatch 
   }
 }
 
-// ------------------------------------------------------ dual radial kernels -
-// One warp per node: chi_wl and H on lanes 0-7, the lensing integrand over 32
-// lanes in Dual<8> (probes.py:44-51), four tracers per pass.
-__global__ void __launch_bounds__(256) grad_kern_kernel(GradBatch gb, const ConstTables* __restrict__ c, int only_wide) {
-  const int item = blockIdx.y;
-  if (item >= gb.n_items) return;
-  const GradItem gi = grad_item(gb, item);
-  if (only_wide && !gi.tab->wide) return;
-  const GeoHeader* geo = gi.geo;
-  const int na = geo->na, n_tr = geo->n_tr;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = blockIdx.x * 8 + warp;
-  if (n >= na) return;
-  const TabD* tb = gi.tab;
-  const int dir = lane & 7;
-  const double* Z = geo_ptr<double>(geo, geo->off_z);
-  const double* AWL = geo_ptr<double>(geo, geo->off_awl);
-  const int64_t* SW = geo_ptr<int64_t>(geo, geo->off_seg_chiwl);
-  const double* NZL = geo_ptr<double>(geo, geo->off_nzl);
-  const double awl = AWL[n], z = Z[n];
-  D1 sD[NSCAL];
-  for (int i = 0; i < NSCAL; ++i) sD[i] = mk1(tb->sv[i], tb->sd[dir][i]);
-  const D1 chi_wl = xfmax(interp_d1(awl, c->atab_chi, tb->chiv, tb->chid[dir], unpack_seg(SW[n])), 0.0);
-  const D1 cf = 3.0 * (H0 * H0) * sD[S_OMEGA_M] / 2.0 / C_KMS;  // probes.py:71
-  const D8 chiwl8 = gather8(chi_wl);
-  double* kd = gi.kernd;
-  for (int t0 = 0; t0 < n_tr; t0 += 4) {
-    int tl[4];
-    int cnt = 0;
-    for (int t = t0; t < min(t0 + 4, n_tr); ++t) tl[cnt++] = t;
-    D8 acc[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) acc[u] = dconst<NDIR>(0.0);
-    bool any_wl = false;
-    for (int u = 0; u < cnt; ++u) any_wl |= geo->kind[tl[u]] == JCG_TRACER_WL;
-    if (any_wl) {
-      for (int g = 0; g < geo->n_groups; ++g) {
-        const size_t row = (size_t)n * NZP;
-        const double* AP = geo_ptr<double>(geo, geo->off_ap[g]) + row;
-        const int64_t* SP = geo_ptr<int64_t>(geo, geo->off_segp[g]) + row;
-        for (int j = lane; j < NZP; j += 32) {
-          const double ap = AP[j];
-          const int2 sg = unpack_seg(SP[j]);
-          const double ixp = 1.0 / (c->atab_chi[sg.y] - c->atab_chi[sg.x]);
-          D8 chip;
-          {
-            const double a_s = (tb->chiv[sg.y] - tb->chiv[sg.x]) * ixp;
-            const double b_s = tb->chiv[sg.x] - a_s * c->atab_chi[sg.x];
-            chip.v = a_s * ap + b_s;
-#pragma unroll
-            for (int d = 0; d < NDIR; ++d) {
-              const double ad = (tb->chid[d][sg.y] - tb->chid[d][sg.x]) * ixp;
-              chip.d[d] = tb->chid[d][sg.x] + ad * (ap - c->atab_chi[sg.x]);
-            }
-          }
-          chip = xfmax(chip, 0.0);
-          const D8 ratio = xfmax(chip - chiwl8, 0.0) / xfmax(chip, 1.0);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (u < cnt && geo->kind[tl[u]] == JCG_TRACER_WL && geo->group[tl[u]] == g) {
-              const double Wv = geo_ptr<double>(geo, geo->off_W[tl[u]])[row + j];
-              acc[u] = acc[u] + Wv * ratio;
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          acc[u].v += __shfl_xor_sync(0xffffffffu, acc[u].v, o);
-#pragma unroll
-          for (int d = 0; d < NDIR; ++d) acc[u].d[d] += __shfl_xor_sync(0xffffffffu, acc[u].d[d], o);
-        }
-      }
-    }
-    if (lane < NDIR) {
-      for (int u = 0; u < cnt; ++u) {
-        const int t = tl[u];
-        D1 kv;
-        if (geo->kind[t] == JCG_TRACER_WL) {
-          double ad = 0.0;
-#pragma unroll
-          for (int d = 0; d < NDIR; ++d)
-            if (d == dir) ad = acc[u].d[d];
-          D1 racc = mk1(acc[u].v, ad);
-          if (geo->nz_kind[t] == JCG_NZ_DELTA) {
-            // single plane (probes.py:53-64): clip(chi(z0) - chi, 0) / clip(chi(z0), 1)
-            const double a0 = 1.0 / (1.0 + geo->nz_z0[t]);
-            const int2 sg0 = interp_segment_inc(a0, c->atab_chi, NCHI, logspace_guess(a0, NCHI));
-            const D1 chi0 = xfmax(interp_d1(a0, c->atab_chi, tb->chiv, tb->chid[dir], sg0), 0.0);
-            racc = xfmax(chi0 - chi_wl, 0.0) / xfmax(chi0, 1.0);
-          }
-          const D1 rk = racc * (1.0 + z) * chi_wl;
-          kv = cf * rk;
-          if (geo->bias_kind[t] != JCG_BIAS_NONE) {
-            double iv, id;
-            bias_term_d1(tb, c, geo, t, dir, awl, z, NZL[(size_t)t * na + n], true, &iv, &id);
-            kv = kv + mk1(iv, id);
-          }
-          kv = kv * (1.0 + geo->mult[t]);
-        } else {
-          double iv, id;
-          bias_term_d1(tb, c, geo, t, dir, awl, z, NZL[(size_t)t * na + n], false, &iv, &id);
-          kv = mk1(iv, id);
-        }
-        double* dst = kd + ((size_t)t * na + n) * (NDIR + 1);
-        if (dir == 0) dst[0] = kv.v;
-        dst[1 + dir] = kv.d[0];
-      }
-    }
-  }
-}
-
 // ------------------------------------------------ Limber integrand adjoint --
 struct NodeX {
   double chic, g, knl, beta, alpha, an, bn, lcf3, f1, f2, gam, nu, mu;
@@ -1878,8 +1764,7 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
     if (gb.precision == JCG_FP32C) {
       launch_grad_kern32(gb, c, st);
     } else {
-      dim3 gr((gb.na + 7) / 8, gb.n_items);
-      grad_kern_kernel<<<gr, 256, 0, st>>>(gb, c, 0);
+      launch_grad_kern64(gb, c, st, 0);
     }
   }
 }
@@ -1892,7 +1777,7 @@ void launch_grad(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
     launch_grad_limber64(gb, c, st);
     // cosmologies out of the pairs' range: rows, kernels and integral in float64
     grad_rows_kernel<<<dim3((gb.na + 31) / 32, gb.n_items), 256, 0, st>>>(gb, c, 1);
-    grad_kern_kernel<<<dim3((gb.na + 7) / 8, gb.n_items), 256, 0, st>>>(gb, c, 1);
+    launch_grad_kern64(gb, c, st, 1);
     const int lt = grad_limber_tile(gb.n_ell, gb.n_cls);
     const size_t sml = grad_limber_smem(gb.n_cls, lt);
     cudaFuncSetAttribute(grad_limber_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sml);
@@ -2142,6 +2027,7 @@ void grad_run(const GeoHeader* geo, const GeoHeader& h, const double* params, in
   gb.jac = jac;
   gb.na = h.na;
   gb.n_tr = h.n_tr;
+  gb.n_wl = h.n_wl;
   gb.n_cls = h.n_cls;
   gb.n_ell = h.n_ell;
   gb.n_split = grad_n_split(h, n_cosmo, precision);

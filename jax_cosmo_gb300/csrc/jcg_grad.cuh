@@ -293,6 +293,9 @@ enum GradStage : unsigned { GS_TABLES = 1, GS_ROWS = 2, GS_KERNELS = 4, GS_PRODU
 
 // FP64 tables with tangents (jcg_grad64.cu)
 void launch_grad_tables64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
+// FP64 radial kernels with tangents (jcg_gradkern64.cu); only_wide: of the
+// cosmologies with TabD::wide set
+void launch_grad_kern64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
 // FP64 Limber integral with tangents in float pairs (jcg_gradlim64.cu)
 void launch_grad_limber64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 void grad_limber64_tile(int n_ell, int n_cls, int* lt, int* ta);

@@ -22,42 +22,14 @@
 // 5 bins, 513 nodes, 4096 cosmologies: 30.6 -> 3.5 ms; one cosmology, 2 bins, 257
 // nodes: 82 -> 15 us; 5 + 5 bins, 513 nodes: 195 -> 28 us.
 #include "jcg_internal.cuh"
-#include "jcg_px.cuh"
+#include "jcg_wl64.cuh"
 
 namespace jcg {
 
 constexpr int T64_WARPS = 8;
-constexpr int T64_RUN = 8;                       // points per run
-constexpr int T64_RUNS = (NZP + T64_RUN - 1) / T64_RUN;  // 33: 32 full runs and the last point
 constexpr int T64_PAD = 33;
+constexpr int T64_NODES = 32;                    // nodes per CTA at most
 
-// v of either sign as a pair; 0 below 2^-70
-__device__ __forceinline__ FF px_split_s(double v) {
-  const double u = fabs(v);
-  if (u < 8.5e-22) return FF{0.f, 0.f};
-  const FF a = px_split(u);
-  return v < 0.0 ? FF{-a.hi, -a.lo} : a;
-}
-// v 2^(1023 - ex) as a pair, ex the largest exponent field of the row; 0 where
-// it is below 2^-70 of the row's largest
-__device__ __forceinline__ FF px_split_scaled(double v, int ex) {
-  const int h = __double2hiint(v), f = (h >> 20) & 0x7ff;
-  if (f <= ex - 70 || f == 0) return FF{0.f, 0.f};
-  return px_split_s(__hiloint2double(h + ((1023 - ex) << 20), __double2loint(v)));
-}
-__device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-
-// chi_x - chi of the node, chi = chi_w + sdw on its own segment, from three-float
-// table values: far above a bin's redshift the points next to the node are the
-// integral, and a rounding of chi would be 1e-13 of their differences
-struct WlNode {
-  F3 cw;
-  FF sdw;
-};
-__device__ __forceinline__ FF wl_base(float2 cx, float cll, const WlNode& w) {
-  const FF d = px_two_sum(cx.x, -w.cw.hi);
-  return px_add(px_two_sum(d.hi, d.lo + ((cx.y - w.cw.lo) + (cll - w.cw.ll))), FF{-w.sdw.hi, -w.sdw.lo});
-}
 // clip(chi' - chi, 0) / clip(chi', 1) at a' = a_x + dx on the segment (chi_x,
 // slope); base = chi_x - chi
 __device__ __forceinline__ FF wl_ratio(float2 cx, FF base, float2 sl, FF dx) {
@@ -123,6 +95,7 @@ __global__ void __launch_bounds__(T64_WARPS * 32)
   __shared__ double atab[NCHI];
   __shared__ float2 runs[T64_WARPS][T64_RUNS][MAXTR];
   __shared__ int exps[T64_WARPS][MAXTR];
+  __shared__ double accs[MAXTR][T64_NODES], chis[T64_NODES];
   const CosmoTab* ct = it.ctab;
   for (int i = threadIdx.x; i < NCHI; i += blockDim.x) {
     const F3 a = px3_of(ct->chi[i]);
@@ -186,9 +159,7 @@ __global__ void __launch_bounds__(T64_WARPS * 32)
       }
     }
     __syncwarp();
-    double hz = 0.0, dz = 1.0;
-    if (geo->n_nc > 0 || geo->special_bias) hz = bg_H(make_bg(ct->s), awl);
-    if (geo->special_bias) dz = growth_at(ct->g, c, awl);
+    if (lane == 0) chis[n - n0] = chi_wl;
     if (lane < n_tr) {
       const int t = lane;
       double acc = 0.0;
@@ -202,9 +173,25 @@ __global__ void __launch_bounds__(T64_WARPS * 32)
           acc = scalbn(px_d3(tot), ex - 1023);
         }
       }
-      it.kern[(size_t)t * na + n] = tracer_value(geo, ct, c, t, n, acc, chi_wl, Z[n], om, hz, dz);
+      accs[t][n - n0] = acc;
     }
     __syncwarp();
+  }
+  // A thread per (tracer, node): H, the growth factor and the bias are some
+  // hundred float64 operations, which cost a warp the same with one lane live as
+  // with 32 (on n_tr lanes of each node's warp: 61 cosmologies, 3 + 2 bins with
+  // alignment terms 838 us, now 404 us)
+  __syncthreads();
+  const int nn = n_end - n0;
+  for (int q = threadIdx.x; q < nn * n_tr; q += blockDim.x) {
+    const int t = q / nn, i = q - t * nn, n = n0 + i;
+    const bool wl = geo->kind[t] == JCG_TRACER_WL;
+    const double awl = AWL[n];
+    double hz = 0.0, dz = 1.0;
+    if (!wl || geo->bias_kind[t] != JCG_BIAS_NONE) hz = bg_H(make_bg(ct->s), awl);
+    if (geo->bias_kind[t] == JCG_BIAS_INV_GROWTH || (wl && geo->bias_kind[t] != JCG_BIAS_NONE))
+      dz = growth_at(ct->g, c, awl);
+    it.kern[(size_t)t * na + n] = tracer_value(geo, ct, c, t, n, accs[t][i], chis[i], Z[n], om, hz, dz);
   }
 }
 
@@ -346,9 +333,9 @@ __global__ void __launch_bounds__(T64_WARPS * 32, 2)
   }
 }
 
-// nodes per CTA: 32 pay for the table loads; fewer while the CTAs do not fill the SMs
+// nodes per CTA: T64_NODES pay for the table loads; fewer while the CTAs do not fill the SMs
 static int t64_nodes(int na, int rows) {
-  int per = 32;
+  int per = T64_NODES;
   while (per > T64_WARPS && (long long)rows * ((na + per - 1) / per) < 2 * device_sm_count()) per >>= 1;
   return per;
 }
