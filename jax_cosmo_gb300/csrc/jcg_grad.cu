@@ -491,222 +491,6 @@ __global__ void __launch_bounds__(NRT) grad_moments32_kernel(GradBatch gb, const
 
 size_t grad_tables_smem() { return sizeof(double) * (NSCAL * (1 + NDIR) + GNODE_U + NDIR + 1); }
 
-// ----------------------------------------------------------- dual rows -----
-// FP64 Jacobian rows.  One warp per 4 Limber nodes: lane = 8 * node slot +
-// tangent direction.
-//   prelude (per lane, Dual<1>): growth, chi, the root find (index from the
-//     values with the forward's arithmetic, tangent through the interpolation
-//     formula), R = 1 / k_nl;
-//   moments (power.py:121-139), node by node over all 32 lanes, as scalar sums
-//     with their R-derivatives and their P(k) k^3 tangents:
-//       S1 = sum w q3 2 y^2 e^{-y^2},  S2 = sum w q3 4 (y^2 - y^4) e^{-y^2},
-//       y = k R, q3 = P(k) k^3 / (2 pi^2);  dS = S_q3[d] + dS/dR dR[d];
-//     every term with y^2 <= 60 (the rest is below 1e-20 of the sums);
-//   epilogue (per lane, Dual<1>): n_eff, C, takahashi2012 coefficients, the
-//     Limber weight; rows out.
-__global__ void __launch_bounds__(256) grad_rows_kernel(GradBatch gb, const ConstTables* __restrict__ c, int only_wide) {
-  const int item = blockIdx.y;
-  if (item >= gb.n_items) return;
-  const GradItem gi = grad_item(gb, item);
-  if (only_wide && !gi.tab->wide) return;
-  const GeoHeader* geo = gi.geo;
-  const int na = geo->na;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slot = lane >> 3, dir = lane & 7;
-  const int n_first = (blockIdx.x * 8 + warp) * 4;
-  if (n_first >= na) return;
-  const int n_raw = n_first + slot;
-  const bool live = n_raw < na;
-  const int n = live ? n_raw : na - 1;  // dead slots evaluate a valid node, write nothing
-  const TabD* tb = gi.tab;
-  const double* A = geo_ptr<double>(geo, geo->off_a);
-  const double* WS = geo_ptr<double>(geo, geo->off_wsimp);
-  const int64_t* SC = geo_ptr<int64_t>(geo, geo->off_seg_chi);
-  const int64_t* SG = geo_ptr<int64_t>(geo, geo->off_seg_grow);
-  const double a = A[n];
-  D1 g = interp_d1(a, c->atab_grow, tb->gv, tb->gd[dir], unpack_seg(SG[n]));
-  g = xfmin(xfmax(g, 0.0), 1.0);
-  D1 chi = interp_d1(a, c->atab_chi, tb->chiv, tb->chid[dir], unpack_seg(SC[n]));
-  chi = xfmax(chi, 0.0);
-  const D1 g2 = g * g;
-  int ind, j2;
-  if (gb.seg_in) {
-    // the segment of another parameter point: differentiate on its branch
-    const int pk = gb.seg_in[(size_t)item * na + n];
-    ind = min(max(pk & 0xffff, 1), NRT - 2);
-    j2 = ind + ((pk >> 16) ? 1 : -1);
-  } else {
-    int best;
-    int lo = 0, hi = NRT;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (tb->sigv[mid] * g2.v > 1.0) lo = mid + 1;
-      else hi = mid;
-    }
-    const int cc = lo;
-    best = cc < NRT ? cc : NRT - 1;
-    if (cc >= 1) {
-      const double dlo = 1.0 - tb->sigv[cc - 1] * g2.v;
-      if (cc < NRT) {
-        const double dhi = 1.0 - tb->sigv[cc] * g2.v;
-        best = (dlo * dlo <= dhi * dhi) ? cc - 1 : cc;
-      } else {
-        best = cc - 1;
-      }
-    }
-    ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-    const double xpi = tb->sigv[ind] * g2.v;
-    const double xc = fmin(fmax(1.0, tb->sigv[1] * g2.v), tb->sigv[NRT - 2] * g2.v);
-    j2 = ind + ((xc - xpi >= 0.0) ? 1 : -1);
-  }
-  if (gb.seg_out && live && dir == 0) gb.seg_out[(size_t)item * na + n] = ind | ((j2 > ind ? 1 : 0) << 16);
-  const D1 xp0 = mk1(tb->sigv[ind], tb->sigd[dir][ind]) * g2;
-  const D1 xp1 = mk1(tb->sigv[j2], tb->sigd[dir][j2]) * g2;
-  const D1 slope = (c->logr[j2] - c->logr[ind]) / (xp1 - xp0);
-  const D1 bb = c->logr[ind] - slope * xp0;
-  const D1 root = slope * 1.0 + bb;
-  const D1 R = xfmax(xexp(root), 1e-6);
-  const D1 knl = 1.0 / R;
-  const D1 inv = 1.0 / knl;
-  const int ilo = 0, ihi = NKH - 1;
-  // explicit terms, node by node over the warp
-  double m_s1 = 0, m_s2 = 0, m_s1r = 0, m_s2r = 0, m_s1d = 0, m_s2d = 0;
-  const double q3s = 1.0 / TWO_PI2_G;
-  for (int q = 0; q < 4; ++q) {
-    const double Rq = __shfl_sync(0xffffffffu, inv.v, q * 8);
-    const int lo = __shfl_sync(0xffffffffu, ilo, q * 8), hi = __shfl_sync(0xffffffffu, ihi, q * 8);
-    const double iRq = 1.0 / Rq;
-    double s1 = 0, s2 = 0, s1r = 0, s2r = 0, s1d[NDIR], s2d[NDIR];
-#pragma unroll
-    for (int d = 0; d < NDIR; ++d) s1d[d] = s2d[d] = 0.0;
-    for (int i = lo + lane; i <= hi; i += 32) {
-      const double y = c->kh[i] * Rq;
-      const double y2 = y * y;
-      if (y2 > Y2_SKIP) continue;
-      const double E = exp(-y2);
-      const double wq = c->simpson_kh[i] * E * q3s;
-      const double Av = wq * tb->pk3v[i];
-      const double c1 = 2.0 * y2, c2 = 4.0 * (y2 - y2 * y2);
-      s1 += Av * c1;
-      s2 += Av * c2;
-      s1r += 4.0 * Av * y2 * (1.0 - y2) * iRq;
-      s2r += 8.0 * Av * y2 * (1.0 - 3.0 * y2 + y2 * y2) * iRq;
-      const double w1 = wq * c1, w2 = wq * c2;
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d) {
-        const double p = tb->pk3d[d][i];
-        s1d[d] += w1 * p;
-        s2d[d] += w2 * p;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      s1r += __shfl_xor_sync(0xffffffffu, s1r, o);
-      s2r += __shfl_xor_sync(0xffffffffu, s2r, o);
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d) {
-        s1d[d] += __shfl_xor_sync(0xffffffffu, s1d[d], o);
-        s2d[d] += __shfl_xor_sync(0xffffffffu, s2d[d], o);
-      }
-    }
-    if (slot == q) {
-      m_s1 = s1;
-      m_s2 = s2;
-      m_s1r = s1r;
-      m_s2r = s2r;
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d)
-        if (d == dir) {
-          m_s1d = s1d[d];
-          m_s2d = s2d[d];
-        }
-    }
-  }
-  // moments with their tangents in this lane's direction, times g^2
-  const D1 S1 = mk1(m_s1, m_s1d + m_s1r * inv.d[0]);
-  const D1 S2 = mk1(m_s2, m_s2d + m_s2r * inv.d[0]);
-  const D1 I1 = S1 * g2, I2 = S2 * g2;
-
-  const D1 neff = I1 - 3.0;
-  const D1 C = I1 * I1 + I2;
-  // coefficients (power.py:177-238)
-  D1 sD[NSCAL];
-  for (int i = 0; i < NSCAL; ++i) sD[i] = mk1(tb->sv[i], tb->sd[dir][i]);
-  const BgT<D1> bg = make_bgT(sD);
-  const double lna = log(a);
-  D1 om_m, om_de;
-  omT(bg, a, lna, om_m, om_de);
-  const D1 w = wT(bg, a);
-  const HfCoef<D1> hc = hf_coefs<D1>(pk_model(gi.geo->physics), neff, C, om_m, om_de, w);
-  D1 outv[NA_IN];
-  outv[A_CHIC] = xfmax(chi, 1.0);
-  outv[A_G] = g;
-  outv[A_KNL] = knl;
-  outv[A_BETA] = hc.beta;
-  outv[A_ALPHA] = hc.alpha;
-  outv[A_AN] = hc.an;
-  outv[A_BN] = hc.bn;
-  outv[A_LCF3] = hc.lcf3;
-  outv[A_F1] = hc.f1;
-  outv[A_F2] = hc.f2;
-  outv[A_GAM] = hc.gam;
-  outv[A_NU] = hc.nu;
-  outv[A_MU] = hc.mu;
-  const D1 dchi = dchioverdaT(bg, a, lna);
-  outv[A_U] = WS[n] * dchi / xfmax(chi * chi, 1.0) / C2_G;
-  if (live) {
-    if (gb.precision == JCG_FP64) {
-      double* row = gi.rowd + (size_t)n * NROWD;
-      for (int i = 0; i < NA_IN; ++i) {
-        if (dir == 0) row[i] = outv[i].v;
-        row[NA_IN * (1 + dir) + i] = outv[i].d[0];
-      }
-    } else {
-      // FP32 row: values in the forward row's units, tangents of the inputs
-      constexpr double LOG2E = 1.4426950408889634;
-      float* row = gi.rowg + (size_t)n * NROWG;
-      const D1 chic = outv[A_CHIC], kn = outv[A_KNL];
-      const D1 d2fac = outv[A_G] * outv[A_G] * sD[S_PKNORM] / TWO_PI2_G;
-      if (dir == 0) {
-        row[F_INVCHI] = (float)(1.0 / chic.v);
-        row[F_LG2INVCHI] = (float)(-log2(chic.v));
-        row[F_CHIC] = (float)chic.v;
-        row[F_LG2KNL] = (float)log2(kn.v);
-        row[F_INVKNL] = (float)(1.0 / kn.v);
-        row[F_D2FAC] = (float)d2fac.v;
-        row[F_BETAN] = (float)outv[A_BETA].v;
-        row[F_ALPHAN] = (float)outv[A_ALPHA].v;
-        row[F_AN] = (float)outv[A_AN].v;
-        row[F_3F1] = (float)(3.0 * outv[A_F1].v);
-        row[F_F2] = (float)outv[A_F2].v;
-        row[F_BN] = (float)outv[A_BN].v;
-        row[F_LG2CF3] = (float)(LOG2E * outv[A_LCF3].v);
-        row[F_3MGAMMA] = (float)(3.0 - outv[A_GAM].v);
-        row[F_NUN] = (float)outv[A_NU].v;
-        row[F_MUN] = (float)outv[A_MU].v;
-        row[F_U] = (float)outv[A_U].v;
-      }
-      float* tg = row + NROWV;
-      tg[T_CHIC * NDIR + dir] = (float)chic.d[0];
-      tg[T_D2FAC * NDIR + dir] = (float)d2fac.d[0];
-      tg[T_KNL * NDIR + dir] = (float)kn.d[0];
-      tg[T_BETAN * NDIR + dir] = (float)outv[A_BETA].d[0];
-      tg[T_ALPHAN * NDIR + dir] = (float)outv[A_ALPHA].d[0];
-      tg[T_AN * NDIR + dir] = (float)outv[A_AN].d[0];
-      tg[T_3F1 * NDIR + dir] = (float)(3.0 * outv[A_F1].d[0]);
-      tg[T_F2 * NDIR + dir] = (float)outv[A_F2].d[0];
-      tg[T_BN * NDIR + dir] = (float)outv[A_BN].d[0];
-      tg[T_LG2CF3 * NDIR + dir] = (float)(LOG2E * outv[A_LCF3].d[0]);
-      tg[T_3MG * NDIR + dir] = (float)(-outv[A_GAM].d[0]);
-      tg[T_NUN * NDIR + dir] = (float)outv[A_NU].d[0];
-      tg[T_MUN * NDIR + dir] = (float)outv[A_MU].d[0];
-      tg[T_U * NDIR + dir] = (float)outv[A_U].d[0];
-    }
-  }
-}
-
 // ------------------------------------------------------- fp32c rows -------
 __device__ __forceinline__ F8 interp_f8(double x, const double* xp, const double* fv, const double* fd,
                                         int stride, int2 sg) {
@@ -717,7 +501,7 @@ __device__ __forceinline__ F8 interp_f8(double x, const double* xp, const double
 }
 
 // fp32c Jacobian rows: one node per thread in DualF<8> (value FP64, the 8
-// tangents FP32), the same operations as grad_rows_kernel's FP32C path: root
+// tangents FP32), the operations: root
 // find, moments (exp terms for y^2 in [1, 60], Taylor prefix tables below),
 // takahashi2012 coefficients, Limber weight; the row is written as computed.
 // interpolation on the segment sg of a table with tangents, by the segment's
@@ -1717,10 +1501,11 @@ __global__ void __launch_bounds__(32 * NDIR) grad_growth_gamma_kernel(GradBatch 
       if (d == 0) {
         tb->gv[i] = g.v;
         const FF gf = ff_of(g.v);
-        tb->gF[i] = make_float2(gf.hi, gf.lo);  // the row stage's copy
+        // the fp32c row stage's copy (FP64: other numbers are kept there)
+        if (gb.precision == JCG_FP32C) tb->gF[i] = make_float2(gf.hi, gf.lo);
       }
       tb->gd[d][i] = g.d[0];
-      tb->gdF[i][d] = (float)g.d[0];
+      if (gb.precision == JCG_FP32C) tb->gdF[i][d] = (float)g.d[0];
     }
   }
 }
@@ -1756,8 +1541,7 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
                                  : dim3((unsigned)(((long long)gb.na * gb.n_items + GR32_THREADS - 1) / GR32_THREADS));
       grad_rows32_kernel<<<grw, GR32_THREADS, 0, st>>>(gb, c);
     } else {
-      dim3 grw((gb.na + 31) / 32, gb.n_items);
-      grad_rows_kernel<<<grw, 256, 0, st>>>(gb, c, 0);
+      launch_grad_rows64(gb, c, st, 0);
     }
   }
   if (stages & GS_KERNELS) {
@@ -1776,7 +1560,7 @@ void launch_grad(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
   } else {
     launch_grad_limber64(gb, c, st);
     // cosmologies out of the pairs' range: rows, kernels and integral in float64
-    grad_rows_kernel<<<dim3((gb.na + 31) / 32, gb.n_items), 256, 0, st>>>(gb, c, 1);
+    launch_grad_rows64(gb, c, st, 1);
     launch_grad_kern64(gb, c, st, 1);
     const int lt = grad_limber_tile(gb.n_ell, gb.n_cls);
     const size_t sml = grad_limber_smem(gb.n_cls, lt);

@@ -293,8 +293,18 @@ enum GradStage : unsigned { GS_TABLES = 1, GS_ROWS = 2, GS_KERNELS = 4, GS_PRODU
 
 // FP64 tables with tangents (jcg_grad64.cu)
 void launch_grad_tables64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
-// FP64 radial kernels with tangents (jcg_gradkern64.cu); only_wide: of the
+// simpson_kh[i] * (P(k_i) k_i^3 and its tangents) / (2 pi^2) as pairs
+// [NDIR + 1][NKH], in the part of TabD past the tables' node scratch
+constexpr int GRAD_NEH = NROMB + NKH;
+__device__ __forceinline__ float2* grad_kw64(TabD* t) {
+  return reinterpret_cast<float2*>(reinterpret_cast<double*>(&t->c32[0][0]) + (NDIR + 1) * GRAD_NEH);
+}
+__device__ __forceinline__ const float2* grad_kw64(const TabD* t) { return grad_kw64(const_cast<TabD*>(t)); }
+static_assert(sizeof(TabD) - offsetof(TabD, c32) >= sizeof(double) * (NDIR + 1) * (GRAD_NEH + NKH), "scratch fits");
+// FP64 rows and radial kernels with tangents (jcg_gradrows64.cu,
+// jcg_gradkern64.cu); only_wide: of the
 // cosmologies with TabD::wide set
+void launch_grad_rows64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
 void launch_grad_kern64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
 // FP64 Limber integral with tangents in float pairs (jcg_gradlim64.cu)
 void launch_grad_limber64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);

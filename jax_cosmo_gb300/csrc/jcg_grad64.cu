@@ -16,13 +16,13 @@
 // One cosmology 1,453 -> 119 us (75 + 23 + 21), 61 cosmologies 1,456 -> 210 us; what is left is
 // latency: serial float64 code of a thread, the scans and 257 loads of E per R.
 #include "jcg_grad.cuh"
+#include "jcg_px.cuh"
 
 namespace jcg {
 
 // node scratch in the part of TabD that only fp32c uses: exp(n_s ln k) T^2 (times
 // the window for the Romberg nodes) as [NDIR + 1][NROMB + NKH]
-constexpr int NEH = NROMB + NKH;
-static_assert(sizeof(TabD) - offsetof(TabD, c32) >= sizeof(double) * (NDIR + 1) * NEH, "node scratch fits");
+constexpr int NEH = GRAD_NEH;
 static_assert(offsetof(TabD, c32) % 8 == 0, "node scratch alignment");
 __device__ __forceinline__ double* eh_scratch(TabD* t) { return reinterpret_cast<double*>(&t->c32[0][0]); }
 
@@ -376,6 +376,10 @@ __global__ void __launch_bounds__(SG64_THREADS) grad_sigma64_kernel(GradBatch gb
     const double v = u[NROMB + i], p = (comp ? ud[NROMB + i] * pn + v * dpn : v * pn) * c->kh3[i];
     if (part == 0) (comp ? tb->pk3d[comp - 1] : tb->pk3v)[i] = p;
     pq[i] = c->simpson_kh[i] * (p / (2.0 * (PI * PI)));
+    if (part == 0) {
+      const FF f = px_of(pq[i]);
+      grad_kw64(tb)[comp * NKH + i] = make_float2(f.hi, f.lo);
+    }
   }
   __syncthreads();
   const int j = part * SG64_THREADS + t;

@@ -232,33 +232,6 @@ __device__ __forceinline__ double chi_at(const CosmoTab* ct, const ConstTables* 
 constexpr int HF_WARPS = 8;
 constexpr int HF_NODES = 256;  // fp32c: Limber nodes per CTA (every thread busy in the thread-per-node phases)
 
-// argmin_j (1 - sig_j g2)^2 with the first index on ties, by one thread: c =
-// #{j : sig_j g2 > 1} by bisection (the sequence is strictly decreasing), then
-// the nearer of c - 1, c; and the other end of the segment on the side of
-// sign(clip(1, v_1, v_{n-2}) - v_ind) (scipy/interpolate.py:47-57).
-__device__ __forceinline__ void root_segment(const double* sig, double g2, int& ind, int& j2) {
-  int lo = 0, hi = NRT;  // invariant: v_j > 1 for j < lo, v_j <= 1 for j >= hi
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (sig[mid] * g2 > 1.0) lo = mid + 1;
-    else hi = mid;
-  }
-  const int cc = lo;
-  int best = cc < NRT ? cc : NRT - 1;
-  if (cc >= 1) {
-    const double dlo = 1.0 - sig[cc - 1] * g2;
-    if (cc < NRT) {
-      const double dhi = 1.0 - sig[cc] * g2;
-      best = (dlo * dlo <= dhi * dhi) ? cc - 1 : cc;
-    } else {
-      best = cc - 1;
-    }
-  }
-  ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-  const double xc = fmin(fmax(1.0, sig[1] * g2), sig[NRT - 2] * g2);  // clip(x, xp[1], xp[-2])
-  j2 = ind + ((xc - sig[ind] * g2 >= 0.0) ? 1 : -1);
-}
-
 // fp32c: the same root find with the interpolation (power.py:112-115) in
 // float pairs: the segment is chosen in float64 exactly as above (the
 // decision), then R = exp(root) with root = logr[ind] + slope (1 - xp_ind) by

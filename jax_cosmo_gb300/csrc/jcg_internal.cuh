@@ -353,6 +353,33 @@ __device__ __forceinline__ double npow(double x, double y) {
   return pow(x, y);
 }
 
+// argmin_j (1 - sig_j g2)^2 with the first index on ties, by one thread: c =
+// #{j : sig_j g2 > 1} by bisection (the sequence is strictly decreasing), then
+// the nearer of c - 1, c; and the other end of the segment on the side of
+// sign(clip(1, v_1, v_{n-2}) - v_ind) (scipy/interpolate.py:47-57).
+__device__ __forceinline__ void root_segment(const double* sig, double g2, int& ind, int& j2) {
+  int lo = 0, hi = NRT;  // invariant: v_j > 1 for j < lo, v_j <= 1 for j >= hi
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (sig[mid] * g2 > 1.0) lo = mid + 1;
+    else hi = mid;
+  }
+  const int cc = lo;
+  int best = cc < NRT ? cc : NRT - 1;
+  if (cc >= 1) {
+    const double dlo = 1.0 - sig[cc - 1] * g2;
+    if (cc < NRT) {
+      const double dhi = 1.0 - sig[cc] * g2;
+      best = (dlo * dlo <= dhi * dhi) ? cc - 1 : cc;
+    } else {
+      best = cc - 1;
+    }
+  }
+  ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
+  const double xc = fmin(fmax(1.0, sig[1] * g2), sig[NRT - 2] * g2);  // clip(x, xp[1], xp[-2])
+  j2 = ind + ((xc - sig[ind] * g2 >= 0.0) ? 1 : -1);
+}
+
 // jnp.clip(x, lo) / jnp.clip(x, lo, hi)
 __device__ __forceinline__ double clip_lo(double x, double lo) { return fmax(x, lo); }
 __device__ __forceinline__ double clip_lohi(double x, double lo, double hi) {
