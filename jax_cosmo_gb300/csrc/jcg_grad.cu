@@ -1584,25 +1584,17 @@ namespace jcg {
 // ell tile and a-chunk of the Limber Jacobian kernel of each precision
 int grad_tile(int precision, int n_ell, int n_cls) {
   if (precision == JCG_FP32C) return grad_limber32_tile(n_ell, n_cls);
-  int lt, ta;
-  grad_limber64_tile(n_ell, n_cls, &lt, &ta);
-  return lt;
-}
-
-static int grad_chunk(int precision, int n_cls) {
-  if (precision == JCG_FP32C) return grad_limber32_chunk(n_cls);
-  int lt, ta;
-  grad_limber64_tile(1, n_cls, &lt, &ta);
-  return ta;
+  return grad_limber64_tile(n_ell, n_cls);
 }
 
 // a-splits of the Limber Jacobian: enough CTAs to fill the GPU for small batches
 int grad_n_split(const GeoHeader& h, int n_cosmo, int precision) {
   const int lt = grad_tile(precision, h.n_ell, h.n_cls);
   const int tiles = (h.n_ell + lt - 1) / lt;
+  if (precision != JCG_FP32C) return grad_limber64_split((long long)tiles * n_cosmo, h.na, lt);
   const int ctas = tiles * n_cosmo;
   int ns = (2 * 152 + ctas - 1) / ctas;
-  const int ta = grad_chunk(precision, h.n_cls);
+  const int ta = grad_limber32_chunk(h.n_cls);
   const int max_ns = (h.na + ta - 1) / ta;
   if (ns > max_ns) ns = max_ns;
   if (ns < 1) ns = 1;
@@ -1847,8 +1839,9 @@ int grad_listed_auto_split(const GradReq* r, int n, int precision) {
   const int lt = grad_tile(precision, max_ell, max_cls);
   long ctas = 0;
   for (int i = 0; i < n; ++i) ctas += (r[i].h->n_ell + lt - 1) / lt;
+  if (precision != JCG_FP32C) return grad_limber64_split(ctas, min_na, lt);
   int ns = (int)((2 * 152 + ctas - 1) / ctas);
-  const int ta = grad_chunk(precision, max_cls);
+  const int ta = grad_limber32_chunk(max_cls);
   const int max_ns = (min_na + ta - 1) / ta;
   if (ns > max_ns) ns = max_ns;
   return ns < 1 ? 1 : ns;

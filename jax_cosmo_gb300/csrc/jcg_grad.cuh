@@ -308,7 +308,8 @@ void launch_grad_rows64(const GradBatch& gb, const ConstTables* c, cudaStream_t 
 void launch_grad_kern64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
 // FP64 Limber integral with tangents in float pairs (jcg_gradlim64.cu)
 void launch_grad_limber64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
-void grad_limber64_tile(int n_ell, int n_cls, int* lt, int* ta);
+int grad_limber64_tile(int n_ell, int n_cls);
+int grad_limber64_split(long long tiles, int na, int lt);
 // FP32 compensated stages (jcg_grad32.cu)
 void launch_grad_kern32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 void launch_grad_limber32(const GradBatch& gb, const ConstTables* c, cudaStream_t st);

@@ -18,10 +18,11 @@
 // the 17 products of its value and tangents in pairs and adds the block to
 // three-float totals.
 //
-// 10 tracers (55 spectra), 200 ell, 513 nodes, one cosmology: 1,195 -> 300 us with
-// the two packing kernels; 61 cosmologies, 15 spectra, 97 ell, all operator points
-// but the default ones: 14.6 -> 2.04 ms.  Bound by FP32 issue: 7,000 instructions
-// a node and 220 per spectrum and node.  Three-float totals in the node and runs
+// 10 tracers (55 spectra), 200 ell, 513 nodes, one cosmology: 1,195 -> 178 us and
+// 26 us for the two packing kernels; 61 cosmologies, 15 spectra, 97 ell: 14.6 ->
+// 1.81 ms and 0.15.  Bound by the latency of FP32 chains (8,000 instructions a
+// node, 220 per spectrum and node; 4 warps per scheduler at 128 registers, 0.4 to
+// 0.5 instructions per cycle; three CTAs an SM spill: 1.92 ms).  Three-float totals in the node and runs
 // of 4 nodes cost 20% of that and bring the tangents' error, which cancelling
 // terms amplify, below the float64 kernels' on the former tables (1.46e-15 and
 // 2.27e-15 of their norm against 1.58e-15 and 2.75e-15, by 80-bit arithmetic).
@@ -286,12 +287,13 @@ __global__ void __launch_bounds__(GXP_THREADS) grad_pack64_kernel(GradBatch gb, 
 }
 
 // -------------------------------------------------------------- integral ---
-constexpr int GX_TA = 16;  // a nodes per chunk at most (32: as fast, more shared memory)
 constexpr int GX_RUN = 4;  // a nodes summed in pairs before the three-float totals
 struct GxLayout {
   size_t tab, g, kh, l2kh, P, K, M, tot, total;
   int mb;
 };
+// a nodes per chunk at most: as many as give every thread one node
+__host__ __device__ inline int gx_ta(int LT) { return GX_THREADS / LT; }
 __host__ __device__ inline GxLayout gx_layout_mb(int n_cls, int n_tr, int LT, int mb) {
   GxLayout L;
   size_t o = 0;
@@ -305,7 +307,7 @@ __host__ __device__ inline GxLayout gx_layout_mb(int n_cls, int n_tr, int LT, in
   L.l2kh = o;
   o += (size_t)LT * 8;
   L.P = o;
-  o += (size_t)GX_TA * (NDIR + 1) * LT * 8;
+  o += (size_t)gx_ta(LT) * (NDIR + 1) * LT * 8;
   L.K = o;
   o += (size_t)mb * n_tr * 2 * (NDIR + 1) * 8;
   L.M = o;
@@ -364,7 +366,8 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
     l2kh[l] = px_log2_d(e, T);
     bad |= !(e > 1e-7 && e < 1e7);
   }
-  const int span = max(a_end - a_begin, 0), nch = (span + GX_TA - 1) / GX_TA, TA = nch ? (span + nch - 1) / nch : 0;
+  const int tm = gx_ta(LT), span = max(a_end - a_begin, 0), nch = (span + tm - 1) / tm;
+  const int TA = nch ? (span + nch - 1) / nch : 0;
   __syncthreads();
   for (int base = a_begin; base < a_end; base += TA) {
     const int tc = min(TA, a_end - base);
@@ -468,20 +471,39 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
   }
 }
 
-// ell per CTA: a power of two up to 32 whose tile fits twice on an SM; nodes per
-// chunk
-void grad_limber64_tile(int n_ell, int n_cls, int* lt, int* ta) {
+// ell per CTA: a power of two up to 32 whose tile fits twice on an SM
+int grad_limber64_tile(int n_ell, int n_cls) {
   int l = 32;
   while (l > 1 && gx_layout_mb(n_cls, n_cls, l, 2).total > 100 * 1024) l >>= 1;
   const int tiles = (n_ell + l - 1) / l;
-  *lt = (n_ell + tiles - 1) / tiles;
-  *ta = GX_TA;
+  return (n_ell + tiles - 1) / tiles;
+}
+
+// Splits of the a nodes, `tiles` ell tiles in all: no more CTAs than fit the SMs at
+// once (two each; 25 tiles x 13 splits, 21 CTAs more than that: 264 us, x 12: 178),
+// or, past that, the least number whose last wave leaves 10% idle (427 tiles:
+// 1,880 us; x 5: 1,812)
+int grad_limber64_split(long long tiles, int na, int lt) {
+  const long long slots = 2LL * 152;
+  const int most = max(1, min(na / gx_ta(lt), 64));
+  if (tiles <= slots) {
+    const int ns = (int)(slots / tiles);
+    return ns < most ? ns : most;
+  }
+  int best = 1;
+  double eff = 0.0;
+  for (int ns = 1; ns <= 8 && ns <= most; ++ns) {
+    const long long c = tiles * ns, w = (c + slots - 1) / slots;
+    const double e = (double)c / (double)(w * slots);
+    if (e > eff + 0.01) best = ns, eff = e;
+    if (eff >= 0.9) break;
+  }
+  return best;
 }
 
 template <bool GEN>
 static void launch_limber64g(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
-  int lt, ta;
-  grad_limber64_tile(gb.n_ell, gb.n_cls, &lt, &ta);
+  const int lt = grad_limber64_tile(gb.n_ell, gb.n_cls);
   const size_t sm = gx_layout(gb.n_cls, gb.n_tr, lt).total;
   cudaFuncSetAttribute(grad_limber64_kernel<GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   grad_limber64_kernel<GEN><<<dim3((gb.n_ell + lt - 1) / lt, gb.n_split, gb.n_items), GX_THREADS, sm, st>>>(gb, c, lt);

@@ -11,7 +11,8 @@
 //
 // One kernel did both, 32 lanes of (node, direction) in Dual<1> float64: the
 // coefficients' exponentials eight times over, the moments on the FP64 pipe.
-// One cosmology, 513 nodes 200 -> @R1@ us, 61 cosmologies 1,260 -> @R61@ us.
+// One cosmology, 513 nodes 200 -> 17 + 26 us, 61 cosmologies 1,260 -> 142 + 128
+// us; the second kernel is bound by the FP64 pipe, the first by issue.
 #include "jcg_grad.cuh"
 #include "jcg_px_node.cuh"
 
@@ -296,8 +297,8 @@ void launch_grad_rows64(const GradBatch& gb, const ConstTables* c, cudaStream_t 
   cudaFuncSetAttribute(grad_moments64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Gr64Smem));
   grad_moments64_kernel<<<dim3((gb.na + nb - 1) / nb, gb.n_items), GR64_WARPS * 32, sizeof(Gr64Smem), st>>>(gb, c, nb,
                                                                                                          only_wide);
-  // two directions a thread while that leaves SMs idle (513 nodes: 8 us against 16
-  // for all eight), all eight from there on (61 cosmologies: 90 us against 150)
+  // two directions a thread while that leaves SMs idle (513 nodes: 26 us against 60
+  // for all eight), all eight from there on (61 cosmologies: 128 us against 228)
   if ((long long)gb.na * gb.n_items * 4 <= 32LL * 4 * device_sm_count())
     grad_rowfin64_kernel<4><<<dim3((gb.na * 4 + 63) / 64, gb.n_items), 64, 0, st>>>(gb, c, only_wide);
   else
