@@ -387,6 +387,19 @@ int jcg_gaussian_covariance(const double* ell_dev, int n_ell, int n_tracers,
                             const double* tracer_noise_dev, int n_cosmo, double f_sky, int sparse,
                             double* out_dev, cudaStream_t stream);
 
+/* Gradient of a scalar in cl_signal from its gradient cov_bar in the covariance
+ * (shapes, noise and `sparse` as above); cl_bar [n_cosmo][n_cls][n_ell].  A dense
+ * cov_bar is read on its per-ell diagonals, where the covariance depends on C_ell. */
+int jcg_gaussian_covariance_vjp(const double* ell_dev, int n_ell, int n_tracers,
+                                const double* cl_signal_dev, const double* cl_noise_dev,
+                                const double* tracer_noise_dev, int n_cosmo, double f_sky, int sparse,
+                                const double* cov_bar_dev, double* cl_bar_dev, cudaStream_t stream);
+/* Gradient of jcg_gaussian_loglike_sparse in its covariance: out_bar [n_cosmo]
+ * times (alpha alpha^T + C^-1) / 2 per ell, with alpha = C^-1 (mu - data) and C^-1
+ * in the sparse format (NULL: without log-determinant); cov_bar_dev may be inv_dev. */
+int jcg_gaussian_loglike_cov_grad(const double* alpha_dev, const double* inv_dev, const double* out_bar_dev,
+                                  int n_cosmo, int n_cls, int n_ell, double* cov_bar_dev, cudaStream_t stream);
+
 /* Gaussian log-likelihood with a covariance in the sparse block format
  * (likelihood.py:9-61; sparse.py:295-366): per-ell blocks factored by
  * Cholesky in float64.  data/mu [n_cosmo][n_cls*n_ell] (p*n_ell + l),

@@ -168,6 +168,20 @@ class _Covariance(torch.autograd.Function):
         s3 = sig if batched else sig[None]
         g = gcov if batched else gcov[None]
         B, n_cls, n_ell = s3.shape
+        if not (torch.is_grad_enabled() and g.requires_grad):
+            cn = None
+            if cl_noise is not None:
+                cn = torch.as_tensor(cl_noise, dtype=torch.float64).to(ell_t.device).expand(n_cls, n_ell).contiguous()
+            tn = None if tracer_noise is None else tracer_noise.to(ell_t.device, torch.float64).contiguous()
+            s3 = s3.detach().to(device=ell_t.device, dtype=torch.float64).contiguous()
+            g = g.to(torch.float64).contiguous()
+            go = torch.empty_like(s3)
+            _lib.call("jcg_gaussian_covariance_vjp", _lib.ptr(ell_t), n_ell, n_tr, _lib.ptr(s3), _lib.ptr(cn),
+                      _lib.ptr(tn), B, ctypes.c_double(float(f_sky)), 1 if sparse else 0, _lib.ptr(g), _lib.ptr(go),
+                      _lib.stream_of(ell_t.device))
+            go = go.to(device=sig.device, dtype=sig.dtype)
+            return (go if batched else go[0]), None, None, None, None, None, None
+        # a graph of the gradient is asked for: in torch operations
         if not sparse:  # the entries that depend on C_ell: the per-ell diagonals of each block
             g4 = g.reshape(B, n_cls, n_ell, n_cls, n_ell)
             idx = torch.arange(n_ell, device=g.device)
@@ -225,7 +239,11 @@ class _LogLike(torch.autograd.Function):
         g_C = None
         if ctx.needs_input_grad[2]:
             B = alpha.shape[0]
-            if sparse:
+            if sparse and not (torch.is_grad_enabled() and gout.requires_grad):
+                g_C = _sparse_inv_batched(C) if include_logdet else torch.empty_like(C)
+                _lib.call("jcg_gaussian_loglike_cov_grad", _lib.ptr(alpha), _lib.ptr(g_C) if include_logdet else None,
+                          _lib.ptr(go.contiguous()), B, n_cls, n_ell, _lib.ptr(g_C), _lib.stream_of(C.device))
+            elif sparse:
                 a3 = alpha.reshape(B, n_cls, n_ell)
                 g = torch.einsum("bpl,bql->bpql", a3, a3)
                 if include_logdet:

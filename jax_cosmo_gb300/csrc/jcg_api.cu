@@ -15,6 +15,11 @@
 #include "jcg_grad.cuh"
 
 namespace jcg {
+void launch_covariance_vjp(const double* ell, int n_ell, int n_tr, const double* cl, const double* cl_noise,
+                           const double* tr_noise, int n_cosmo, double f_sky, int sparse, const double* g, double* out,
+                           cudaStream_t st);
+void launch_loglike_cov_grad(const double* alpha, const double* inv, const double* go, int n_cosmo, int n_cls,
+                             int n_ell, double* out, cudaStream_t st);
 void launch_covariance(const double* ell, int n_ell, int n_tr, const double* cl,
                        const double* cl_noise, const double* tr_noise, int n_cosmo, double f_sky,
                        int sparse, double* out, cudaStream_t st);
@@ -605,6 +610,27 @@ int jcg_gaussian_covariance(const double* ell, int n_ell, int n_tr, const double
   launch_covariance(ell, n_ell, n_tr, cl, cl_noise, tr_noise, n_cosmo, f_sky, sparse ? 1 : 0, out,
                     stream);
   return cuda_check("covariance");
+}
+
+int jcg_gaussian_covariance_vjp(const double* ell, int n_ell, int n_tr, const double* cl,
+                                const double* cl_noise, const double* tr_noise, int n_cosmo, double f_sky,
+                                int sparse, const double* cov_bar, double* cl_bar, cudaStream_t stream) {
+  if (!ell || !cl || !cov_bar || !cl_bar) return fail(JCG_ERR_ARG, "NULL pointer");
+  if (n_cosmo < 1) return fail(JCG_ERR_SHAPE, "n_cosmo = %d", n_cosmo);
+  if (n_tr < 1 || n_tr > JCG_MAX_TRACERS) return fail(JCG_ERR_SHAPE, "n_tracers = %d", n_tr);
+  if (n_ell < 2) return fail(JCG_ERR_SHAPE, "np.gradient needs at least 2 ell values (n_ell = %d)", n_ell);
+  if (!isfinite(f_sky)) return fail(JCG_ERR_VALUE, "f_sky = %g", f_sky);
+  launch_covariance_vjp(ell, n_ell, n_tr, cl, cl_noise, tr_noise, n_cosmo, f_sky, sparse ? 1 : 0, cov_bar, cl_bar,
+                        stream);
+  return cuda_check("covariance gradient");
+}
+
+int jcg_gaussian_loglike_cov_grad(const double* alpha, const double* inv, const double* out_bar, int n_cosmo,
+                                  int n_cls, int n_ell, double* cov_bar, cudaStream_t stream) {
+  if (!alpha || !out_bar || !cov_bar) return fail(JCG_ERR_ARG, "NULL pointer");
+  if (n_cosmo < 1 || n_cls < 1 || n_ell < 1) return fail(JCG_ERR_SHAPE, "bad sizes");
+  launch_loglike_cov_grad(alpha, inv, out_bar, n_cosmo, n_cls, n_ell, cov_bar, stream);
+  return cuda_check("loglike covariance gradient");
 }
 
 int jcg_loglike_workspace_size(int n_cosmo, int n_cls, int n_ell, size_t* bytes) {

@@ -127,6 +127,77 @@ void launch_covariance(const double* ell, int n_ell, int n_tr, const double* cl,
                                                                      f_sky, out);
 }
 
+// Gradient of the covariance in C_ell.  C_pq with p = (i, j), q = (m, n) is
+// (O_im O_jn + O_in O_jm) / norm, so for the spectrum (x, y) the sum over its
+// places in all blocks is, over ordered (u, v) = (x, y) and (y, x) and all tracers
+// s, t,   (1 + [s = u]) (1 + [t = v]) g_{(u s), (v t)} O_st / norm.
+// A CTA per spectrum and cosmology, threads over ell: each entry of g that
+// contributes is read once or twice, in whole lines in the sparse form.  Scatters
+// by index (four index_add of n_cls^2 n_ell products, and a host copy of ell) took
+// 25 launches and two waits on the device.
+__global__ void __launch_bounds__(128)
+    covariance_vjp_kernel(const double* __restrict__ ell, int n_ell, int n_tr, const double* __restrict__ cl,
+                          const double* __restrict__ cl_noise, const double* __restrict__ tr_noise, int n_cosmo,
+                          double f_sky, int sparse, const double* __restrict__ g, double* __restrict__ out) {
+  const int n_cls = n_tr * (n_tr + 1) / 2;
+  const int2 xy = pair_of(blockIdx.x, n_tr);
+  const size_t N = (size_t)n_cls * n_ell;
+  for (int ci = blockIdx.y; ci < n_cosmo; ci += gridDim.y) {
+    const double* sig = cl + (size_t)ci * N;
+    const double* gc = g + (size_t)ci * (sparse ? (size_t)n_cls : N) * N;
+    for (int l = threadIdx.x; l < n_ell; l += blockDim.x) {
+      double sum = 0.0;
+      for (int o = 0; o < (xy.x == xy.y ? 1 : 2); ++o) {
+        const int u = o ? xy.y : xy.x, v = o ? xy.x : xy.y;
+        for (int s = 0; s < n_tr; ++s) {
+          const int p = pair_index(u, s, n_tr);
+          const double* row = sparse ? gc + (size_t)p * N + l : gc + ((size_t)p * n_ell + l) * N + l;
+          double part = 0.0;
+          for (int t = 0; t < n_tr; ++t) {
+            const double w = row[(size_t)pair_index(v, t, n_tr) * n_ell] *
+                             cl_obs(sig, cl_noise, tr_noise, pair_index(s, t, n_tr), l, n_ell, n_tr);
+            part += t == v ? 2.0 * w : w;
+          }
+          sum += s == u ? 2.0 * part : part;
+        }
+      }
+      out[(size_t)ci * N + (size_t)blockIdx.x * n_ell + l] =
+          sum / ((2.0 * ell[l] + 1.0) * ell_gradient(ell, n_ell, l) * f_sky);
+    }
+  }
+}
+
+void launch_covariance_vjp(const double* ell, int n_ell, int n_tr, const double* cl, const double* cl_noise,
+                           const double* tr_noise, int n_cosmo, double f_sky, int sparse, const double* g, double* out,
+                           cudaStream_t st) {
+  const int n_cls = n_tr * (n_tr + 1) / 2;
+  covariance_vjp_kernel<<<dim3(n_cls, (unsigned)(n_cosmo < 65535 ? n_cosmo : 65535)), 128, 0, st>>>(
+      ell, n_ell, n_tr, cl, cl_noise, tr_noise, n_cosmo, f_sky, sparse, g, out);
+}
+
+// Gradient of the log-likelihood in the sparse covariance, go / 2 (a a^T + C^-1)
+// with a = C^-1 r, in place of C^-1 where out = inv: a CTA per (p, q) and cosmology
+__global__ void __launch_bounds__(128)
+    loglike_cov_grad_kernel(const double* __restrict__ alpha, const double* inv, const double* __restrict__ go,
+                            int n_cosmo, int n_cls, int n_ell, double* out) {
+  const int p = blockIdx.x / n_cls, q = blockIdx.x - p * n_cls;
+  for (int ci = blockIdx.y; ci < n_cosmo; ci += gridDim.y) {
+    const double* a = alpha + (size_t)ci * n_cls * n_ell;
+    const size_t o = ((size_t)ci * n_cls * n_cls + blockIdx.x) * n_ell;
+    const double h = 0.5 * go[ci];
+    for (int l = threadIdx.x; l < n_ell; l += blockDim.x) {
+      const double v = a[(size_t)p * n_ell + l] * a[(size_t)q * n_ell + l];
+      out[o + l] = h * (inv ? v + inv[o + l] : v);
+    }
+  }
+}
+
+void launch_loglike_cov_grad(const double* alpha, const double* inv, const double* go, int n_cosmo, int n_cls,
+                             int n_ell, double* out, cudaStream_t st) {
+  loglike_cov_grad_kernel<<<dim3(n_cls * n_cls, (unsigned)(n_cosmo < 65535 ? n_cosmo : 65535)), 128, 0, st>>>(
+      alpha, inv, go, n_cosmo, n_cls, n_ell, out);
+}
+
 // ---------------------------------------- symmetric blocks in registers -----
 // A symmetric n x n block is kept as its lower triangle, column by column, in the
 // registers of a CTA: element e = tid + m * THREADS of the triangle with R extra
