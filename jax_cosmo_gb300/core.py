@@ -99,8 +99,20 @@ class Cosmology:
         """[B, 8] float64 tensor on ``device`` (B = 1 for a single cosmology);
         [B, 9] with gamma last when the growth is parametrised by gamma."""
         B = self.batch_size or 1
+        params = self.param_list()
+        # host values go up in one copy (a copy of pageable memory waits for the
+        # device, some 35 us each)
+        host = {i: np.asarray(v, dtype=np.float64) for i, v in enumerate(params) if not isinstance(v, torch.Tensor)}
+        if host and all(h.ndim == 0 or h.size == B for h in host.values()):
+            up = np.empty((B, len(host)))
+            for c, h in enumerate(host.values()):
+                up[:, c] = h.reshape(-1)
+            up = torch.as_tensor(up, device=device)
+            if len(host) == len(params):
+                return self._checked(up)
+            params = [up[:, list(host).index(i)] if i in host else v for i, v in enumerate(params)]
         cols = []
-        for v in self.param_list():
+        for v in params:
             if isinstance(v, torch.Tensor):
                 t = v.to(device=device, dtype=torch.float64)
                 if not differentiable:
@@ -110,7 +122,10 @@ class Cosmology:
             if t.dim() == 0:
                 t = t.expand(B)
             cols.append(t.reshape(B))
-        p = torch.stack(cols, dim=1).contiguous()
+        return self._checked(torch.stack(cols, dim=1).contiguous())
+
+    @staticmethod
+    def _checked(p):
         if p.device.type == "cpu":
             if not bool(torch.isfinite(p.detach()).all()):
                 raise ValueError("Cosmology parameters must be finite")
