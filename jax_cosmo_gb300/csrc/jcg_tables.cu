@@ -390,22 +390,21 @@ void launch_geometry_build(const GeoHeader& h, double* geo, const double* pz, co
 
 // ------------------------------------------------------ cosmology tables ----
 
-// NW: some item may use the transfer type "eisenhu" (a separate
-// instantiation keeps the default one's registers).  FAST (fp32c): the
-// per-node evaluations (chi and growth right-hand sides, the Romberg
-// integrand, P(k) k^3) in float-pair arithmetic on the FP32 pipe; the scans,
-// sigma8's weighted sum and the tables' values stay float64.  Most phases
-// keep one or two warps of a block busy, so the fp32c form is held to 64
-// registers: four blocks per SM overlap their phases.
-template <bool NW, bool FAST>
-__global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch bt, const ConstTables* __restrict__ c) {
+// The fp32c tables.  NW: some item may use the transfer type "eisenhu" (a
+// separate instantiation keeps the default one's registers).  The per-node
+// evaluations (chi and growth right-hand sides, the Romberg integrand, P(k) k^3)
+// are in float-pair arithmetic on the FP32 pipe; the scans, sigma8's weighted
+// sum and the tables' values stay float64.  Most phases keep one or two warps of
+// a block busy: held to 64 registers, four blocks per SM overlap their phases.
+template <bool NW>
+__global__ void __launch_bounds__(256, 4) cosmo_tables_kernel(Batch bt, const ConstTables* __restrict__ c) {
   const int item = blockIdx.x;
   if (item >= bt.n_items) return;
   const Item it = batch_item(bt, item);
   __shared__ double s[NSCAL];
   __shared__ double inc[NCHI];
   __shared__ double fnode[NCHI];
-  __shared__ double pq[NKH];
+  __shared__ FF pk3ff[NKH];         // P(k) k^3 as pairs
   __shared__ double qa[NGROW], ra[NGROW], qm[NGROW], rm[NGROW];
   __shared__ double fr[NROMB];
   __shared__ double pk3[NKH];
@@ -413,28 +412,23 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   __shared__ double gs[NGROW];
   __shared__ double mv[4 * NGROW];  // per-step growth matrices
   __shared__ double yv[2 * NGROW];  // growth ODE solution (D, dD/da) unnormalised
-  __shared__ float2 wpp[NKH];       // fp32c: w pk3 as float pairs
-  __shared__ FF sff[FAST ? NSCAL : 1];                  // fp32c: the scalars as pairs
-  __shared__ float2 e2s[FAST ? 64 : 1], scs[FAST ? 256 : 1];  // tables of the pair exp and sin
-  FF* pk3ff = reinterpret_cast<FF*>(pq);                // fp32c: P(k) k^3 as pairs (pq is free until then)
+  __shared__ float2 wpp[NKH];       // w pk3 as float pairs
+  __shared__ FF sff[NSCAL];         // the scalars as pairs
+  __shared__ float2 e2s[64], scs[256];  // tables of the pair exp and sin
   const int t = threadIdx.x;
   for (int i = t; i < NSCAL; i += blockDim.x) {
     s[i] = it.ctab->s[i];  // from cosmo_scalars_kernel
-    if (FAST) sff[i] = ff_of(s[i]);
+    sff[i] = ff_of(s[i]);
   }
-  if (FAST) {
-    for (int i = t; i < 64; i += blockDim.x) e2s[i] = c->exp2_ff[i];
-    for (int i = t; i < 256; i += blockDim.x) scs[i] = c->sincos_ff[i];
-  }
+  for (int i = t; i < 64; i += blockDim.x) e2s[i] = c->exp2_ff[i];
+  for (int i = t; i < 256; i += blockDim.x) scs[i] = c->sincos_ff[i];
   __syncthreads();
-  const Bg bg = make_bg(s);
   const auto F2 = [](float2 v) { return FF{v.x, v.y}; };
-  BgF bgf;
-  if (FAST) bgf = BgF{sff[S_OMEGA_M], sff[S_OMEGA_K], sff[S_OMEGA_DE], sff[S_W0], sff[S_WA]};
+  const BgF bgf{sff[S_OMEGA_M], sff[S_OMEGA_K], sff[S_OMEGA_DE], sff[S_W0], sff[S_WA]};
   // chi RK4 in ln a (background.py:227-231, scipy/ode.py:11-19): the
   // right-hand side does not depend on chi, so each step needs f at its two
   // ends (shared with the neighbouring steps) and at its midpoint.
-  if (FAST) {
+  {
     if (t < NCHI) {
       fnode[t] = ffd(ff_dchi_dlna(bgf, F2(c->chi_a_ff[t]), F2(c->lna_chi_ff[t]), F2(c->chi_ia_ff[t]), e2s));
       if (t > 0) inc[t] = ffd(ff_dchi_dlna(bgf, F2(c->chi_am_ff[t]), F2(c->chi_lnam_ff[t]), F2(c->chi_iam_ff[t]), e2s));
@@ -452,23 +446,6 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
       const FF logk = F2(c->romb_logk_ff[t]);
       const FF T = ff_eh_transfer<NW>(sff, F2(c->romb_k_ff[t]), logk, F2(c->romb_ik_ff[t]), s[S_TFNW] != 0.0, e2s, scs);
       fr[t] = ffd(F2(c->romb_kw2_ff[t]) * (ff_sqr(T) * ff_exp(sff[S_NS] * logk, e2s)));
-    }
-  } else {
-    if (t < NCHI) {
-      fnode[t] = dchi_dlna_c(bg, c->chi_a[t], c->lna_chi[t], c->chi_ia[t]);
-      if (t > 0) inc[t] = dchi_dlna_c(bg, c->chi_am[t], c->chi_lnam[t], c->chi_iam[t]);
-    }
-    // growth ODE coefficients at nodes and midpoints
-    if (t < NGROW) {
-      growth_qr_c(bg, c->atab_grow[t], c->grow_lna[t], c->grow_ia[t], qa[t], ra[t]);
-      if (t > 0) growth_qr_c(bg, c->grow_am[t], c->grow_lnam[t], c->grow_iam[t], qm[t], rm[t]);
-    }
-    // sigmasqr(8) integrand at the romb nodes (power.py:70-75): the window
-    // factor k (k W(8k))^2 is a constant of the node
-    if (t < NROMB) {
-      const double logk = c->romb_logk[t];
-      const double T = eh_transfer_lki<NW>(s, c->romb_k[t], logk, c->romb_ik[t]);
-      fr[t] = c->romb_kw2[t] * ((T * T) * exp(s[S_NS] * logk));
     }
   }
   __syncthreads();
@@ -490,7 +467,7 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   }
   const int warp = t >> 5, lane = t & 31;
   if (warp == 0) {
-    chi_scan_warp<!FAST>(fnode, inc, c->lna_chi, lane, chis);
+    chi_scan_warp<false>(fnode, inc, c->lna_chi, lane, chis);
   } else if (warp == 2) {
     // sigmasqr(8) (power.py:70-78): romb is linear in the integrand values,
     // sum_e w_e f_e with the weights of its Richardson combination
@@ -524,7 +501,7 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   }
   __syncthreads();
   // linear P(k_i, a = 1) * k_i^3 on the halofit k grid (power.py:102, 124)
-  if (FAST) {
+  {
     const FF g1 = ff_of(s[S_G1]);
     const FF fac = ff_sqr(g1) * ff_of(s[S_PKNORM]);  // sigma8^2 / sigmasqr(8), set above
     for (int i = t; i < NKH; i += blockDim.x) {
@@ -537,27 +514,13 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
       wpp[i] = make_float2(w.hi, w.lo);
       pk3ff[i] = p;
     }
-  } else {
-    for (int i = t; i < NKH; i += blockDim.x) {
-      const double tk = eh_transfer_lki<NW>(s, c->kh[i], c->logk[i], c->ikh[i]);
-      const double g1 = s[S_G1];
-      pk3[i] = exp(s[S_NS] * c->logk[i]) * (tk * tk) * (g1 * g1) * s[S_PKNORM] * c->kh3[i];
-    }
   }
   __syncthreads();
-  // sigma^2(R_j) without g^2: simps over ln k of pk k^3 exp(-(k R)^2) / (2 pi^2),
-  // with the Simpson weights and 1 / (2 pi^2) folded into the k-node factor:
-  // one FMA per (k, R) term
-  if (!FAST) {
-    for (int i = t; i < NKH; i += blockDim.x) {
-      pq[i] = c->simpson_kh[i] * (pk3[i] / (2.0 * (PI * PI)));
-      it.ctab->rtay[0][i] = f2_of(pq[i]);  // as a pair, for the moments of the float64 rows
-    }
-    __syncthreads();
-  }
   CosmoTab* out = it.ctab;
-  if (FAST) {
-    // fp32c: the same sums in float-pair arithmetic (about 1e-13 relative, all
+  // sigma^2(R_j) without g^2: simps over ln k of pk k^3 exp(-(k R)^2) / (2 pi^2),
+  // with the Simpson weights and 1 / (2 pi^2) folded into the k-node factor
+  {
+    // in float-pair arithmetic (about 1e-13 relative, all
     // terms positive): the FP32 pipe instead of the 1/64-rate FP64 one; the
     // halofit root find on this table then takes the same nodes as with
     // float64 sums except within ~1e-13 of a decision boundary
@@ -567,26 +530,16 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
       out->sig[j] = (double)ah + (double)al;
     }
     __syncthreads();
-  } else {
-    for (int j = t; j < NRT; j += blockDim.x) {
-      double acc = 0.0;
-      for (int i = 0; i < NKH; ++i) acc = fma(pq[i], c->E[i * NRT + j], acc);
-      out->sig[j] = acc;
-    }
   }
   for (int i = t; i < NSCAL; i += blockDim.x) out->s[i] = s[i];
   for (int i = t; i < NCHI; i += blockDim.x) {
     // segment [i, i+1] slope of the chi table: the `a` of scipy/interpolate.py:55
-    // (fp32c: times the reciprocal of the node spacing)
-    const double sl = (i < NCHI - 1)
-                          ? (FAST ? (chis[i + 1] - chis[i]) * c->chi_ida[i]
-                                  : (chis[i + 1] - chis[i]) / (c->atab_chi[i + 1] - c->atab_chi[i]))
-                          : 0.0;
+    const double sl = (i < NCHI - 1) ? (chis[i + 1] - chis[i]) * c->chi_ida[i] : 0.0;
     out->chi_slope[i] = sl;
     out->chi32[i] = (float)chis[i];
     out->slope32[i] = (float)sl;
   }
-  if (FAST) {
+  {
     // fp32c halofit moments: w pk3 as float pairs (float copy for the exp
     // terms), then the Taylor tables by the contracting recurrence
     // Q_m[i + 1] = (Q_m[i] + w_i pk3_i) rho_m in float pairs, one lane per m
@@ -624,6 +577,158 @@ __global__ void __launch_bounds__(256, FAST ? 4 : 3) cosmo_tables_kernel(Batch b
   // recurrences (warp 0) leave idle
   if (t == 32) make_eh32(s, &out->eh32);
 }
+
+// The float64 tables, in three launches:
+//   tables_nodes64_kernel    Eisenstein-Hu at the Romberg and P(k) nodes, the chi
+//     right-hand sides, the growth steps' matrices: a node or step per thread,
+//     CTAs of a warp;
+//   tables_scan64_kernel     the scans, sigma8, P(k) k^3 (a CTA per cosmology);
+//   tables_sigma64_kernel    sigma^2(R), quarters of the R grid, four threads per R.
+// A node is 400 float64 operations in a row, and the FP64 pipe takes 64 cycles per
+// warp of them: one CTA per cosmology had two or three warps queue on each
+// scheduler, twice.  One cosmology 84 -> 32 us (11 + 15 + 7), 4096
+// 1.68 -> 1.65 ms.
+// Node values between the launches: in the part of rtay that only fp32c uses.
+struct Tab64 {
+  double fn[NCHI], fm[NCHI], M[4 * NGROW], u[NROMB + NKH], pq[NKH];
+};
+static_assert(sizeof(Tab64) <= sizeof(float2) * (NTAYLOR - 1) * (NKH + 1), "node values fit");
+__device__ __forceinline__ Tab64* tab64_of(CosmoTab* t) { return reinterpret_cast<Tab64*>(t->rtay[1]); }
+static_assert(offsetof(CosmoTab, rtay) % 8 == 0 && sizeof(float2) * (NKH + 1) % 8 == 0, "node values aligned");
+
+// M of one RK4 step of the growth equation, y_i = M y_{i-1} with y = (D, dD/da)
+// (jcg_grad64.cu has it with tangents)
+__device__ __forceinline__ void growth_step_matrix(double h, double q0, double r0, double qm, double rm, double q1,
+                                                   double r1, double* M) {
+  const double h2 = 0.5 * h, h6 = h / 6.0;
+  const double X2[4] = {1.0, h2, h2 * r0, 1.0 - h2 * q0};
+  const double K2[4] = {X2[2], X2[3], rm * X2[0] - qm * X2[2], rm * X2[1] - qm * X2[3]};
+  const double X3[4] = {1.0 + h2 * K2[0], h2 * K2[1], h2 * K2[2], 1.0 + h2 * K2[3]};
+  const double K3[4] = {X3[2], X3[3], rm * X3[0] - qm * X3[2], rm * X3[1] - qm * X3[3]};
+  const double X4[4] = {1.0 + h * K3[0], h * K3[1], h * K3[2], 1.0 + h * K3[3]};
+  M[0] = 1.0 + h6 * (2.0 * (K2[0] + K3[0]) + X4[2]);
+  M[1] = h6 * (1.0 + 2.0 * (K2[1] + K3[1]) + X4[3]);
+  M[2] = h6 * (r0 + 2.0 * (K2[2] + K3[2]) + (r1 * X4[0] - q1 * X4[2]));
+  M[3] = 1.0 + h6 * (-q0 + 2.0 * (K2[3] + K3[3]) + (r1 * X4[1] - q1 * X4[3]));
+}
+
+constexpr int T64_EH = (NROMB + NKH + 31) / 32, T64_CHI = 2 * NCHI / 32, T64_GROW = NGROW / 32;
+constexpr int T64_JOBS = T64_EH + T64_CHI + T64_GROW;  // CTAs per cosmology
+__global__ void __launch_bounds__(32) tables_nodes64_kernel(Batch bt, const ConstTables* __restrict__ c) {
+  const Item it = batch_item(bt, blockIdx.x / T64_JOBS);
+  const double* s = it.ctab->s;
+  Tab64* o = tab64_of(it.ctab);
+  const int b = blockIdx.x % T64_JOBS, lane = threadIdx.x;
+  if (b < T64_EH) {
+    const int e = b * 32 + lane;
+    if (e >= NROMB + NKH) return;
+    // sigmasqr(8)'s integrand (power.py:70-75; the window factor is a constant of the
+    // node), or k^{n_s} T^2
+    const bool romb = e < NROMB;
+    const int i = romb ? e : e - NROMB;
+    const double lk = romb ? c->romb_logk[i] : c->logk[i];
+    const double T = eh_transfer_lki<true>(s, romb ? c->romb_k[i] : c->kh[i], lk, romb ? c->romb_ik[i] : c->ikh[i]);
+    const double v = (T * T) * exp(s[S_NS] * lk);
+    o->u[e] = romb ? c->romb_kw2[i] * v : v;
+    return;
+  }
+  const Bg bg = make_bg(s);
+  if (b < T64_EH + T64_CHI) {
+    const int e = (b - T64_EH) * 32 + lane;
+    if (e < NCHI) o->fn[e] = dchi_dlna_c(bg, c->chi_a[e], c->lna_chi[e], c->chi_ia[e]);
+    else if (e > NCHI) o->fm[e - NCHI] = dchi_dlna_c(bg, c->chi_am[e - NCHI], c->chi_lnam[e - NCHI], c->chi_iam[e - NCHI]);
+    return;
+  }
+  const int i = (b - T64_EH - T64_CHI) * 32 + lane;
+  double M[4] = {1.0, 0.0, 0.0, 1.0};
+  if (i > 0) {
+    double q0, r0, qm, rm, q1, r1;
+    growth_qr_c(bg, c->atab_grow[i - 1], c->grow_lna[i - 1], c->grow_ia[i - 1], q0, r0);
+    growth_qr_c(bg, c->grow_am[i], c->grow_lnam[i], c->grow_iam[i], qm, rm);
+    growth_qr_c(bg, c->atab_grow[i], c->grow_lna[i], c->grow_ia[i], q1, r1);
+    growth_step_matrix(c->atab_grow[i] - c->atab_grow[i - 1], q0, r0, qm, rm, q1, r1, M);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o->M[4 * i + q] = M[q];
+}
+
+constexpr int TS64_THREADS = 128;
+__global__ void __launch_bounds__(TS64_THREADS) tables_scan64_kernel(Batch bt, const ConstTables* __restrict__ c) {
+  const Item it = batch_item(bt, blockIdx.x);
+  CosmoTab* out = it.ctab;
+  Tab64* n = tab64_of(out);
+  __shared__ double mv[4 * NGROW], yv[2 * NGROW], fn[NCHI], fm[NCHI], chis[NCHI], gs[NGROW], sc[3];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  for (int i = t; i < 4 * NGROW; i += TS64_THREADS) mv[i] = n->M[i];
+  for (int i = t; i < NCHI; i += TS64_THREADS) fn[i] = n->fn[i], fm[i] = n->fm[i];
+  __syncthreads();
+  if (warp == 0) {
+    chi_scan_warp<true>(fn, fm, c->lna_chi, lane, chis);
+  } else if (warp == 1) {
+    double d4[4];
+    const double yf = growth_scan_warp(mv, c->atab_grow[0], 1.0, lane, d4, yv);
+    for (int k = 0; k < 4; ++k) {
+      const int i = lane * 4 + k;
+      const double g = d4[k] / yf;
+      gs[i] = g;
+      out->g[i] = g;
+      // dlnD/dlna = a / D dD/da (background.py:484-485)
+      out->f[i] = yv[2 * i + 1] / yf * c->atab_grow[i] / g;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      // growth_factor(1.0) (power.py:44 with the default a = 1)
+      const int2 sg = interp_segment_inc(1.0, c->atab_grow, NGROW, NGROW - 1);
+      sc[2] = clip_lohi(interp_eval(1.0, c->atab_grow, gs, sg), 0.0, 1.0);
+    }
+  } else if (warp == 2) {
+    // sigmasqr(8) (power.py:70-78): romb is linear in the integrand values,
+    // sum_e w_e f_e with the weights of its Richardson combination
+    double acc = 0.0;
+    for (int e = lane; e < NROMB; e += 32) acc = fma(c->romb_w[e], n->u[e], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+      const double s8 = out->s[S_SIGMA8];
+      sc[0] = 1.0 / (2.0 * (PI * PI)) * acc;
+      sc[1] = (s8 * s8) / sc[0];
+    }
+  }
+  __syncthreads();
+  if (t == 0) out->s[S_SIGMASQR8] = sc[0], out->s[S_PKNORM] = sc[1], out->s[S_G1] = sc[2];
+  // linear P(k_i, a = 1) k_i^3 (power.py:102, 124), the moments' weights
+  const double pn = (sc[2] * sc[2]) * sc[1];
+  for (int i = t; i < NKH; i += TS64_THREADS) {
+    const double p = n->u[NROMB + i] * pn * c->kh3[i], w = c->simpson_kh[i] * (p / (2.0 * (PI * PI)));
+    out->pk3[i] = p;
+    n->pq[i] = w;
+    out->rtay[0][i] = f2_of(w);  // as a pair, for the moments of the float64 rows
+  }
+  for (int i = t; i < NCHI; i += TS64_THREADS) {
+    // segment [i, i+1] slope of the chi table: the `a` of scipy/interpolate.py:55
+    const double sl = (i < NCHI - 1) ? (chis[i + 1] - chis[i]) / (c->atab_chi[i + 1] - c->atab_chi[i]) : 0.0;
+    out->chi[i] = chis[i];
+    out->chi_slope[i] = sl;
+  }
+}
+
+// sigma^2(R_j) without g^2: simps over ln k of pk k^3 exp(-(k R)^2) / (2 pi^2), one
+// FMA per (k, R) term
+__global__ void __launch_bounds__(256) tables_sigma64_kernel(Batch bt, const ConstTables* __restrict__ c) {
+  const Item it = batch_item(bt, blockIdx.x / 4);
+  const Tab64* n = tab64_of(it.ctab);
+  __shared__ double pq[NKH], part[4][64];
+  const int t = threadIdx.x, q = t >> 6, jj = t & 63, j = (blockIdx.x & 3) * 64 + jj;
+  for (int i = t; i < NKH; i += 256) pq[i] = n->pq[i];
+  __syncthreads();
+  double acc = 0.0;
+#pragma unroll 8
+  for (int i = q; i < NKH; i += 4) acc = fma(pq[i], c->E[i * NRT + j], acc);
+  part[q][jj] = acc;
+  __syncthreads();
+  if (q == 0) it.ctab->sig[j] = (part[0][jj] + part[1][jj]) + (part[2][jj] + part[3][jj]);
+}
+static_assert(NRT == 4 * 64, "quarters of the R grid");
 
 // The scalars, one half warp per cosmology: the independent pow / sqrt /
 // log calls of each level of the chain on different lanes at once
@@ -695,12 +800,15 @@ __global__ void __launch_bounds__(128) growth_gamma_kernel(Batch bt, const Const
 
 void launch_cosmo_tables(const Batch& b, const ConstTables* c, cudaStream_t st) {
   cosmo_scalars_kernel<<<(b.n_items + 7) / 8, 128, 0, st>>>(b);
-  if (tf_nowiggle(b.physics_or))
-    b.precision == JCG_FP32C ? cosmo_tables_kernel<true, true><<<b.n_items, 256, 0, st>>>(b, c)
-                             : cosmo_tables_kernel<true, false><<<b.n_items, 256, 0, st>>>(b, c);
-  else
-    b.precision == JCG_FP32C ? cosmo_tables_kernel<false, true><<<b.n_items, 256, 0, st>>>(b, c)
-                             : cosmo_tables_kernel<false, false><<<b.n_items, 256, 0, st>>>(b, c);
+  if (b.precision != JCG_FP32C) {
+    tables_nodes64_kernel<<<(unsigned)b.n_items * T64_JOBS, 32, 0, st>>>(b, c);
+    tables_scan64_kernel<<<b.n_items, TS64_THREADS, 0, st>>>(b, c);
+    tables_sigma64_kernel<<<(unsigned)b.n_items * 4, 256, 0, st>>>(b, c);
+  } else if (tf_nowiggle(b.physics_or)) {
+    cosmo_tables_kernel<true><<<b.n_items, 256, 0, st>>>(b, c);
+  } else {
+    cosmo_tables_kernel<false><<<b.n_items, 256, 0, st>>>(b, c);
+  }
   if (growth_gamma(b.physics_or)) growth_gamma_kernel<<<b.n_items, 128, 0, st>>>(b, c);
 }
 
