@@ -5,16 +5,16 @@
 // One CTA per cosmology with one tangent direction per lane spent 1.45 ms on
 // them: 1,154 node evaluations on one SM's FP64 pipe (2 lanes per clock), the
 // value repeated in every direction, then serial scans by single lanes.  Here
-//   grad_eh64_kernel      Eisenstein-Hu at the 386 Romberg and P(k) nodes, one
-//     node per thread, CTAs of a warp: T and its partials in the 11 inputs by a
-//     reverse sweep, then the 8 directions by one product each;
-//   grad_bg64_kernel      the chi and growth nodes by thread, tangents in closed
-//     form; chi by suffix sums, growth by scans of the RK4 steps' matrices and of
+//   grad_nodes64_kernel   a node or step per thread, CTAs of a warp: Eisenstein-Hu at
+//     the 386 Romberg and P(k) nodes, T and its partials in 12 inputs by a reverse
+//     sweep, then the 8 directions by one product each; chi's increments, and the
+//     growth steps' matrices for two directions a thread, tangents in closed form;
+//   grad_bg64_kernel      chi by suffix sums, growth by scans of the matrices and of
 //     their tangents' affine maps, a warp per component;
 //   grad_sigma64_kernel   sigma8's weighted sum, P(k) k^3 and sigma^2(R): a CTA per
 //     component and quarter of the R nodes.
-// One cosmology 1,453 -> 119 us (75 + 23 + 21), 61 cosmologies 1,456 -> 210 us; what is left is
-// latency: serial float64 code of a thread, the scans and 257 loads of E per R.
+// One cosmology 1,453 -> 57 us (23 + 23 + 11); what is left is latency: serial float64 code of
+// a thread and the scans.
 #include "jcg_grad.cuh"
 #include "jcg_px.cuh"
 
@@ -98,9 +98,7 @@ __device__ EhGrad eh_grad_nowiggle(const double* s, double k) {
   return g;
 }
 
-__global__ void __launch_bounds__(32) grad_eh64_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
-  const GradItem gi = grad_item(gb, blockIdx.y);
-  TabD* tb = gi.tab;
+__device__ __forceinline__ void eh_nodes64(TabD* tb, const ConstTables* c, int job) {
   __shared__ double s[NSCAL];
   // d ln x of the scalars above (d x of f_b, f_c and n_s), per direction
   constexpr int NX = 13;
@@ -125,7 +123,7 @@ __global__ void __launch_bounds__(32) grad_eh64_kernel(GradBatch gb, const Const
     dl[x][d] = si == S_FB || si == S_FC || si == S_NS ? t : t == 0.0 ? 0.0 : t / v;
   }
   __syncwarp();
-  const int e = blockIdx.x * 32 + lane;
+  const int e = job * 32 + lane;
   if (e >= NEH) return;
   const bool romb = e < NROMB;
   const int i = romb ? e : e - NROMB;
@@ -148,21 +146,30 @@ __global__ void __launch_bounds__(32) grad_eh64_kernel(GradBatch gb, const Const
 }
 
 // -------------------------------------------------------------- background --
-constexpr int BG64_THREADS = 512;
-constexpr int BG64_SMEM = (int)sizeof(double) * ((NDIR + 1) * (2 * NCHI + 4 * NGROW) + NSCAL * (NDIR + 1) + 2 * NGROW);
-
-// E^2 with its tangents: values shared by the chi and growth nodes
-struct E2D {
-  double e2, ef, d[NDIR], def[NDIR];
+// chi increments and growth step matrices with tangents, between the nodes' kernel
+// and the scans: in the place of tables that are written later
+struct Bg64 {  // over sigv .. pk3d
+  double M[NGROW][4], dM[NDIR][NGROW][4];
 };
-__device__ __forceinline__ E2D e2_grad(const double* s, const double* sd, double a, double lna, double ia) {
-  E2D r;
+static_assert(sizeof(Bg64) <= sizeof(double) * (NDIR + 1) * (NRT + NKH), "matrices fit");
+__device__ __forceinline__ Bg64* bg_scratch(TabD* t) { return reinterpret_cast<Bg64*>(t->sigv); }
+static_assert(offsetof(TabD, pk3d) - offsetof(TabD, sigv) == sizeof(double) * ((NDIR + 1) * NRT + NKH), "contiguous");
+__device__ __forceinline__ double* inc_scratch(TabD* t) { return reinterpret_cast<double*>(grad_kw64(t)); }  // [9][NCHI]
+
+// E^2 with the tangents of ND directions
+template <int ND>
+struct E2D {
+  double e2, ef, d[ND], def[ND];
+};
+template <int ND>
+__device__ __forceinline__ E2D<ND> e2_grad(const double* s, const double* sd, double a, double lna, double ia) {
+  E2D<ND> r;
   const double f = -3.0 * (1.0 + s[S_W0] + s[S_WA]) * lna + 3.0 * s[S_WA] * (a - 1.0);
   r.ef = exp(f);
   const double ia2 = ia * ia, ia3 = ia2 * ia;
   r.e2 = s[S_OMEGA_M] * ia3 + s[S_OMEGA_K] * ia2 + s[S_OMEGA_DE] * r.ef;
 #pragma unroll
-  for (int d = 0; d < NDIR; ++d) {
+  for (int d = 0; d < ND; ++d) {
     const double* t = sd + d * NSCAL;
     const double df = -3.0 * (t[S_W0] + t[S_WA]) * lna + 3.0 * t[S_WA] * (a - 1.0);
     r.def[d] = t[S_OMEGA_DE] * r.ef + s[S_OMEGA_DE] * r.ef * df;  // d(Omega_de exp(f_de))
@@ -171,71 +178,60 @@ __device__ __forceinline__ E2D e2_grad(const double* s, const double* sd, double
   return r;
 }
 
-__global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
-  const GradItem gi = grad_item(gb, blockIdx.x);
-  TabD* tb = gi.tab;
-  extern __shared__ __align__(16) double sm[];
-  double* s = sm;                            // [NSCAL]
-  double* sd = s + NSCAL;                    // [NDIR][NSCAL]
-  double* fn = sd + NDIR * NSCAL;            // [NDIR + 1][NCHI] chi right-hand sides at the nodes
-  double* fm = fn + (NDIR + 1) * NCHI;       // at the midpoints
-  double* qr = fm + (NDIR + 1) * NCHI;       // [4][NDIR + 1][NGROW] growth coefficients qa, ra, qm, rm
-  double* yv = qr + 4 * (NDIR + 1) * NGROW;  // [NGROW][2] growth solution
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  if (t == 0) tb->wide = 0;
-  for (int i = t; i < NSCAL; i += BG64_THREADS) s[i] = tb->sv[i];
-  for (int i = t; i < NDIR * NSCAL; i += BG64_THREADS) sd[i] = tb->sd[i / NSCAL][i % NSCAL];
-  __syncthreads();
-  // dchi/dln a = R_H / (a sqrt(E^2)) at nodes and midpoints (background.py:227-231)
-  if (t < 2 * NCHI && t != NCHI) {
-    const bool mid = t > NCHI;
-    const int i = mid ? t - NCHI : t;
-    const double a = mid ? c->chi_am[i] : c->chi_a[i], lna = mid ? c->chi_lnam[i] : c->lna_chi[i];
-    const double ia = mid ? c->chi_iam[i] : c->chi_ia[i];
-    const E2D e = e2_grad(s, sd, a, lna, ia);
-    const double r = rsqrt(e.e2), f = RH * ia * r, h = -0.5 * f * (r * r);
-    double* dst = (mid ? fm : fn) + i;
-    dst[0] = f;
+// dchi/dln a = R_H / (a sqrt(E^2)) (background.py:227-231) times w, added to f
+__device__ __forceinline__ void chi_rhs(const double* s, const double* sd, double a, double lna, double ia, double w,
+                                        double* f) {
+  const E2D<NDIR> e = e2_grad<NDIR>(s, sd, a, lna, ia);
+  const double r = rsqrt(e.e2), v = w * (RH * ia * r), h = -0.5 * v * (r * r);
+  f[0] += v;
 #pragma unroll
-    for (int d = 0; d < NDIR; ++d) dst[(1 + d) * NCHI] = h * e.d[d];
+  for (int d = 0; d < NDIR; ++d) f[1 + d] = fma(h, e.d[d], f[1 + d]);
+}
+
+// growth ODE coefficients D'' = -q D' + r D (background.py:96-106), ND directions
+template <int ND>
+struct QR {
+  double q, r, dq[ND], dr[ND];
+};
+template <int ND>
+__device__ __forceinline__ QR<ND> growth_qr_grad(const double* s, const double* sd, double a, double lna, double ia) {
+  QR<ND> o;
+  const E2D<ND> e = e2_grad<ND>(s, sd, a, lna, ia);
+  const double ie = 1.0 / e.e2, ia2 = ia * ia, ia3 = ia2 * ia;
+  const double om = s[S_OMEGA_M] * ia3 * ie, de = s[S_OMEGA_DE] * e.ef * ie;
+  const double w1 = 1.0 + 3.0 * (s[S_W0] + (1.0 - a) * s[S_WA]);
+  o.q = (2.0 - 0.5 * (om + w1 * de)) * ia;
+  o.r = 1.5 * om * ia2;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const double* td = sd + d * NSCAL;
+    const double dom = (td[S_OMEGA_M] * ia3 - om * e.d[d]) * ie, dde = (e.def[d] - de * e.d[d]) * ie;
+    const double dw1 = 3.0 * (td[S_W0] + (1.0 - a) * td[S_WA]);
+    o.dq[d] = -0.5 * (dom + w1 * dde + dw1 * de) * ia;
+    o.dr[d] = 1.5 * dom * ia2;
   }
-  // growth ODE coefficients D'' = -q D' + r D (background.py:96-106)
-  if (t < 2 * NGROW && t != NGROW) {
-    const bool mid = t > NGROW;
-    const int i = mid ? t - NGROW : t;
-    const double a = mid ? c->grow_am[i] : c->atab_grow[i], lna = mid ? c->grow_lnam[i] : c->grow_lna[i];
-    const double ia = mid ? c->grow_iam[i] : c->grow_ia[i];
-    const E2D e = e2_grad(s, sd, a, lna, ia);
-    const double ie = 1.0 / e.e2, ia2 = ia * ia, ia3 = ia2 * ia;
-    const double om = s[S_OMEGA_M] * ia3 * ie, de = s[S_OMEGA_DE] * e.ef * ie;
-    const double w1 = 1.0 + 3.0 * (s[S_W0] + (1.0 - a) * s[S_WA]);
-    double* q = qr + (mid ? 2 * (NDIR + 1) * NGROW : 0) + i;
-    double* r = q + (NDIR + 1) * NGROW;
-    q[0] = (2.0 - 0.5 * (om + w1 * de)) * ia;
-    r[0] = 1.5 * om * ia2;
+  return o;
+}
+
+// One RK4 step is linear in y = (D, dD/da), y_i = M_i y_{i-1}, with
+// K1 = A0, K2 = Am (1 + h/2 K1), K3 = Am (1 + h/2 K2), K4 = A1 (1 + h K3),
+// M = 1 + h/6 (K1 + 2 K2 + 2 K3 + K4), A = [[0, 1], [r, -q]]; dM by the same
+// products.  A thread per step and two directions.
+constexpr int GST_ND = 2, GST_GRP = NDIR / GST_ND;
+__device__ __forceinline__ void growth_step64(TabD* tb, const ConstTables* c, int idx) {
+  const int i = idx % NGROW, d0 = idx / NGROW * GST_ND;
+  Bg64* o = bg_scratch(tb);
+  double M[4] = {1.0, 0.0, 0.0, 1.0};
+  if (i == 0) {
 #pragma unroll
-    for (int d = 0; d < NDIR; ++d) {
-      const double* td = sd + d * NSCAL;
-      const double dom = (td[S_OMEGA_M] * ia3 - om * e.d[d]) * ie, dde = (e.def[d] - de * e.d[d]) * ie;
-      const double dw1 = 3.0 * (td[S_W0] + (1.0 - a) * td[S_WA]);
-      q[(1 + d) * NGROW] = -0.5 * (dom + w1 * dde + dw1 * de) * ia;
-      r[(1 + d) * NGROW] = 1.5 * dom * ia2;
-    }
-  }
-  __syncthreads();
-  // One RK4 step is linear in y = (D, dD/da), y_i = M_i y_{i-1}, with
-  // K1 = A0, K2 = Am (1 + h/2 K1), K3 = Am (1 + h/2 K2), K4 = A1 (1 + h K3),
-  // M = 1 + h/6 (K1 + 2 K2 + 2 K3 + K4), A = [[0, 1], [r, -q]]; dM by the same
-  // products.  Threads 0 .. 127: M_i and dM_i of the 8 directions, in place of the
-  // coefficients once every thread has read its own.
-  double M[4] = {1.0, 0.0, 0.0, 1.0}, dM[NDIR][4];
-#pragma unroll
-  for (int d = 0; d < NDIR; ++d) dM[d][0] = dM[d][1] = dM[d][2] = dM[d][3] = 0.0;
-  if (t >= 1 && t < NGROW) {
-    constexpr int ST = (NDIR + 1) * NGROW;
-    const double* Q = qr;
-    const double h = c->atab_grow[t] - c->atab_grow[t - 1], h2 = 0.5 * h;
-    const double q0 = Q[t - 1], r0 = Q[ST + t - 1], qm = Q[2 * ST + t], rm = Q[3 * ST + t], q1 = Q[t], r1 = Q[ST + t];
+    for (int d = 0; d < GST_ND; ++d) o->dM[d0 + d][0][0] = o->dM[d0 + d][0][1] = o->dM[d0 + d][0][2] = o->dM[d0 + d][0][3] = 0.0;
+  } else {
+    const double *s = tb->sv, *sd = tb->sd[d0];
+    const QR<GST_ND> A0 = growth_qr_grad<GST_ND>(s, sd, c->atab_grow[i - 1], c->grow_lna[i - 1], c->grow_ia[i - 1]);
+    const QR<GST_ND> Am = growth_qr_grad<GST_ND>(s, sd, c->grow_am[i], c->grow_lnam[i], c->grow_iam[i]);
+    const QR<GST_ND> A1 = growth_qr_grad<GST_ND>(s, sd, c->atab_grow[i], c->grow_lna[i], c->grow_ia[i]);
+    const double h = c->atab_grow[i] - c->atab_grow[i - 1], h2 = 0.5 * h;
+    const double q0 = A0.q, r0 = A0.r, qm = Am.q, rm = Am.r, q1 = A1.q, r1 = A1.r;
     // X2 = 1 + h/2 K1, X3 = 1 + h/2 K2, X4 = 1 + h K3 (K = [[k0, k1], [k2, k3]])
     const double X2[4] = {1.0, h2, h2 * r0, 1.0 - h2 * q0};
     const double K2[4] = {X2[2], X2[3], rm * X2[0] - qm * X2[2], rm * X2[1] - qm * X2[3]};
@@ -249,10 +245,8 @@ __global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, c
     M[2] = h6 * (r0 + 2.0 * (K2[2] + K3[2]) + K4[2]);
     M[3] = 1.0 + h6 * (-q0 + 2.0 * (K2[3] + K3[3]) + K4[3]);
 #pragma unroll
-    for (int d = 0; d < NDIR; ++d) {
-      const double* D = Q + (1 + d) * NGROW;
-      const double dq0 = D[t - 1], dr0 = D[ST + t - 1], dqm = D[2 * ST + t], drm = D[3 * ST + t], dq1 = D[t],
-                   dr1 = D[ST + t];
+    for (int d = 0; d < GST_ND; ++d) {
+      const double dq0 = A0.dq[d], dr0 = A0.dr[d], dqm = Am.dq[d], drm = Am.dr[d], dq1 = A1.dq[d], dr1 = A1.dr[d];
       const double x2 = h2 * dr0, x3 = -h2 * dq0;  // dX2 = [[0, 0], [x2, x3]]
       const double k0 = x2, k1 = x3, k2 = drm * X2[0] - dqm * X2[2] - qm * x2, k3 = drm * X2[1] - dqm * X2[3] - qm * x3;
       const double a0 = h2 * k0, a1 = h2 * k1, a2 = h2 * k2, a3 = h2 * k3;  // dX3
@@ -260,35 +254,85 @@ __global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, c
                    l3 = drm * X3[1] - dqm * X3[3] + rm * a1 - qm * a3;
       const double b0 = h * l0, b1 = h * l1, b2 = h * l2, b3 = h * l3;  // dX4
       const double m2 = dr1 * X4[0] - dq1 * X4[2] + r1 * b0 - q1 * b2, m3 = dr1 * X4[1] - dq1 * X4[3] + r1 * b1 - q1 * b3;
-      dM[d][0] = h6 * (2.0 * (k0 + l0) + b2);
-      dM[d][1] = h6 * (2.0 * (k1 + l1) + b3);
-      dM[d][2] = h6 * (dr0 + 2.0 * (k2 + l2) + m2);
-      dM[d][3] = h6 * (-dq0 + 2.0 * (k3 + l3) + m3);
-    }
-  } else if (warp >= 4 && warp < 4 + NDIR + 1) {
-    // chi (background.py:227-233), value and tangents
-    const int comp = warp - 4;
-    chi_scan_warp<true>(fn + comp * NCHI, fm + comp * NCHI, c->lna_chi, lane, comp ? tb->chid[comp - 1] : tb->chiv);
-  }
-  __syncthreads();
-  double* Mv = qr;                 // [NGROW][4]
-  double* dMv = qr + 4 * NGROW;    // [NDIR][NGROW][4]
-  if (t < NGROW) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      Mv[t * 4 + q] = M[q];
-#pragma unroll
-      for (int d = 0; d < NDIR; ++d) dMv[(d * NGROW + t) * 4 + q] = dM[d][q];
+      o->dM[d0 + d][i][0] = h6 * (2.0 * (k0 + l0) + b2);
+      o->dM[d0 + d][i][1] = h6 * (2.0 * (k1 + l1) + b3);
+      o->dM[d0 + d][i][2] = h6 * (dr0 + 2.0 * (k2 + l2) + m2);
+      o->dM[d0 + d][i][3] = h6 * (-dq0 + 2.0 * (k3 + l3) + m3);
     }
   }
+  if (d0 == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o->M[i][q] = M[q];
+  }
+}
+
+// CTAs per cosmology: Eisenstein-Hu nodes, chi steps, growth steps x direction pairs
+constexpr int N64_EH = (NEH + 31) / 32, N64_CHI = NCHI / 32, N64_GROW = GST_GRP * NGROW / 32;
+__global__ void __launch_bounds__(32) grad_nodes64_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+  const GradItem gi = grad_item(gb, blockIdx.y);
+  TabD* tb = gi.tab;
+  const int b = blockIdx.x, lane = threadIdx.x;
+  if (b < N64_EH) {
+    eh_nodes64(tb, c, b);
+  } else if (b < N64_EH + N64_CHI) {
+    // chi's step i - 1 -> i (scipy/ode.py:11-19: the right-hand side has no chi in it)
+    const int i = (b - N64_EH) * 32 + lane;
+    double f[NDIR + 1];
+#pragma unroll
+    for (int q = 0; q <= NDIR; ++q) f[q] = 0.0;
+    if (i > 0) {
+      const double w = (c->lna_chi[i] - c->lna_chi[i - 1]) / 6.0;
+      chi_rhs(tb->sv, tb->sd[0], c->chi_a[i - 1], c->lna_chi[i - 1], c->chi_ia[i - 1], w, f);
+      chi_rhs(tb->sv, tb->sd[0], c->chi_am[i], c->chi_lnam[i], c->chi_iam[i], 4.0 * w, f);
+      chi_rhs(tb->sv, tb->sd[0], c->chi_a[i], c->lna_chi[i], c->chi_ia[i], w, f);
+    }
+    double* o = inc_scratch(tb) + i;
+#pragma unroll
+    for (int q = 0; q <= NDIR; ++q) o[q * NCHI] = f[q];
+  } else {
+    growth_step64(tb, c, (b - N64_EH - N64_CHI) * 32 + lane);
+  }
+}
+
+// The scans: warps 0 .. 7 growth (each the values, then the tangents of its
+// direction), 8 .. 16 chi by suffix sums of the increments
+constexpr int BG64_THREADS = 32 * (2 * NDIR + 1);
+__global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+  const GradItem gi = grad_item(gb, blockIdx.x);
+  TabD* tb = gi.tab;
+  const Bg64* m64 = bg_scratch(tb);
+  __shared__ double Mv[NGROW * 4], yv[NGROW * 2];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) tb->wide = 0;
+  for (int i = t; i < NGROW * 4; i += BG64_THREADS) Mv[i] = m64->M[0][i];
   __syncthreads();
+  if (warp >= NDIR) {
+    const int comp = warp - NDIR;
+    const double* inc = inc_scratch(tb) + comp * NCHI;
+    double* out = comp ? tb->chid[comp - 1] : tb->chiv;
+    double loc[8], x = 0.0;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+      loc[k] = x;
+      x += inc[lane * 8 + k];
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double u = __shfl_down_sync(0xffffffffu, x, o);
+      if (lane + o < 32) x += u;
+    }
+    double off = __shfl_down_sync(0xffffffffu, x, 1);
+    if (lane == 31) off = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[lane * 8 + k] = off + loc[k];
+  }
   double d4[4], yf = 0.0;
   if (warp < NDIR) yf = growth_scan_warp(Mv, c->atab_grow[0], 1.0, lane, d4, warp == 0 ? yv : nullptr);
   __syncthreads();
   if (warp < NDIR) {
     // dy_i = M_i dy_{i-1} + dM_i y_{i-1}, dy_0 = 0: a scan of affine maps (A, b)
     const double iyf = 1.0 / yf;
-    const double* dMd = dMv + (size_t)warp * NGROW * 4;
+    const double* dMd = m64->dM[warp][0];
     double A[4] = {1.0, 0.0, 0.0, 1.0}, b0 = 0.0, b1 = 0.0, c0[4], c1[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -337,63 +381,62 @@ __global__ void __launch_bounds__(BG64_THREADS) grad_bg64_kernel(GradBatch gb, c
 }
 
 // ---------------------------------------- sigma8, P(k) k^3 and sigma^2(R) ---
-constexpr int SG64_THREADS = 64;
+constexpr int SG64_THREADS = 256, SG64_R = 64;  // four threads per R
 __global__ void __launch_bounds__(SG64_THREADS) grad_sigma64_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
   const GradItem gi = grad_item(gb, blockIdx.y);
   TabD* tb = gi.tab;
   const int comp = blockIdx.x % (NDIR + 1), part = blockIdx.x / (NDIR + 1), t = threadIdx.x;
   const double* u = eh_scratch(tb);
   const double* ud = u + comp * NEH;
-  __shared__ double red[2][2];
+  __shared__ double sums[4][SG64_R], norm[2];
   __shared__ double pq[NKH];
-  // sigmasqr(8) (power.py:70-78): romb is linear in the integrand's values
-  double a = 0.0, b = 0.0;
-  for (int e = t; e < NROMB; e += SG64_THREADS) a = fma(c->romb_w[e], u[e], a), b = fma(c->romb_w[e], ud[e], b);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  if ((t & 31) == 0) red[t >> 5][0] = a, red[t >> 5][1] = b;
-  __syncthreads();
   const double i2 = 1.0 / (2.0 * (PI * PI));
-  const double sig = i2 * (red[0][0] + red[1][0]), dsig = i2 * (red[0][1] + red[1][1]);
-  // P(k) normalisation sigma8^2 / sigmasqr(8) (power.py:47) and its tangent
-  const double s8 = tb->sv[S_SIGMA8], pn = s8 * s8 / sig;
-  const double ds8 = comp ? tb->sd[comp - 1][S_SIGMA8] : 0.0;
-  const double dpn = comp ? (2.0 * s8 * ds8 - pn * dsig) / sig : 0.0;
-  if (t == 0 && part == 0) {
-    if (comp == 0) {
-      tb->sv[S_SIGMASQR8] = sig;
-      tb->sv[S_PKNORM] = pn;
-    } else {
-      tb->sd[comp - 1][S_SIGMASQR8] = dsig;
-      tb->sd[comp - 1][S_PKNORM] = dpn;
+  if (t < 32) {
+    // sigmasqr(8) (power.py:70-78): romb is linear in the integrand's values
+    double a = 0.0, b = 0.0;
+    for (int e = t; e < NROMB; e += 32) a = fma(c->romb_w[e], u[e], a), b = fma(c->romb_w[e], ud[e], b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    // P(k) normalisation sigma8^2 / sigmasqr(8) (power.py:47) and its tangent
+    const double sig = i2 * a, dsig = i2 * b, s8 = tb->sv[S_SIGMA8], pn = s8 * s8 / sig;
+    const double ds8 = comp ? tb->sd[comp - 1][S_SIGMA8] : 0.0;
+    const double dpn = comp ? (2.0 * s8 * ds8 - pn * dsig) / sig : 0.0;
+    if (t == 0) {
+      norm[0] = pn, norm[1] = dpn;
+      if (part == 0 && comp == 0) tb->sv[S_SIGMASQR8] = sig, tb->sv[S_PKNORM] = pn;
+      if (part == 0 && comp != 0) tb->sd[comp - 1][S_SIGMASQR8] = dsig, tb->sd[comp - 1][S_PKNORM] = dpn;
     }
   }
+  __syncthreads();
+  const double pn = norm[0], dpn = norm[1];
   // P(k_i, a = 1) k_i^3 (the growth table is normalised to 1 at a = 1)
   for (int i = t; i < NKH; i += SG64_THREADS) {
     const double v = u[NROMB + i], p = (comp ? ud[NROMB + i] * pn + v * dpn : v * pn) * c->kh3[i];
     if (part == 0) (comp ? tb->pk3d[comp - 1] : tb->pk3v)[i] = p;
-    pq[i] = c->simpson_kh[i] * (p / (2.0 * (PI * PI)));
+    pq[i] = c->simpson_kh[i] * (p * i2);
     if (part == 0) {
       const FF f = px_of(pq[i]);
       grad_kw64(tb)[comp * NKH + i] = make_float2(f.hi, f.lo);
     }
   }
   __syncthreads();
-  const int j = part * SG64_THREADS + t;
+  const int q = t / SG64_R, jj = t % SG64_R, j = part * SG64_R + jj;
   double acc = 0.0;
-  for (int i = 0; i < NKH; ++i) acc = fma(pq[i], c->E[i * NRT + j], acc);
-  (comp ? tb->sigd[comp - 1] : tb->sigv)[j] = acc;
+#pragma unroll 8
+  for (int i = q; i < NKH; i += 4) acc = fma(pq[i], c->E[i * NRT + j], acc);
+  sums[q][jj] = acc;
+  __syncthreads();
+  if (q == 0) (comp ? tb->sigd[comp - 1] : tb->sigv)[j] = (sums[0][jj] + sums[1][jj]) + (sums[2][jj] + sums[3][jj]);
 }
-static_assert(NRT % SG64_THREADS == 0, "whole parts of the R nodes");
+static_assert(NRT % SG64_R == 0, "whole parts of the R nodes");
 
 void launch_grad_tables64(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
-  grad_eh64_kernel<<<dim3((NEH + 31) / 32, gb.n_items), 32, 0, st>>>(gb, c);
-  cudaFuncSetAttribute(grad_bg64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BG64_SMEM);
-  grad_bg64_kernel<<<gb.n_items, BG64_THREADS, BG64_SMEM, st>>>(gb, c);
-  grad_sigma64_kernel<<<dim3((NDIR + 1) * (NRT / SG64_THREADS), gb.n_items), SG64_THREADS, 0, st>>>(gb, c);
+  grad_nodes64_kernel<<<dim3(N64_EH + N64_CHI + N64_GROW, gb.n_items), 32, 0, st>>>(gb, c);
+  grad_bg64_kernel<<<gb.n_items, BG64_THREADS, 0, st>>>(gb, c);
+  grad_sigma64_kernel<<<dim3((NDIR + 1) * (NRT / SG64_R), gb.n_items), SG64_THREADS, 0, st>>>(gb, c);
 }
 
 }  // namespace jcg

@@ -7,13 +7,13 @@
 //     B = sum W / chi' (dK_d = A_d - dchi_d B) are ten sums of products in float
 //     pairs (jcg_px.cuh), weights scaled per (node, bin) as in jcg_tracer64.cu.  A
 //     warp per (cosmology, node), points over lanes, three bins at a time in
-//     registers; the lanes' sums are added by one lane per sum.
+//     registers (a warp per pass); the lanes' sums are added by one lane per sum.
 //   grad_kernfin64_kernel   a thread per (node, tracer): prefactors, single planes,
 //     NumberCounts and alignment terms in float64.
 //
 // One kernel did both in Dual<8> float64 (a warp per node, the second part on 8
 // of its lanes): 61 cosmologies, 3 + 2 bins with alignment terms, 513 nodes
-// 5.00 -> 0.56 + 0.31 ms; one cosmology, 5 + 5 bins 208 -> 61 + 12 us.  The first
+// 5.00 -> 0.57 + 0.31 ms; one cosmology, 5 + 5 bins 208 -> 40 + 12 us.  The first
 // is bound by issue (some 500 instructions a point and three bins), the second
 // by the FP64 pipe (pow, exp and log of its terms).
 #include "jcg_grad.cuh"
@@ -67,7 +67,17 @@ __global__ void __launch_bounds__(GK_WARPS * 32, 2)
   const double* AWL = geo_ptr<double>(geo, geo->off_awl);
   const int64_t* SW = geo_ptr<int64_t>(geo, geo->off_seg_chiwl);
   const int n_end = min(na, n0 + per);
-  for (int n = n0 + warp; n < n_end; n += GK_WARPS) {
+  // a warp per (node, pass of three bins)
+  int passes = 0;
+  for (int g = 0; g < geo->n_groups; ++g) {
+    int k = 0;
+    for (int t = 0; t < n_tr; ++t)
+      k += geo->kind[t] == JCG_TRACER_WL && geo->group[t] == g && geo->nz_kind[t] != JCG_NZ_DELTA;
+    passes += (k + GK_BINS - 1) / GK_BINS;
+  }
+  for (int w = warp; w < (n_end - n0) * passes; w += GK_WARPS) {
+    const int n = n0 + w / passes;
+    int skip = w % passes;
     const double awl = AWL[n];
     const int2 sw = unpack_seg(SW[n]);
     const D1 cw = xfmax(interp_d1(awl, c->atab_chi, tb->chiv, tb->chid[lane & 7], sw), 0.0);
@@ -92,6 +102,7 @@ __global__ void __launch_bounds__(GK_WARPS * 32, 2)
             ++nb;
           }
         if (nb == 0) break;
+        if (skip-- != 0) continue;
         int ex[GK_BINS];
         const double* W[GK_BINS];
 #pragma unroll
@@ -269,7 +280,8 @@ __global__ void __launch_bounds__(GKF_THREADS)
 void launch_grad_kern64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide) {
   // nodes per CTA: 32 pay for the tables; fewer while the CTAs do not fill the SMs
   int per = 32;
-  while (per > GK_WARPS && (long long)gb.n_items * ((gb.na + per - 1) / per) < 2 * device_sm_count()) per >>= 1;
+  const int least = gb.listed || gb.n_wl > GK_BINS ? GK_WARPS / 2 : GK_WARPS;
+  while (per > least && (long long)gb.n_items * ((gb.na + per - 1) / per) < 2 * device_sm_count()) per >>= 1;
   if (gb.listed || gb.n_wl > 0) {
     cudaFuncSetAttribute(grad_wlsum64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GkSmem));
     grad_wlsum64_kernel<<<dim3((gb.na + per - 1) / per, gb.n_items), GK_WARPS * 32, sizeof(GkSmem), st>>>(gb, c, per,

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(GXS_THREADS) grad_scale64_kernel(GradBatch gb)
   TabD* tb = gi.tab;
   GxScratch* sc = gx_scratch(tb);
   if (i < n_tr) {
-    __shared__ unsigned mx, mp;
+    __shared__ unsigned mx;
     if (t == 0) mx = 0;
     __syncthreads();
     const double* K = gi.kernd + (size_t)i * na * (NDIR + 1);
@@ -74,28 +74,21 @@ __global__ void __launch_bounds__(GXS_THREADS) grad_scale64_kernel(GradBatch gb)
     bad |= ex == 0x7ff || (ex != 0 && (ex < 64 || ex > 1983));
     // the exponent of an all-zero kernel is that of 1 (its tangents may not be 0)
     if (t == 0) sc->kexp[i] = ex == 0 ? 1023 : ex;
-    for (int p = 0; p < n_cls; ++p) {
+    // a warp per spectrum of the tracer
+    for (int p = 0, k = 0; p < n_cls; ++p) {
       if (geo->pair_i[p] != i) continue;
+      if ((k++ & (GXS_THREADS / 32 - 1)) != (t >> 5)) continue;
       const double* Kj = gi.kernd + (size_t)geo->pair_j[p] * na * (NDIR + 1);
-      __syncthreads();
-      if (t == 0) mp = 0;
-      __syncthreads();
       unsigned q = 0, qj = 0;
-      for (int n = t; n < na; n += GXS_THREADS) {
+#pragma unroll 4
+      for (int n = t & 31; n < na; n += 32) {
         const double kj = Kj[(size_t)n * (NDIR + 1)];
         q = max(q, (unsigned)__double2hiint(K[(size_t)n * (NDIR + 1)] * kj) & 0x7fffffffu);
         qj = max(qj, (unsigned)__double2hiint(kj) & 0x7fffffffu);
       }
-      atomicMax(&mp, q);
-      __syncthreads();
-      const unsigned ep = mp >> 20;
-      __syncthreads();
-      if (t == 0) mp = 0;
-      __syncthreads();
-      atomicMax(&mp, qj);
-      __syncthreads();
+      const unsigned ep = __reduce_max_sync(0xffffffffu, q) >> 20, ej = __reduce_max_sync(0xffffffffu, qj) >> 20;
       // largest product below 2^-66 of the product of the largest: not for pairs
-      if (ep != 0 && (int)ep - ex - ((int)(mp >> 20) - 1023) < -66) bad = true;
+      if (ep != 0 && (int)ep - ex - ((int)ej - 1023) < -66) bad = true;
     }
     if (bad) tb->wide = 1;
     return;
