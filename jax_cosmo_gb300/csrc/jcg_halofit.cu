@@ -707,8 +707,9 @@ __global__ void eval_points_kernel(const double* __restrict__ params, int n_cosm
                                    const double* __restrict__ kv, int n, int what_phys,
                                    double* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int what = what_phys & 0xff, model = pk_model(what_phys >> 8);
-  const long gw = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int what = what_phys & 0xff;
+  const bool by_warp = what == 12;  // a warp per point, else a thread
+  const long gt = (long)blockIdx.x * blockDim.x + threadIdx.x, gw = by_warp ? gt >> 5 : gt;
   if (gw >= (long)n_cosmo * n) return;
   const int ci = (int)(gw / n), pi = (int)(gw % n);
   const CosmoTab* ct = ctab + ci;
@@ -756,33 +757,78 @@ __global__ void eval_points_kernel(const double* __restrict__ params, int n_cosm
     v = eh_transfer(s, k);
   } else if (what == 5) {
     v = pk_linear(s, k, growth(a));
-  } else {
-    const double g = growth(a);
-    const HfParams hp = halofit_params_warp(ct->sig, ct->pk3, g, c, lane);
-    if (what == 6) {
-      double row[NROW64];
-      row[R_G] = g;
-      halofit_coefs(bg, a, log(a), hp, row, model);
-      v = halofit_node(s, row, k, model);
-    } else if (what == 7) {
-      v = hp.knl;
-    } else if (what == 8) {
-      v = hp.neff;
-    } else {
-      v = hp.C;
+  }
+  if (!by_warp || lane == 0) out[(size_t)ci * n + pi] = v;
+}
+
+// nonlinear_matter_power (what 6), k_nl, n_eff, C (7, 8, 9) at P consecutive points
+// of the flat (cosmology, point) index per CTA: linear P(k) a thread per point and
+// the moments a warp per point (threads count down, so that with one or two points
+// the two run on different warps), then the coefficients and P(k) a thread per
+// point.  With all of it on every lane of a point's warp, 256 points took 89 us,
+// now @E1@, and 20,000 points @E2@ ms, now @E3@.
+__global__ void __launch_bounds__(256)
+    eval_halofit_kernel(int n_cosmo, const CosmoTab* __restrict__ ctab, const ConstTables* __restrict__ c,
+                        const double* __restrict__ av, const double* __restrict__ kv, int n, int what_phys, int P,
+                        double* __restrict__ out) {
+  __shared__ double knl[256], neff[256], cur[256], gs[256], pl[256];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int what = what_phys & 0xff, model = pk_model(what_phys >> 8);
+  const long p0 = (long)blockIdx.x * P, all = (long)n_cosmo * n;
+  const int cnt = (int)(all - p0 < P ? all - p0 : P);
+  auto growth = [&](const CosmoTab* ct, double x) {
+    const int2 sg = interp_segment_inc(x, c->atab_grow, NGROW, logspace_guess(x, NGROW));
+    return clip_lohi(interp_eval(x, c->atab_grow, ct->g, sg), 0.0, 1.0);
+  };
+  if (what == 6) {
+    for (int q = (int)blockDim.x - 1 - tid; q < cnt; q += blockDim.x) {
+      const long e = p0 + q;
+      const CosmoTab* ct = ctab + e / n;
+      const double k = kv ? kv[e % n] : 1.0;
+      pl[q] = pk_linear_lk(ct->s, k, log(k), growth(ct, av ? av[e % n] : 1.0));
     }
   }
-  if (lane == 0) out[(size_t)ci * n + pi] = v;
+  for (int q = warp; q < cnt; q += (int)blockDim.x >> 5) {
+    const long e = p0 + q;
+    const CosmoTab* ct = ctab + e / n;
+    const double g = growth(ct, av ? av[e % n] : 1.0);
+    const HfParams hp = halofit_params_warp(ct->sig, ct->pk3, g, c, lane);
+    if (lane == 0) knl[q] = hp.knl, neff[q] = hp.neff, cur[q] = hp.C, gs[q] = g;
+  }
+  __syncthreads();
+  for (int q = tid; q < cnt; q += blockDim.x) {
+    const long e = p0 + q;
+    HfParams hp;
+    hp.knl = knl[q], hp.neff = neff[q], hp.C = cur[q];
+    double v = what == 7 ? hp.knl : what == 8 ? hp.neff : hp.C;
+    if (what == 6) {
+      const double a = av ? av[e % n] : 1.0, k = kv ? kv[e % n] : 1.0;
+      double row[NROW64];
+      row[R_G] = gs[q];
+      halofit_coefs(make_bg(ctab[e / n].s), a, log(a), hp, row, model);
+      v = halofit_from_linear(row, k, log(k), pl[q], model);
+    }
+    out[e] = v;
+  }
 }
 
 void launch_eval_points(const double* params, int n_cosmo, CosmoTab* ctab, const ConstTables* c,
                         const double* a, const double* k, int n, int what, double* out,
                         cudaStream_t st) {
-  const long warps = (long)n_cosmo * n;
-  const int threads = 256;
-  const long blocks = (warps * 32 + threads - 1) / threads;
-  eval_points_kernel<<<(unsigned)blocks, threads, 0, st>>>(params, n_cosmo, ctab, c, a, k, n, what,
-                                                            out);
+  const long points = (long)n_cosmo * n;
+  const long sms = device_sm_count();
+  if ((what & 0xff) >= 6 && (what & 0xff) <= 9) {
+    // two CTAs per SM before a CTA takes more points; warps as it has points, two at least
+    const long want = (points + 2 * sms - 1) / (2 * sms);
+    const int P = (int)(want < 256 ? want : 256), warps = P < 2 ? 2 : P < 8 ? P : 8;
+    eval_halofit_kernel<<<(unsigned)((points + P - 1) / P), warps * 32, 0, st>>>(n_cosmo, ctab, c, a, k, n, what, P, out);
+    return;
+  }
+  // small CTAs: a few hundred points spread over the SMs
+  const long threads = (what & 0xff) == 12 ? points * 32 : points;
+  const int block = threads <= 64 * sms ? 32 : 256;
+  eval_points_kernel<<<(unsigned)((threads + block - 1) / block), block, 0, st>>>(params, n_cosmo, ctab, c, a, k, n, what,
+                                                                               out);
 }
 
 }  // namespace jcg

@@ -785,9 +785,7 @@ __device__ __forceinline__ double pk_linear(const double* s, double k, double g)
 // the row's coefficients; d2h = d2h' / (1 + mu/y + nu/y^2) evaluated as
 // d2h' y^2 / (y^2 + mu y + nu)), or the linear power for JCG_PK_LINEAR
 // (nonlinear_fn = linear_matter_power).
-__device__ __forceinline__ double halofit_node_lk(const double* s, const double* row, double k,
-                                                  double lk, int model) {
-  const double pklin = pk_linear_lk(s, k, lk, row[R_G]);
+__device__ __forceinline__ double halofit_from_linear(const double* row, double k, double lk, double pklin, int model) {
   if (model == JCG_PK_LINEAR) return pklin;
   const double k3 = k * k * k;
   const double d2l = k3 * pklin / (2.0 * (PI * PI));
@@ -803,8 +801,10 @@ __device__ __forceinline__ double halofit_node_lk(const double* s, const double*
   const double d2h = d2hprime * y2 / ((y2 + row[R_MUN] * y) + row[R_NUN]);
   return 2.0 * (PI * PI) / k3 * (d2q + d2h);
 }
-__device__ __forceinline__ double halofit_node(const double* s, const double* row, double k, int model) {
-  return halofit_node_lk(s, row, k, log(k), model);
+// from the cosmology's scalars
+__device__ __forceinline__ double halofit_node_lk(const double* s, const double* row, double k,
+                                                  double lk, int model) {
+  return halofit_from_linear(row, k, lk, pk_linear_lk(s, k, lk, row[R_G]), model);
 }
 
 // ------------------------------------------------------------- launches ----
