@@ -247,6 +247,9 @@ static int make_header(const jcg_geometry* g, GeoHeader* h) {
   h->off_seg_grow = take(na);
   h->off_seg_chiwl = take(na);
   h->off_nzl = take((int64_t)h->n_tr * na);
+  h->off_bz = take((int64_t)h->n_tr * na);
+  h->off_lnawl = take(na);
+  h->off_seg_growwl = take(na);
   h->off_ell = take(h->n_ell);
   h->off_ellfac = take((int64_t)h->n_tr * h->n_ell);
   h->off_lg2ellh = take(h->n_ell);

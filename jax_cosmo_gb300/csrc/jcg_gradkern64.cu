@@ -207,7 +207,7 @@ __device__ __noinline__ D1 wl_sum_d1(const TabD* tb, const ConstTables* c, const
 }
 
 constexpr int GKF_THREADS = 64;
-__global__ void __launch_bounds__(GKF_THREADS)
+__global__ void __launch_bounds__(GKF_THREADS, 10)
     grad_kernfin64_kernel(GradBatch gb, const ConstTables* __restrict__ c, int only_wide) {
   const GradItem gi = grad_item(gb, blockIdx.z);
   const TabD* tb = gi.tab;
@@ -245,15 +245,14 @@ __global__ void __launch_bounds__(GKF_THREADS)
     // n(z) b(z) H(a) (probes.py:94), or the alignment term n(z) b(z) H(a)
     // (-C_1 rho_crit Omega_m / D(a)) (probes.py:102-129)
     const double nz = geo_ptr<double>(geo, geo->off_nzl)[(size_t)t * na + n];
-    const double lna = log(awl), ia = 1.0 / awl, ia2 = ia * ia, ia3 = ia2 * ia;
+    const double lna = geo_ptr<double>(geo, geo->off_lnawl)[n], ia = 1.0 / awl, ia2 = ia * ia, ia3 = ia2 * ia;
     const double f = -3.0 * (1.0 + tb->sv[S_W0] + tb->sv[S_WA]) * lna + 3.0 * tb->sv[S_WA] * (awl - 1.0);
     const double ef = exp(f);
     const double e2 = om * ia3 + tb->sv[S_OMEGA_K] * ia2 + tb->sv[S_OMEGA_DE] * ef;
     const double H = H0 * sqrt(e2), h2 = 0.5 / e2;
     const bool grow = wl || bk == JCG_BIAS_INV_GROWTH;
-    int2 sg = make_int2(0, 1);
-    if (grow) sg = interp_segment_inc(awl, c->atab_grow, NGROW, logspace_guess(awl, NGROW));
-    const double b0 = bk == JCG_BIAS_INV_GROWTH ? geo->bias[t] : bias_at(geo, t, z, 1.0);
+    const int2 sg = unpack_seg(geo_ptr<int64_t>(geo, geo->off_seg_growwl)[n]);
+    const double b0 = geo_ptr<double>(geo, geo->off_bz)[(size_t)t * na + n];
     double bv = 0.0;
     for (int d = 0; d < NDIR; ++d) {
       const double* sd = tb->sd[d];

@@ -539,7 +539,7 @@ __device__ void halofit_coefs64(double om_m, double om_de, double w, const HfPar
   row[R_LGCF3] = L10 * e_cn + (small ? ex[2] : log(f[2]));
 }
 
-__global__ void __launch_bounds__(HF_WARPS * 32, 3)
+__global__ void __launch_bounds__(HF_WARPS * 32, 5)
     halofit_rows64_kernel(Batch bt, const ConstTables* __restrict__ c, int nb) {
   const int item = blockIdx.y;
   const Item it = batch_item(bt, item);

@@ -260,6 +260,9 @@ struct GeoHeader {
   int64_t off_a, off_z, off_wsimp, off_awl;
   int64_t off_seg_chi, off_seg_grow, off_seg_chiwl;  // int32 pairs, packed as int64 per node
   int64_t off_nzl;                                   // [n_tr][na] n_t(z_n)
+  // float64 radial kernels: b_t(z_n) [n_tr][na] (without the growth factor of
+  // JCG_BIAS_INV_GROWTH), ln a and the growth table's segment at the off_awl nodes
+  int64_t off_bz, off_lnawl, off_seg_growwl;
   int64_t off_ell, off_ellfac;                       // [n_ell], [n_tr][n_ell]
   int64_t off_lg2ellh;                               // [n_ell] log2(ell + 1/2) (fp32 path)
   int64_t off_kh4;                                   // [n_ell] float4 (l + 1/2, log2(l + 1/2), 1 / (l + 1/2), 0)

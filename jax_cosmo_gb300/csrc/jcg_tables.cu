@@ -327,9 +327,17 @@ __global__ void geo_tables_kernel(const GeoHeader* __restrict__ hp, double* geo,
     SG[n] = pack_seg(interp_segment_inc(a, c->atab_grow, NGROW, logspace_guess(a, NGROW)));
     const int2 swl = interp_segment_inc(awl, c->atab_chi, NCHI, logspace_guess(awl, NCHI));
     SW[n] = pack_seg(swl);
+    geo[h.off_lnawl + n] = log(awl);
+    reinterpret_cast<int64_t*>(geo + h.off_seg_growwl)[n] =
+        pack_seg(interp_segment_inc(awl, c->atab_grow, NGROW, logspace_guess(awl, NGROW)));
     reinterpret_cast<int32_t*>(geo + h.off_qwl32)[n] = swl.x | (min(swl.x, swl.y) << 16);
     reinterpret_cast<float*>(geo + h.off_dxwl32)[n] = (float)(awl - c->atab_chi[swl.x]);
     for (int t = 0; t < h.n_tr; ++t) NZL[(size_t)t * na + n] = tracer_pz(h, pz, t, NZP + n, z) / h.nz_norm[t];
+  }
+  for (int q = tid; q < h.n_tr * na; q += nth) {
+    const int t = q / na, n = q % na;
+    const double z = h.custom_nodes ? Z[n] : 1.0 / np_linspace(a0, 1.0, N, n) - 1.0;
+    geo[h.off_bz + q] = bias_at(&h, t, z, 1.0);
   }
   // ell grid factors (probes.py:73; NumberCounts: 1)
   const double* ell = geo + h.off_ell;

@@ -60,13 +60,26 @@ __device__ __noinline__ double wl_sum_f64(const GeoHeader* geo, const CosmoTab* 
   return acc;
 }
 
+// H and the growth factor at node n (bg_H, growth_at with the geometry's logarithm
+// and segment)
+__device__ __forceinline__ double node_H(const GeoHeader* geo, const CosmoTab* ct, int n, double awl) {
+  return H0 * sqrt(bg_esqr_l(make_bg(ct->s), awl, geo_ptr<double>(geo, geo->off_lnawl)[n], nullptr));
+}
+__device__ __forceinline__ double node_D(const GeoHeader* geo, const CosmoTab* ct, const ConstTables* c, int n,
+                                         double awl) {
+  const int2 sg = unpack_seg(geo_ptr<int64_t>(geo, geo->off_seg_growwl)[n]);
+  return clip_lohi(interp_eval(awl, c->atab_grow, ct->g, sg), 0.0, 1.0);
+}
+
 // tracer t's kernel at node n from its z' integral acc; hz = H, dz = growth
 // factor (used where the tracer needs them)
 __device__ __forceinline__ double tracer_value(const GeoHeader* geo, const CosmoTab* ct, const ConstTables* c, int t,
                                                int n, double acc, double chi_wl, double z, double om, double hz,
                                                double dz) {
   const double nz = geo_ptr<double>(geo, geo->off_nzl)[(size_t)t * geo->na + n];
-  if (geo->kind[t] != JCG_TRACER_WL) return nz * bias_at(geo, t, z, dz) * hz;
+  const double b = geo->bias_kind[t] == JCG_BIAS_INV_GROWTH ? geo->bias[t] / dz
+                                                            : geo_ptr<double>(geo, geo->off_bz)[(size_t)t * geo->na + n];
+  if (geo->kind[t] != JCG_TRACER_WL) return nz * b * hz;
   if (geo->nz_kind[t] == JCG_NZ_DELTA) {
     // single plane (probes.py:53-64): clip(chi(z0) - chi, 0) / clip(chi(z0), 1)
     const double a0 = 1.0 / (1.0 + geo->nz_z0[t]);
@@ -77,13 +90,13 @@ __device__ __forceinline__ double tracer_value(const GeoHeader* geo, const Cosmo
   double kv = 3.0 * (H0 * H0) * om / 2.0 / C_KMS * (acc * (1.0 + z) * chi_wl);  // probes.py:71
   if (geo->bias_kind[t] != JCG_BIAS_NONE) {
     // NLA intrinsic alignment (probes.py:102-129), same ell factor as the shear
-    kv = kv + nz * bias_at(geo, t, z, dz) * hz * (-IA_C1_RHOCRIT * om / dz);
+    kv = kv + nz * b * hz * (-IA_C1_RHOCRIT * om / dz);
   }
   return kv * (1.0 + geo->mult[t]);
 }
 
 // ------------------------------------------------- a warp per (item, node) --
-__global__ void __launch_bounds__(T64_WARPS * 32)
+__global__ void __launch_bounds__(T64_WARPS * 32, 4)
     tracer64_kernel(Batch bt, const ConstTables* __restrict__ c, int per) {
   const Item it = batch_item(bt, blockIdx.y);
   const GeoHeader* geo = it.geo;
@@ -188,9 +201,9 @@ __global__ void __launch_bounds__(T64_WARPS * 32)
     const bool wl = geo->kind[t] == JCG_TRACER_WL;
     const double awl = AWL[n];
     double hz = 0.0, dz = 1.0;
-    if (!wl || geo->bias_kind[t] != JCG_BIAS_NONE) hz = bg_H(make_bg(ct->s), awl);
+    if (!wl || geo->bias_kind[t] != JCG_BIAS_NONE) hz = node_H(geo, ct, n, awl);
     if (geo->bias_kind[t] == JCG_BIAS_INV_GROWTH || (wl && geo->bias_kind[t] != JCG_BIAS_NONE))
-      dz = growth_at(ct->g, c, awl);
+      dz = node_D(geo, ct, c, n, awl);
     it.kern[(size_t)t * na + n] = tracer_value(geo, ct, c, t, n, accs[t][i], chis[i], Z[n], om, hz, dz);
   }
 }
@@ -205,7 +218,7 @@ struct T64Rec {
 __host__ __device__ inline size_t t64_tab_bytes(int wn) { return ((size_t)wn * T64_PAD * 20 + 15) & ~(size_t)15; }
 
 template <int NW>
-__global__ void __launch_bounds__(T64_WARPS * 32, 2)
+__global__ void __launch_bounds__(T64_WARPS * 32, 3)
     tracer64_uniform_kernel(Batch bt, const ConstTables* __restrict__ c, int per) {
   const GeoHeader* geo = bt.geo;
   const int na = geo->na, n_tr = geo->n_tr;
@@ -317,8 +330,8 @@ __global__ void __launch_bounds__(T64_WARPS * 32, 2)
     }
     if (live) {
       double hz = 0.0, dz = 1.0;
-      if (geo->n_nc > 0 || geo->special_bias) hz = bg_H(make_bg(ct->s), awl);
-      if (geo->special_bias) dz = growth_at(ct->g, c, awl);
+      if (geo->n_nc > 0 || geo->special_bias) hz = node_H(geo, ct, n, awl);
+      if (geo->special_bias) dz = node_D(geo, ct, c, n, awl);
       const double z = Z[n];
 #pragma unroll
       for (int u = 0; u < NW; ++u) {
