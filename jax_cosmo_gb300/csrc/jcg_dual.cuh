@@ -607,11 +607,26 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   const T h2 = h * h;
   const T w_m = Om * h2;
   const T w_b = Ob * h2;
-  const T fb = Ob / Om;
-  const T fc = (Om - Ob) / Om;
-  const T k_eq = 7.46e-2 * w_m / T27 / h;
-  const T z_eq = 2.50e4 * w_m / (T27 * T27);
-  const T R_eq = 31.5 * w_b / (T27 * T27) * (1.0e3 / z_eq);
+  // quotients side by side too (a float64 division is about 10 operations)
+  T nu = one, de = one;
+  switch (lane) {
+    case 0: nu = Ob, de = Om; break;
+    case 1: nu = Om - Ob, de = Om; break;
+    case 2: nu = 7.46e-2 * w_m, de = T27 * one; break;
+    case 3: nu = 2.50e4 * w_m, de = (T27 * T27) * one; break;
+    case 4: nu = 31.5 * w_b, de = (T27 * T27) * one; break;
+    case 5: nu = T27 * one, de = Om * h; break;
+    default: break;
+  }
+  const T Q1 = nu / de;
+  const T fb = shfl_t(Q1, 0), fc = shfl_t(Q1, 1), keqh = shfl_t(Q1, 2), z_eq = shfl_t(Q1, 3);
+  const T wbT = shfl_t(Q1, 4), nwq = shfl_t(Q1, 5);
+  nu = one, de = one;
+  if (lane == 0) nu = keqh, de = h;
+  if (lane == 1) nu = 1.0e3 * one, de = z_eq;
+  const T Q2 = nu / de;
+  const T k_eq = shfl_t(Q2, 0);
+  const T R_eq = wbT * shfl_t(Q2, 1);
   // level 1: pow(w, e), sqrt, log of the parameters
   T pb = one, sq = one, lg = one;
   double pe = 1.0;
@@ -653,10 +668,18 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   // level 2: pows with parameter-dependent exponents, log(k_silk)
   const T b1 = 0.313 * A0 * (1.0 + 0.607 * A1);
   const T b2 = 0.238 * A2;
-  const T k_silk = 1.6 * A5 * A6 * (1.0 + A7) / h;
+  nu = one, de = one;
+  switch (lane) {
+    case 0: nu = 1.6 * A5 * A6 * (1.0 + A7), de = h; break;
+    case 1: nu = 0.944 * one, de = 1.0 + A12; break;
+    case 2: nu = 1291.0 * A3, de = 1.0 + 0.659 * A4; break;
+    case 3: nu = 2.0 * one, de = 3.0 * k_eq; break;
+    default: break;
+  }
+  const T Q3 = nu / de;
+  const T k_silk = shfl_t(Q3, 0), b1c = shfl_t(Q3, 1), zdq = shfl_t(Q3, 2), shq = shfl_t(Q3, 3);
   const T a1 = A8 * (1.0 + A9);
   const T a2 = A10 * (1.0 + A11);
-  const T b1c = 0.944 / (1.0 + A12);
   const T b2c = A13;
   T qb = one, qe = one;
   switch (lane) {
@@ -670,12 +693,18 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   const T B0 = shfl_t(P2, 0), B1 = shfl_t(P2, 1), B2 = shfl_t(P2, 2), B3 = shfl_t(P2, 3);
   const T lgks = shfl_t(L2, 0);
   // level 3
-  const T z_d = 1291.0 * A3 / (1.0 + 0.659 * A4) * (1.0 + b1 * B0);
-  const T R_d = 31.5 * w_b / (T27 * T27) * (1.0e3 / z_d);
+  const T z_d = zdq * (1.0 + b1 * B0);
   const T alpha_c = B1 * B2;
-  T beta_c = 1.0 + b1c * (B3 - 1.0);
-  beta_c = 1.0 / beta_c;
-  const T y = (1.0 + z_eq) / (1.0 + z_d);
+  nu = one, de = one;
+  switch (lane) {
+    case 0: nu = 1.0e3 * one, de = z_d; break;
+    case 1: de = 1.0 + b1c * (B3 - 1.0); break;
+    case 2: nu = 1.0 + z_eq, de = 1.0 + z_d; break;
+    default: break;
+  }
+  const T Q4 = nu / de;
+  const T R_d = wbT * shfl_t(Q4, 0);
+  const T beta_c = shfl_t(Q4, 1), y = shfl_t(Q4, 2);
   T sq3 = one;
   switch (lane) {
     case 0: sq3 = 1.0 + R_d; break;
@@ -686,13 +715,13 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   const T S3 = xsqrt(sq3), P3 = xpow(lane == 0 ? 1.0 + R_d : one, lane == 0 ? -0.75 : 1.0);
   const T C0 = shfl_t(S3, 0), C1 = shfl_t(S3, 1), x = shfl_t(S3, 2), C3 = shfl_t(P3, 0);
   // level 4
-  T lg4 = one;
-  if (lane == 0) lg4 = (C0 + C1) / (1.0 + sqeq);
-  if (lane == 1) lg4 = (x + 1.0) / (x - 1.0);
-  const T L4 = xlog(lg4);
+  nu = one, de = one;
+  if (lane == 0) nu = C0 + C1, de = 1.0 + sqeq;
+  if (lane == 1) nu = x + 1.0, de = x - 1.0;
+  const T L4 = xlog(nu / de);
   const T D0 = shfl_t(L4, 0), D1v = shfl_t(L4, 1);
   // level 5
-  const T sh_d = 2.0 / (3.0 * k_eq) * sq6 * D0;
+  const T sh_d = shq * sq6 * D0;
   const T G = eh_G(y, x, D1v);
   const T alpha_b = 2.07 * k_eq * sh_d * C3 * G;
   const T beta_node = 8.41 * A14;
@@ -713,12 +742,21 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   s[S_FC] = fc;
   s[S_LGQ] = lgq;
   s[S_LGKSILK] = lgks;
-  s[S_QINV] = 1.0 / (13.41 * k_eq);
-  s[S_ISH] = 1.0 / sh_d;
-  s[S_C142AC] = 14.2 / alpha_c;
+  nu = one, de = one;
+  switch (lane) {
+    case 0: de = 13.41 * k_eq; break;
+    case 1: de = sh_d; break;
+    case 2: nu = 14.2 * one, de = alpha_c; break;
+    case 3: nu = 0.328 * lg431 * w_b, de = w_m; break;
+    default: break;
+  }
+  const T Q5 = nu / de;
+  s[S_QINV] = shfl_t(Q5, 0);
+  s[S_ISH] = shfl_t(Q5, 1);
+  s[S_C142AC] = shfl_t(Q5, 2);
   // transfer.py:88-100
-  s[S_AGAM] = 1.0 - 0.328 * lg431 * w_b / w_m + 0.38 * lg223 * ((Ob / Om) * (Ob / Om));
-  s[S_NWQ] = T27 / (Om * h);
+  s[S_AGAM] = 1.0 - shfl_t(Q5, 3) + 0.38 * lg223 * (fb * fb);
+  s[S_NWQ] = nwq;
   s[S_TFNW] = T(p[0] * 0.0 + (nowiggle ? 1.0 : 0.0));
 }
 
