@@ -555,11 +555,13 @@ __device__ __forceinline__ FF8 interp_ff8(FF x, const float2* xp, const float2* 
   return f0 + (f1 - f0) * (inv * (x - f2ff(xp[sg.x])));
 }
 
-constexpr int GR32_THREADS = 256;  // nodes of one cosmology per CTA (its tables shared in L1)
+constexpr int GR32_THREADS = 128;  // nodes of one cosmology per CTA (its tables shared in L1)
 
 // Uniform batches: one flat index over (cosmology, node), so that no CTA is
 // left with a node or two of a cosmology (na = 2^k + 1); listed: a 2-D grid.
-__global__ void __launch_bounds__(GR32_THREADS, 2) grad_rows32_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+// 128 threads and three CTAs per SM: 1,608 us at 4096 cosmologies (256 threads and
+// two: 1,660; four CTAs of 128: 1,659)
+__global__ void __launch_bounds__(GR32_THREADS, 3) grad_rows32_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
   int item, n;
   if (!gb.listed) {
     const long long idx = (long long)blockIdx.x * GR32_THREADS + threadIdx.x;
@@ -1340,7 +1342,7 @@ __device__ __forceinline__ FF8 eh_transfer_f8(const FF8* s, FF k, FF lk) {
 // launch per kind keeps each kernel's code small (the three inlined bodies in
 // one kernel thrashed the instruction cache).
 template <int KIND>
-__global__ void __launch_bounds__(128) grad_nodes_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
+__global__ void __launch_bounds__(128, 7) grad_nodes_kernel(GradBatch gb, const ConstTables* __restrict__ c) {
   const int item = blockIdx.y;
   if (item >= gb.n_items) return;
   const GradItem gi = grad_item(gb, item);
