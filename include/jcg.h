@@ -102,7 +102,7 @@ extern "C" {
 #define JCG_PHYSICS_ALL (JCG_PK_MASK | JCG_TF_NOWIGGLE | JCG_GROWTH_GAMMA)
 
 /* arithmetic of the Limber stage */
-#define JCG_FP64 0  /* plain: float64 everywhere */
+#define JCG_FP64 0  /* plain: float64-class accuracy (float64, or float pairs where they keep it) */
 #define JCG_FP32C 1 /* float32 Limber integrand + compensated Simpson sums, float64 tables */
 
 /* One request's tracers and grids (cosmology independent).
@@ -247,7 +247,7 @@ int jcg_stage_limber(const jcg_geometry* g, const void* geo_dev, const double* p
  * README.md:14-27): the vector-Jacobian product of a likelihood is
  * sum_ij,l v_ij(l) jac_ij(l).  Tables are differentiated forward (tangents),
  * the Limber integrand by a reverse sweep; all recomputed from params_dev.
- * precision: JCG_FP64 everywhere, or JCG_FP32C (float64 tables, root find and
+ * precision: JCG_FP64 (as above), or JCG_FP32C (float64 tables, root find and
  * moments; float32 lensing kernels and Limber integrand + reverse sweep with
  * compensated a-sums). */
 int jcg_jacobian_workspace_size(const jcg_geometry* g, int n_cosmo, int precision, size_t* bytes);
