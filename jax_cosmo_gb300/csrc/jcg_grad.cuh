@@ -301,6 +301,12 @@ __device__ __forceinline__ float2* grad_kw64(TabD* t) {
 }
 __device__ __forceinline__ const float2* grad_kw64(const TabD* t) { return grad_kw64(const_cast<TabD*>(t)); }
 static_assert(sizeof(TabD) - offsetof(TabD, c32) >= sizeof(double) * (NDIR + 1) * (GRAD_NEH + NKH), "scratch fits");
+// Directions in which the background (distances in Mpc/h, H / h, growth, Omega(a))
+// has a tangent: all but h, n_s and sigma_8.  (The growth's tangent in gamma stands
+// in the direction gamma_dir, which may be one of these three.)
+__host__ __device__ constexpr bool bg_dir(int d) { return d < 2 || d > 4; }
+constexpr int NBG = 5;
+__host__ __device__ constexpr int bg_dir_of(int i) { return i < 2 ? i : i + 3; }
 // FP64 rows and radial kernels with tangents (jcg_gradrows64.cu,
 // jcg_gradkern64.cu); only_wide: of the
 // cosmologies with TabD::wide set

@@ -3,8 +3,8 @@
 //
 //   grad_wlsum64_kernel   the z' integral of the WeakLensing bins.  With
 //     r = (chi' - chi) / chi',   dr = (chi / chi'^2) dchi' - dchi / chi'
-//     a bin's sum, its 8 tangent sums A_d = sum W (chi / chi'^2) dchi'_d and
-//     B = sum W / chi' (dK_d = A_d - dchi_d B) are ten sums of products in float
+//     a bin's sum, its tangent sums A_d = sum W (chi / chi'^2) dchi'_d and
+//     B = sum W / chi' (dK_d = A_d - dchi_d B) are sums of products in float
 //     pairs (jcg_px.cuh), weights scaled per (node, bin) as in jcg_tracer64.cu.  A
 //     warp per (cosmology, node), points over lanes, three bins at a time in
 //     registers (a warp per pass); the lanes' sums are added by one lane per sum.
@@ -13,9 +13,10 @@
 //
 // One kernel did both in Dual<8> float64 (a warp per node, the second part on 8
 // of its lanes): 61 cosmologies, 3 + 2 bins with alignment terms, 513 nodes
-// 5.00 -> 0.57 + 0.31 ms; one cosmology, 5 + 5 bins 208 -> 40 + 12 us.  The first
-// is bound by issue (some 500 instructions a point and three bins), the second
-// by the FP64 pipe (pow, exp and log of its terms).
+// 5.00 -> 0.47 + 0.23 ms; one cosmology, 5 + 5 bins 208 -> 30 + 12 us (all eight
+// directions: 0.57 ms and 40 us; four bins a pass: 0.51 ms and 38 us).  The first
+// is bound by issue (some 400 instructions a point and three bins), the second by
+// the FP64 pipe.
 #include "jcg_grad.cuh"
 #include "jcg_px.cuh"
 #include "jcg_wl64.cuh"
@@ -24,11 +25,11 @@ namespace jcg {
 
 constexpr int GK_WARPS = 8;
 constexpr int GK_BINS = 3;             // bins per pass
-constexpr int GK_SUMS = NDIR + 2;      // r, A_d, B
+constexpr int GK_SUMS = NBG + 2;       // r, A_d of the background's directions, B
 constexpr int GK_PAD = 33;
 struct GkSmem {
   float2 chi[NCHI], slope[NCHI];
-  float2 dchi[NDIR][NCHI], dslope[NDIR][NCHI];
+  float2 dchi[NBG][NCHI], dslope[NBG][NCHI];
   float chi3[NCHI];
   double atab[NCHI];
   float2 runs[GK_WARPS][GK_BINS * GK_SUMS][GK_PAD];
@@ -56,8 +57,9 @@ __global__ void __launch_bounds__(GK_WARPS * 32, 2)
     S.slope[i] = make_float2(b.hi, b.lo);
     S.atab[i] = c->atab_chi[i];
 #pragma unroll
-    for (int d = 0; d < NDIR; ++d) {
-      const FF e = px_of(tb->chid[d][i]), f = px_of((tb->chid[d][k + 1] - tb->chid[d][k]) * ida);
+    for (int d = 0; d < NBG; ++d) {
+      const double* cd = tb->chid[bg_dir_of(d)];
+      const FF e = px_of(cd[i]), f = px_of((cd[k + 1] - cd[k]) * ida);
       S.dchi[d][i] = make_float2(e.hi, e.lo);
       S.dslope[d][i] = make_float2(f.hi, f.lo);
     }
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(GK_WARPS * 32, 2)
             we[u] = make_float2(x.hi, x.lo);
           }
 #pragma unroll
-          for (int d = 0; d < NDIR; ++d) {
+          for (int d = 0; d < NBG; ++d) {
             const FF dc = px_add(px_f2(S.dchi[d][sg.x]), px_mul(px_f2(S.dslope[d][seg]), dx));
 #pragma unroll
             for (int u = 0; u < GK_BINS; ++u) {
@@ -173,15 +175,23 @@ __global__ void __launch_bounds__(GK_WARPS * 32, 2)
           v = scalbn(px_d3(tot), S.exps[warp][u] - 1023);
         }
         const double B = __shfl_sync(0xffffffffu, v, min(u * GK_SUMS + GK_SUMS - 1, 31));
-        const double dw = __shfl_sync(0xffffffffu, cw.d[0], (s + 7) & 7);
-        if (u < nb && s <= NDIR) {
+        const double dw = __shfl_sync(0xffffffffu, cw.d[0], bg_dir_of(s > 0 && s <= NBG ? s - 1 : 0));
+        if (u < nb && s <= NBG) {
           int t = tl[0];
 #pragma unroll
           for (int q = 1; q < GK_BINS; ++q)
             if (q == u) t = tl[q];
           // a row with a non-finite weight: summed in float64 by the other kernel
           if (S.exps[warp][u] == 0x7ff) v = __longlong_as_double(0x7ff8000000000000LL);
-          gi.kernd[((size_t)t * na + n) * (NDIR + 1) + s] = s == 0 ? v : cwf * v - dw * B;
+          double* K = gi.kernd + ((size_t)t * na + n) * (NDIR + 1);
+          if (s == 0) {
+            K[0] = v;
+#pragma unroll
+            for (int d = 0; d < NDIR; ++d)
+              if (!bg_dir(d)) K[1 + d] = 0.0;
+          } else {
+            K[1 + bg_dir_of(s - 1)] = cwf * v - dw * B;
+          }
         }
         __syncwarp();
       }

@@ -10,22 +10,25 @@
 //   grad_pack64_kernel    the rows and kernels, in place, as the fixed point
 //     numbers and pairs the nodes read;
 //   grad_limber64_kernel  the integral.
+// Tangents that are 0 by the nature of the input (background inputs in the
+// directions of h, n_s and sigma_8) are neither read nor multiplied.
 //
 // A CTA takes a tile of LT ell and a range of the a nodes of one cosmology.  Per
 // chunk of TA nodes: a thread per (a, ell) node evaluates S and its tangents into
 // shared memory; then, in blocks of MB nodes, the weights M_p = K_i K_j V with
 // tangents are formed from the kernels, and a thread per (spectrum, ell) adds
-// the 17 products of its value and tangents in pairs and adds the block to
+// the 14 products of its value and tangents in pairs and adds the block to
 // three-float totals.
 //
-// 10 tracers (55 spectra), 200 ell, 513 nodes, one cosmology: 1,195 -> 178 us and
-// 26 us for the two packing kernels; 61 cosmologies, 15 spectra, 97 ell: 14.6 ->
-// 1.81 ms and 0.15.  Bound by the latency of FP32 chains (8,000 instructions a
-// node, 220 per spectrum and node; 4 warps per scheduler at 128 registers, 0.4 to
-// 0.5 instructions per cycle; three CTAs an SM spill: 1.92 ms).  Three-float totals in the node and runs
-// of 4 nodes cost 20% of that and bring the tangents' error, which cancelling
-// terms amplify, below the float64 kernels' on the former tables (1.46e-15 and
-// 2.27e-15 of their norm against 1.58e-15 and 2.75e-15, by 80-bit arithmetic).
+// 10 tracers (55 spectra), 200 ell, 513 nodes, one cosmology: 1,195 -> 161 us and
+// 22 us for the two packing kernels; 61 cosmologies, 15 spectra, 97 ell: 14.6 ->
+// 1.63 ms and 0.15 (with the zero tangents 178 us and 1.81 ms).  Bound by the
+// latency of FP32 chains (7,700 instructions a node, 190 per spectrum and node; 4
+// warps per scheduler at 128 registers, 0.4 to 0.5 instructions per cycle; three
+// CTAs an SM spill: slower).  Three-float totals in the node and runs of 4 nodes
+// cost 20% of that and bring the tangents' error, which cancelling terms amplify,
+// below the float64 kernels' on the former tables (1.5e-15 and 2.4e-15 of their
+// norm against 1.6e-15 and 2.8e-15, by 80-bit arithmetic).
 //
 // Numbers out of the range that float pairs hold, or a spectrum that lives where
 // its kernels are below 2^-66 of their largest value, set TabD::wide: that
@@ -162,9 +165,7 @@ __global__ void __launch_bounds__(GXS_THREADS) grad_scale64_kernel(GradBatch gb)
     if (nw && x > GC_NWQ) bad = false;
     sc->g.dT[x][d] = px3_of(v);
   }
-  if (t < NDIR) {
-    sc->g.dns[t] = px3_of(tb->sd[t][S_NS]);
-  }
+  if (t == 0) sc->g.dns = px3_of(tb->sd[GX_NS][S_NS]);
   if (bad) tb->wide = 1;
 }
 
@@ -350,6 +351,10 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
   for (int i = tid; i < (int)(sizeof(GxTabs) / 8); i += GX_THREADS)
     reinterpret_cast<double*>(&g)[i] = reinterpret_cast<const double*>(&sc->g)[i];
   const int units = lt * n_cls;
+  // kernels and weights have tangents in the background's directions, and in
+  // gamma's (the growth factor in a bias)
+  const int gd = gb.gamma_dir;
+  auto has = [&](int d) { return bg_dir(d) || d == gd; };
   for (int i = tid; i < 3 * (NDIR + 1) * units; i += GX_THREADS) tot[i] = 0.f;
   __syncthreads();
   bool bad = false;
@@ -390,6 +395,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
         o[NDIR + 1] = k0;
 #pragma unroll
         for (int d = 1; d <= NDIR; ++d) {
+          if (!has(d - 1)) continue;
           const float2 kd = K[d];
           float ah = 0.f, al = 0.f;
           ff_acc_prod(ah, al, kd, v0);
@@ -410,6 +416,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
         o[0] = make_float2(w.hi, w.lo);
 #pragma unroll
         for (int d = 1; d <= NDIR; ++d) {
+          if (!has(d - 1)) continue;
           float ah = 0.f, al = 0.f;
           ff_acc_prod(ah, al, A[d], b0);
           ff_acc_prod(ah, al, a0, B[d]);
@@ -433,7 +440,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
 #pragma unroll
             for (int s = 1; s <= NDIR; ++s) {
               ff_acc_prod(ah[s], al[s], pp[s * LT], w0);
-              ff_acc_prod(ah[s], al[s], p0, mm[s]);
+              if (has(s - 1)) ff_acc_prod(ah[s], al[s], p0, mm[s]);
             }
           }
 #pragma unroll

@@ -33,12 +33,13 @@ static_assert(GR_T % 2 == 0, "tangents are read 16 bytes at a time");
 // ln sh_d, alpha_gamma's ln and ln of the q factor)
 enum GxCos { GC_SH = 0, GC_KEQ, GC_BETAC, GC_ALPHAC, GC_ALPHAB, GC_BETAB, GC_BETANODE, GC_KSILK, GC_FB, GC_FC, GC_N };
 constexpr int GC_AGAM = GC_KEQ, GC_NWQ = GC_BETAC;
+constexpr int GX_NS = 3;  // the direction of n_s
 
 struct GxTabs {
   PxCos c;
   F3 cab;                 // 14.2 / alpha_c
   F3 dT[GC_N][4];         // tangents in directions 0..2
-  F3 dns[NDIR];           // of n_s
+  F3 dns;                 // of n_s, in its direction
 };
 
 struct GxT {  // T / f_c and its partials in the logarithms of GxCos and of k
@@ -168,13 +169,15 @@ __device__ __forceinline__ void gx_acc(F3& a, FF w, F3 b) {
   const FF u = px_two_sum(t.hi, fmaf(w.hi, b.hi, -p));
   a = F3{s.hi, u.hi, a.ll + ((t.lo + u.lo) + fmaf(w.lo, b.hi, fmaf(w.hi, b.lo, w.hi * b.ll)))};
 }
-// dS += w x the 8 tangents at d
+// dS += w x the 8 tangents at d; BG: an input of the background alone
+template <bool BG>
 __device__ __forceinline__ void gx_mac(GxAcc& a, FF w, const float2* d) {
 #pragma unroll
   for (int q = 0; q < NDIR / 2; ++q) {
+    if (BG && !bg_dir(2 * q) && !bg_dir(2 * q + 1)) continue;
     const float4 v = reinterpret_cast<const float4*>(d)[q];
-    gx_acc(a.a[2 * q], w, make_float2(v.x, v.y));
-    gx_acc(a.a[2 * q + 1], w, make_float2(v.z, v.w));
+    if (!BG || bg_dir(2 * q)) gx_acc(a.a[2 * q], w, make_float2(v.x, v.y));
+    if (!BG || bg_dir(2 * q + 1)) gx_acc(a.a[2 * q + 1], w, make_float2(v.z, v.w));
   }
 }
 
@@ -213,17 +216,17 @@ __device__ __forceinline__ void px_node_grad(const GxTabs& g, const PxTab& T, co
     const FF iD = px_rcp2(px_add(px_1p(B), G)), in = px_rcp2(px_add(y2, nm));
     const FF h = px_mul(px_mul(H, y2), px_mul(iD, in));
     const FF hD = px_mul(h, iD), hB = px_neg(px_mul(hD, B)), hG = px_neg(px_mul(hD, G));
-    gx_mac(acc, h, tan + GT_AN * NDIR);
-    gx_mac(acc, hB, tan + GT_BN * NDIR);
-    gx_mac(acc, hG, tan + GT_G0 * NDIR);
-    gx_mac(acc, px_mul(h, lyn), tan + GT_E1 * NDIR);
-    gx_mac(acc, px_mul(hB, lyn), tan + GT_E2 * NDIR);
-    gx_mac(acc, px_mul(hG, lyn), tan + GT_E3 * NDIR);
+    gx_mac<false>(acc, h, tan + GT_AN * NDIR);
+    gx_mac<false>(acc, hB, tan + GT_BN * NDIR);
+    gx_mac<false>(acc, hG, tan + GT_G0 * NDIR);
+    gx_mac<true>(acc, px_mul(h, lyn), tan + GT_E1 * NDIR);
+    gx_mac<true>(acc, px_mul(hB, lyn), tan + GT_E2 * NDIR);
+    gx_mac<false>(acc, px_mul(hG, lyn), tan + GT_E3 * NDIR);
     const FF hn = px_mul(h, in);
     {
       FF w = hn;
       if (GEN) w = px_mul(hn, px_add(FF{1.f, 0.f}, px_mul(y, px_f2(rf[GR_MUC]))));
-      gx_mac(acc, px_neg(w), tan + GT_NU * NDIR);
+      gx_mac<false>(acc, px_neg(w), tan + GT_NU * NDIR);
     }
     // d h / d ln y
     FF wy = px_add(px_mul(h, px_unfix60(row[GR_E1])), px_mul(hB, px_unfix60(row[GR_E2])));
@@ -240,21 +243,19 @@ __device__ __forceinline__ void px_node_grad(const GxTabs& g, const PxTab& T, co
       const FF sa = px_mul(px_mul(s, d2l), ia);  // s d2l / (1 + alpha d2l)
       const FF sy = px_mul(s, px_add(y, y2));
       wy = px_sub(wy, FF{0.25f * sy.hi, 0.25f * sy.lo});
-      gx_mac(acc, px_neg(sa), tan + GT_ALPHA * NDIR);
-      gx_mac(acc, px_mul(s, px_mul(px_unfix60(ld), pxc(8.0 * 0.693147180559945309417))), tan + GT_BETA * NDIR);
+      gx_mac<false>(acc, px_neg(sa), tan + GT_ALPHA * NDIR);
+      gx_mac<false>(acc, px_mul(s, px_mul(px_unfix60(ld), pxc(8.0 * 0.693147180559945309417))), tan + GT_BETA * NDIR);
       wl = px_add(s, px_mul(s, px_mul(px_unfix60(row[GR_BETA]), px_div(d2l, d1))));
       wl = px_sub(wl, px_mul(sa, px_f2(rf[GR_ALPHA])));
       S = px_add(s, h);
     }
-    gx_mac(acc, wy, tan + GT_Y * NDIR);
+    gx_mac<false>(acc, wy, tan + GT_Y * NDIR);
   }
-  gx_mac(acc, wl, tan + GT_A * NDIR);
+  gx_mac<false>(acc, wl, tan + GT_A * NDIR);
   const FF wT = px_x2(px_div(wl, px_of(tr.t)));  // T may be below 0
   const FF nk = px_add(px_mul(wl, px_unfix60(g.c.ns3)), px_mul(wT, tr.k));
-  gx_mac(acc, nk, tan + GT_K * NDIR);
-  const FF ws = px_mul(wl, px_mul(px_unfix60(lk), pxc(8.0 * 0.693147180559945309417)));
-#pragma unroll
-  for (int d = 0; d < NDIR; ++d) gx_acc(acc.a[d], ws, g.dns[d]);
+  gx_mac<true>(acc, nk, tan + GT_K * NDIR);
+  gx_acc(acc.a[GX_NS], px_mul(wl, px_mul(px_unfix60(lk), pxc(8.0 * 0.693147180559945309417))), g.dns);
 #pragma unroll
   for (int x = 0; x < GC_N; ++x) {
     if (GEN && nw && x > GC_NWQ) break;

@@ -63,3 +63,21 @@ def test_chi_below_one():
     """zmax of 5e-4: comoving distances of 0 to 1.5 Mpc/h, k of 10 to 10^4."""
     p = [jc.probes.WeakLensing([jc.redshift.smail_nz(1.0, 2.0, 2e-4, zmax=5e-4)], sigma_e=0.26)]
     check(p, [O.Probe("wl", [O.Smail(1.0, 2.0, 2e-4, 5e-4, 1.0)], sigma_e=0.26)], 16)
+
+
+@pytest.mark.parametrize("gamma_dir", [2, 3, 4])
+def test_gamma_in_a_direction_without_background(gamma_dir):
+    """d C_ell / d gamma does not depend on the direction that carries it: in those of h,
+    n_s and sigma_8 the kernels' tangents are otherwise left out.  Biases with the
+    growth factor give the kernels a tangent in gamma."""
+    from jax_cosmo_gb300 import _lib
+    from jax_cosmo_gb300.autodiff import jacobian_device
+
+    nz = [jc.redshift.smail_nz(1.0, 2.0, z, zmax=4.0) for z in (0.5, 0.9)]
+    p = [jc.probes.WeakLensing(nz[:1], ia_bias=jc.bias.inverse_growth_linear_bias(0.7)),
+         jc.probes.NumberCounts(nz[1:], jc.bias.inverse_growth_linear_bias(1.3))]
+    params = torch.tensor([ROW + [0.55]], dtype=torch.float64, device="cuda")
+    _, a = jacobian_device(params, ELL, p, 64, "fp64", _lib.GROWTH_GAMMA, gamma_dir=0)
+    _, b = jacobian_device(params, ELL, p, 64, "fp64", _lib.GROWTH_GAMMA, gamma_dir=gamma_dir)
+    ref, got = a[0, ..., 0], b[0, ..., gamma_dir]
+    assert float(((got - ref).abs().amax(-1) / ref.abs().amax(-1)).max()) < 2e-12
