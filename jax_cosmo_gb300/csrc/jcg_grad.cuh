@@ -307,6 +307,9 @@ static_assert(sizeof(TabD) - offsetof(TabD, c32) >= sizeof(double) * (NDIR + 1) 
 __host__ __device__ constexpr bool bg_dir(int d) { return d < 2 || d > 4; }
 constexpr int NBG = 5;
 __host__ __device__ constexpr int bg_dir_of(int i) { return i < 2 ? i : i + 3; }
+// P(k) at a = 1 and sigma^2(R) have tangents in the first five directions (Omega_c,
+// Omega_b, h, n_s, sigma_8)
+constexpr int NPW = 5;
 // FP64 rows and radial kernels with tangents (jcg_gradrows64.cu,
 // jcg_gradkern64.cu); only_wide: of the
 // cosmologies with TabD::wide set

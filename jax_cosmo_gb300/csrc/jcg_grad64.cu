@@ -13,7 +13,7 @@
 //     their tangents' affine maps, a warp per component;
 //   grad_sigma64_kernel   sigma8's weighted sum, P(k) k^3 and sigma^2(R): a CTA per
 //     component and quarter of the R nodes.
-// One cosmology 1,453 -> 57 us (23 + 23 + 11); what is left is latency: serial float64 code of
+// One cosmology 1,453 -> 55 us (21 + 23 + 10); what is left is latency: serial float64 code of
 // a thread and the scans.
 #include "jcg_grad.cuh"
 #include "jcg_px.cuh"
@@ -137,7 +137,7 @@ __device__ __forceinline__ void eh_nodes64(TabD* tb, const ConstTables* c, int j
   const double a[NX] = {g.keq, g.sh, g.betac, g.alphac, g.alphab, g.betab, g.betanode, g.ksilk, g.fb, g.fc, g.agam,
                         g.nwq, 0.0};
 #pragma unroll
-  for (int d = 0; d < NDIR; ++d) {
+  for (int d = 0; d < NPW; ++d) {
     double x = 0.0;
 #pragma unroll
     for (int q = 0; q < NX - 1; ++q) x = fma(a[q], dl[q][d], x);
@@ -388,6 +388,15 @@ __global__ void __launch_bounds__(SG64_THREADS) grad_sigma64_kernel(GradBatch gb
   const int comp = blockIdx.x % (NDIR + 1), part = blockIdx.x / (NDIR + 1), t = threadIdx.x;
   const double* u = eh_scratch(tb);
   const double* ud = u + comp * NEH;
+  if (comp > NPW) {
+    // no tangent: the tables' zeros
+    for (int i = part * SG64_R + t; t < SG64_R && i < NRT; i += NRT) tb->sigd[comp - 1][i] = 0.0;
+    if (part == 0) {
+      for (int i = t; i < NKH; i += SG64_THREADS) tb->pk3d[comp - 1][i] = 0.0;
+      if (t == 0) tb->sd[comp - 1][S_SIGMASQR8] = tb->sd[comp - 1][S_PKNORM] = 0.0;
+    }
+    return;
+  }
   __shared__ double sums[4][SG64_R], norm[2];
   __shared__ double pq[NKH];
   const double i2 = 1.0 / (2.0 * (PI * PI));

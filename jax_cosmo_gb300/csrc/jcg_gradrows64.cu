@@ -4,14 +4,14 @@
 //     halofit's moments (power.py:121-139), a warp per node in float pairs
 //     (jcg_px.cuh):
 //       S1 = 2 sum w y^2 e^{-y^2},  S2 = 4 sum w (y^2 - y^4) e^{-y^2},  y = k R,
-//     the same sums with dw_d for w, and S3 = 8 sum w y^2 (1 - 3 y^2 + y^4)
+//     the same sums with dw_d for w (five directions), and S3 = 8 sum w y^2 (1 - 3 y^2 + y^4)
 //     e^{-y^2}: dS1 = S1[dw_d] + S2 dln R, dS2 = S2[dw_d] + S3 dln R;
 //   grad_rowfin64_kernel    the coefficients (power.py:177-242) and the Limber
 //     weight: values once, tangents in closed form, in float64.
 //
 // One kernel did both, 32 lanes of (node, direction) in Dual<1> float64: the
 // coefficients' exponentials eight times over, the moments on the FP64 pipe.
-// One cosmology, 513 nodes 200 -> 17 + 26 us, 61 cosmologies 1,260 -> 142 + 128
+// One cosmology, 513 nodes 200 -> 15 + 26 us, 61 cosmologies 1,260 -> 131 + 128
 // us; the second kernel is bound by the FP64 pipe, the first by issue.
 #include "jcg_grad.cuh"
 #include "jcg_px_node.cuh"
@@ -20,10 +20,10 @@ namespace jcg {
 
 constexpr int GR64_WARPS = 8;
 constexpr int GR64_NODES = 64;             // nodes per CTA at most
-constexpr int GR64_SUMS = 2 * (NDIR + 1) + 1;
+constexpr int GR64_SUMS = 2 * (NPW + 1) + 1;
 struct Gr64Smem {
   PxTab T;
-  float2 w[NDIR + 1][NKH], kh2[NKH];
+  float2 w[NPW + 1][NKH], kh2[NKH];
   double sig[NRT];
   float2 runs[GR64_WARPS][GR64_SUMS][33];
   double R[GR64_NODES];
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(GR64_WARPS * 32)
     reinterpret_cast<uint4*>(&S.T)[i] = reinterpret_cast<const uint4*>(&c->px)[i];
   for (int i = tid; i < NRT; i += GR64_WARPS * 32) S.sig[i] = tb->sigv[i];
   __syncthreads();
-  for (int i = tid; i < (NDIR + 1) * NKH; i += GR64_WARPS * 32) {
+  for (int i = tid; i < (NPW + 1) * NKH; i += GR64_WARPS * 32) {
     const float2 v = kw[i];
     S.w[0][i] = v;
     // outside what the pairs hold: float64 terms
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(GR64_WARPS * 32)
     const double R = S.R[t];
     double* row = gi.rowd + (size_t)(n0 + t) * NROWD;
     if (S.wide) {
-      if (lane < NDIR + 1) {
+      if (lane < NPW + 1) {
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         for (int i = 0; i < NKH; ++i) {
           const double y = c->kh[i] * R, y2 = y * y;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(GR64_WARPS * 32)
           s3 += 8.0 * (r * (1.0 - 3.0 * y2 + y2 * y2));
         }
         row[lane] = s1;
-        row[NDIR + 1 + lane] = s2;
+        row[NPW + 1 + lane] = s2;
         if (lane == 0) row[GR64_SUMS - 1] = s3;
       }
       continue;
@@ -119,10 +119,10 @@ __global__ void __launch_bounds__(GR64_WARPS * 32)
       const float2 v1 = make_float2(f1.hi, f1.lo), v2 = make_float2(f2.hi, f2.lo);
       ff_acc_prod(ah[GR64_SUMS - 1], al[GR64_SUMS - 1], S.w[0][i], make_float2(f3.hi, f3.lo));
 #pragma unroll
-      for (int d = 0; d <= NDIR; ++d) {
+      for (int d = 0; d <= NPW; ++d) {
         const float2 w = S.w[d][i];
         ff_acc_prod(ah[d], al[d], w, v1);
-        ff_acc_prod(ah[NDIR + 1 + d], al[NDIR + 1 + d], w, v2);
+        ff_acc_prod(ah[NPW + 1 + d], al[NPW + 1 + d], w, v2);
       }
     }
 #pragma unroll
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(GR64_WARPS * 32)
     if (lane < GR64_SUMS) {
       F3 tot{0.f, 0.f, 0.f};
       for (int r = 0; r < 32; ++r) px_acc3(tot, px_f2(S.runs[warp][lane][r]));
-      row[lane] = px_d3(tot) * (lane <= NDIR ? 2.0 : lane < GR64_SUMS - 1 ? 4.0 : 8.0);
+      row[lane] = px_d3(tot) * (lane <= NPW ? 2.0 : lane < GR64_SUMS - 1 ? 4.0 : 8.0);
     }
     __syncwarp();
   }
@@ -154,9 +154,13 @@ __global__ void __launch_bounds__(64)
   const int d0 = grp * ND;
   const int model = pk_model(geo->physics);
   double* row = gi.rowd + (size_t)n * NROWD;
-  double S1 = row[0], S2 = row[NDIR + 1], S3 = row[GR64_SUMS - 1], S1d[ND], S2d[ND];
+  double S1 = row[0], S2 = row[NPW + 1], S3 = row[GR64_SUMS - 1], S1d[ND], S2d[ND];
 #pragma unroll
-  for (int q = 0; q < ND; ++q) S1d[q] = row[1 + d0 + q], S2d[q] = row[NDIR + 2 + d0 + q];
+  for (int q = 0; q < ND; ++q) {
+    const int d = d0 + q;
+    S1d[q] = d < NPW ? row[1 + d] : 0.0;
+    S2d[q] = d < NPW ? row[NPW + 2 + d] : 0.0;
+  }
   const int seg = (int)row[GR64_SUMS];
   const double g = row[GR64_SUMS + 1];
   __syncwarp();
