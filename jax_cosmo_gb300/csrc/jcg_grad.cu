@@ -1543,14 +1543,14 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
                                  : dim3((unsigned)(((long long)gb.na * gb.n_items + GR32_THREADS - 1) / GR32_THREADS));
       grad_rows32_kernel<<<grw, GR32_THREADS, 0, st>>>(gb, c);
     } else {
-      launch_grad_rows64(gb, c, st, 0);
+      launch_grad_front64(gb, c, st, 0, 1, (stages & GS_KERNELS) != 0);
     }
   }
   if (stages & GS_KERNELS) {
     if (gb.precision == JCG_FP32C) {
       launch_grad_kern32(gb, c, st);
     } else {
-      launch_grad_kern64(gb, c, st, 0);
+      if (!(stages & GS_ROWS)) launch_grad_front64(gb, c, st, 0, 0, 1);  // else with the rows
     }
   }
 }
@@ -1562,8 +1562,7 @@ void launch_grad(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
   } else {
     launch_grad_limber64(gb, c, st);
     // cosmologies out of the pairs' range: rows, kernels and integral in float64
-    launch_grad_rows64(gb, c, st, 1);
-    launch_grad_kern64(gb, c, st, 1);
+    launch_grad_front64(gb, c, st, 1, 1, 1);
     const int lt = grad_limber_tile(gb.n_ell, gb.n_cls);
     const size_t sml = grad_limber_smem(gb.n_cls, lt);
     cudaFuncSetAttribute(grad_limber_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sml);

@@ -310,11 +310,9 @@ __host__ __device__ constexpr int bg_dir_of(int i) { return i < 2 ? i : i + 3; }
 // P(k) at a = 1 and sigma^2(R) have tangents in the first five directions (Omega_c,
 // Omega_b, h, n_s, sigma_8)
 constexpr int NPW = 5;
-// FP64 rows and radial kernels with tangents (jcg_gradrows64.cu,
-// jcg_gradkern64.cu); only_wide: of the
-// cosmologies with TabD::wide set
-void launch_grad_rows64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
-void launch_grad_kern64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide);
+// FP64 rows and radial kernels with tangents (jcg_gradfront64.cu); only_wide: of the
+// cosmologies with TabD::wide set; rows, kern: which of the two
+void launch_grad_front64(const GradBatch& gb, const ConstTables* c, cudaStream_t st, int only_wide, int rows, int kern);
 // FP64 Limber integral with tangents in float pairs (jcg_gradlim64.cu)
 void launch_grad_limber64(const GradBatch& gb, const ConstTables* c, cudaStream_t st);
 int grad_limber64_tile(int n_ell, int n_cls);
