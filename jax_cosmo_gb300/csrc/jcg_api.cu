@@ -532,8 +532,7 @@ int jcg_angular_cl(const jcg_geometry* g, const void* geo, const double* params,
   if (!cl) return fail(JCG_ERR_ARG, "cl output is NULL");
   const Batch b = make_batch(&h, geo, params, n_cosmo, precision, ws, cl);
   launch_cosmo_tables(b, c, stream);
-  launch_halofit_rows(b, c, stream);
-  launch_tracer_kernels(b, c, stream);
+  launch_rows_tracers(b, c, stream);
   launch_limber(b, c, limber_tile(h.n_ell), stream);
   return cuda_check("angular_cl");
 }
@@ -823,8 +822,7 @@ extern "C" int jcg_angular_cl_noalloc(const jcg_geometry* g, const void* geo, co
   if ((rc = const_tables_on(stream, &c))) return rc;
   const Batch b = make_batch(&h, geo, params, n_cosmo, precision, scratch, cl);
   launch_cosmo_tables(b, c, stream);
-  launch_halofit_rows(b, c, stream);
-  launch_tracer_kernels(b, c, stream);
+  launch_rows_tracers(b, c, stream);
   launch_limber(b, c, limber_tile(h.n_ell), stream);
   return cuda_check("angular_cl_noalloc");
 }
@@ -942,8 +940,7 @@ extern "C" int jcg_angular_cl_host(const jcg_geometry* g, const void* geo, const
     return cuda_check("angular_cl_host parameters");
   const Batch b = make_batch(&h, geo, dparams, n_cosmo, precision, ws, dcl);
   launch_cosmo_tables(b, c, stream);
-  launch_halofit_rows(b, c, stream);
-  launch_tracer_kernels(b, c, stream);
+  launch_rows_tracers(b, c, stream);
   int rb[JCG_HOST_SLICES + 1];
   const int ns = host_ranges(n_cosmo, rb), lt = limber_tile(h.n_ell);
   const size_t per = (size_t)h.n_cls * h.n_ell;
@@ -1222,8 +1219,7 @@ extern "C" int jcg_requests_run(const jcg_request* reqs, int n, int mode, int pr
     b.items = dev_items;
     b.precision = precision;
     launch_cosmo_tables(b, c, stream);
-    launch_halofit_rows(b, c, stream);
-    launch_tracer_kernels(b, c, stream);
+    launch_rows_tracers(b, c, stream);
     launch_limber(b, c, limber_tile(b.max_ell), stream);
     return cuda_check("requests angular_cl");
   }

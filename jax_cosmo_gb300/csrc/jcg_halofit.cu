@@ -11,22 +11,12 @@
 #include "jcg_ff.cuh"
 #include "jcg_internal.cuh"
 #include "jcg_dual.cuh"
-#include "jcg_px_node.cuh"
+#include "jcg_rows.cuh"
 
 namespace jcg {
 
-constexpr double TWO_PI2 = 2.0 * (PI * PI);  // 2.0 * np.pi**2
-constexpr double C2 = C_KMS * C_KMS;          // const.c**2
 
-struct HfParams {
-  double knl, neff, C;
-};
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // argmin_j (1 - sig_j g2)^2 with the first index on ties (scipy/interpolate.py:47).
 // v_j = sig_j g2 is strictly decreasing, so (1 - v_j)^2 is unimodal and the
@@ -220,13 +210,6 @@ __device__ void halofit_coefs_fast(const double* s, float om_m, float om_de, flo
   row[R_LGKNL] = 0.6931471805599453 * f[F_LG2KNL];
   row[R_LGCF3] = 0.6931471805599453 * f[F_LG2CF3];
   row[R_LGCHIC] = -0.6931471805599453 * f[F_LG2INVCHI];
-}
-
-// chi and growth at a from the tables (background.py:242, 488) with the
-// segment chosen by the reference's rule and the precomputed chi slopes.
-__device__ __forceinline__ double chi_at(const CosmoTab* ct, const ConstTables* c, double a, int2 seg) {
-  const int k = min(seg.x, seg.y);
-  return fmax(ct->chi[seg.x] + ct->chi_slope[k] * (a - c->atab_chi[seg.x]), 0.0);
 }
 
 constexpr int HF_WARPS = 8;
@@ -459,208 +442,6 @@ __global__ void __launch_bounds__(HF_WARPS * 32, 8)
   }
 }
 
-// The float64 rows, float64-class numbers on the FP32 pipe where the work is
-// (jcg_px.cuh).  Bound: issue.  The moments (power.py:121-136) take up to 257
-// exponentials per node, each 35 FP64 operations in float64 (9,000 per node, on
-// a pipe of 1/64 rate); a term in pairs is about 130 FP32 and integer
-// instructions.  Terms with y^2 > 60 are below 1e-20 of the sums and end the
-// loop (lanes walk k upwards).  The root find's decisions stay in float64.
-// Phases: a thread per node (growth, chi, root find), a warp per node (the
-// moments), a thread per node (coefficients, Limber weight; exponentials and
-// logarithms by the pair functions, sums in float64: 230 FP64 operations where
-// float64 functions made it 600).
-//   4096 cosmologies x 513 nodes: 52.3 -> 3.5 ms; one cosmology: 241 -> 17 us.
-constexpr int H64_NODES = 64;
-
-// exp(v) and log of positive v by the pair functions, as doubles
-__device__ __forceinline__ double px_expd(double v, const PxTab& T) {
-  return px_join(px_exp2(__double2ll_rn(v * (D_LOG2E * 9007199254740992.0)), T));
-}
-
-// halofit coefficients (power.py:177-244) into a row, as halofit_coefs
-__device__ void halofit_coefs64(double om_m, double om_de, double w, const HfParams& hp, double* row, int model,
-                                const PxTab& T) {
-  const double n = hp.neff, C = hp.C;
-  row[R_KNL] = hp.knl;
-  row[R_NEFF] = n;
-  row[R_C] = C;
-  row[R_OMM] = om_m;
-  row[R_OMDE] = om_de;
-  row[R_W] = w;
-  if (model != JCG_PK_TAKAHASHI2012) {
-    const HfCoef<double> h = hf_coefs<double>(model, n, C, om_m, om_de, w);
-    row[R_AN] = h.an, row[R_BN] = h.bn, row[R_CN] = h.cn, row[R_GAMMAN] = h.gam, row[R_ALPHAN] = h.alpha;
-    row[R_BETAN] = h.beta, row[R_NUN] = h.nu, row[R_MUN] = h.mu, row[R_F1] = h.f1, row[R_F2] = h.f2;
-    row[R_F3] = h.f3, row[R_LGCF3] = h.lcf3;
-    return;
-  }
-  constexpr double L10 = 2.302585092994046;
-  const double dw = om_de * (1.0 + w);
-  const double e_an = 1.5222 + n * (2.8553 + n * (2.3706 + n * (0.9903 + n * 0.2250))) - 0.6038 * C + 0.1749 * dw;
-  const double e_bn = -0.5642 + n * (0.5864 + n * 0.5716) - 1.5474 * C + 0.2279 * dw;
-  const double e_cn = 0.3698 + n * (2.0404 + n * 0.8161) + 0.5869 * C;
-  row[R_AN] = px_expd(L10 * e_an, T);
-  row[R_BN] = px_expd(L10 * e_bn, T);
-  row[R_CN] = px_expd(L10 * e_cn, T);
-  row[R_NUN] = px_expd(L10 * (5.2105 + 3.6902 * n), T);
-  row[R_GAMMAN] = 0.1971 - 0.0843 * n + 0.8460 * C;
-  row[R_ALPHAN] = fabs(6.0835 + n * (1.3373 - n * 0.1959) - 5.5274 * C);
-  row[R_BETAN] = 2.0379 + n * (-0.7354 + n * (0.3157 + n * (1.2490 + n * 0.3980))) - 0.1682 * C;
-  row[R_MUN] = 0.0;
-  // Omega_m^e, e = -0.0307, -0.0585, 0.0743, which scale exponents of P(k):
-  // e^x in float64 by its Taylor polynomial for |x| < 0.25 (Omega_m > 0.035)
-  const double lom = (double)px_log2_d(om_m, T) * (0.69314718055994530942 / 144115188075855872.0);
-  const double ex[3] = {-0.0307 * lom, -0.0585 * lom, 0.0743 * lom};
-  double f[3];
-  const bool small = om_m > 0.035 && om_m < 28.0;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const double x = ex[q];
-    double p = 1.0 / 479001600.0;
-    p = fma(p, x, 1.0 / 39916800.0);
-    p = fma(p, x, 1.0 / 3628800.0);
-    p = fma(p, x, 1.0 / 362880.0);
-    p = fma(p, x, 1.0 / 40320.0);
-    p = fma(p, x, 1.0 / 5040.0);
-    p = fma(p, x, 1.0 / 720.0);
-    p = fma(p, x, 1.0 / 120.0);
-    p = fma(p, x, 1.0 / 24.0);
-    p = fma(p, x, 1.0 / 6.0);
-    p = fma(p, x, 0.5);
-    p = fma(p, x, 1.0);
-    f[q] = fma(p, x, 1.0);
-  }
-  if (!small) {
-    const double l = log(om_m);
-    f[0] = exp(-0.0307 * l), f[1] = exp(-0.0585 * l), f[2] = exp(0.0743 * l);
-  }
-  row[R_F1] = f[0];
-  row[R_F2] = f[1];
-  row[R_F3] = f[2];
-  row[R_LGCF3] = L10 * e_cn + (small ? ex[2] : log(f[2]));
-}
-
-__global__ void __launch_bounds__(HF_WARPS * 32, 5)
-    halofit_rows64_kernel(Batch bt, const ConstTables* __restrict__ c, int nb) {
-  const int item = blockIdx.y;
-  const Item it = batch_item(bt, item);
-  const GeoHeader* geo = it.geo;
-  const int na = geo->na, n0 = blockIdx.x * nb;
-  if (n0 >= na) return;
-  const int cnt = min(na - n0, nb);
-  const int model = pk_model(it.physics);
-  const CosmoTab* ct = it.ctab;
-  __shared__ __align__(16) PxTab T;
-  __shared__ double sig[NRT], s[NSCAL];
-  __shared__ float2 wpk[NKH], kh2[NKH];
-  __shared__ double knl_s[H64_NODES], inv_s[H64_NODES], lgk_s[H64_NODES], g_s[H64_NODES], chi_s[H64_NODES], s1_s[H64_NODES],
-      s2_s[H64_NODES];
-  __shared__ int wide;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < (int)(sizeof(PxTab) / 16); i += HF_WARPS * 32)
-    reinterpret_cast<uint4*>(&T)[i] = reinterpret_cast<const uint4*>(&c->px)[i];
-  for (int i = tid; i < NRT; i += HF_WARPS * 32) sig[i] = ct->sig[i];
-  for (int i = tid; i < NSCAL; i += HF_WARPS * 32) s[i] = ct->s[i];
-  if (tid == 0) wide = 0;
-  __syncthreads();
-  for (int i = tid; i < NKH; i += HF_WARPS * 32) {
-    const float2 w = ct->rtay[0][i];  // w_i P(k_i) k_i^3 / (2 pi^2), written by the float64 table stage
-    wpk[i] = w;
-    kh2[i] = make_float2(c->kh2_hi[i], c->kh2_lo[i]);
-    if (!(w.x > 1e-28f && w.x < 1e28f)) wide = 1;  // outside what the pairs below hold: float64 terms
-  }
-  const double* A = geo_ptr<double>(geo, geo->off_a);
-  const double* WS = geo_ptr<double>(geo, geo->off_wsimp);
-  const int64_t* SC = geo_ptr<int64_t>(geo, geo->off_seg_chi);
-  const int64_t* SG = geo_ptr<int64_t>(geo, geo->off_seg_grow);
-  // growth, chi and the root find (power.py:96-118)
-  for (int t = tid; t < cnt; t += HF_WARPS * 32) {
-    const int n = n0 + t;
-    const double a = A[n];
-    const int2 sg = unpack_seg(SG[n]);
-    const double sl = (ct->g[sg.y] - ct->g[sg.x]) * c->grow_ida[min(sg.x, sg.y)] * (sg.y > sg.x ? 1.0 : -1.0);
-    const double g = clip_lohi(ct->g[sg.x] + sl * (a - c->atab_grow[sg.x]), 0.0, 1.0);
-    const double g2 = g * g;
-    int ind, j2;
-    root_segment(sig, g2, ind, j2);
-    const double xp = sig[ind] * g2;
-    double root = c->logr[ind] + (c->logr[j2] - c->logr[ind]) / (sig[j2] * g2 - xp) * (1.0 - xp);
-    double R = exp(root);
-    if (!(R >= 1e-6)) R = R < 1e-6 ? 1e-6 : R, root = log(R);  // power.py:113-115
-    g_s[t] = g;
-    inv_s[t] = R;
-    knl_s[t] = 1.0 / R;
-    lgk_s[t] = -root;
-    chi_s[t] = chi_at(ct, c, a, unpack_seg(SC[n]));
-    if (!(R < 1e6)) wide = 1;
-  }
-  __syncthreads();
-  // the moments
-  if (model != JCG_PK_LINEAR) {
-    for (int t = warp; t < cnt; t += HF_WARPS) {
-      double s1, s2;
-      const double R = inv_s[t];
-      if (!wide) {
-        const FF R2 = px_split(R * R);
-        FF a1{0.f, 0.f}, a2{0.f, 0.f};  // at most 9 terms per lane
-        for (int i = lane; i < NKH; i += 32) {
-          const FF y2 = px_mul(R2, px_f2(kh2[i]));
-          if (y2.hi > 60.f) break;
-          const FF e = px_exp2(-px_fix53(px_mul(y2, pxc(D_LOG2E))), T);
-          const FF r = px_mul(px_mul(px_f2(wpk[i]), e), y2);
-          a1 = px_add(a1, r);
-          a2 = px_add(a2, px_mul(r, px_1p(FF{-y2.hi, -y2.lo})));
-        }
-        __syncwarp();
-        s1 = 2.0 * warp_sum(px_join(a1));
-        s2 = 4.0 * warp_sum(px_join(a2));
-      } else {
-        s1 = s2 = 0.0;
-        for (int i = lane; i < NKH; i += 32) {
-          const double y = c->kh[i] * R, y2 = y * y;
-          const double r = ct->pk3[i] * exp(-y2) / TWO_PI2;
-          s1 += c->simpson_kh[i] * (2 * r * y2);
-          s2 += c->simpson_kh[i] * (4 * r * (y2 - y2 * y2));
-        }
-        s1 = warp_sum(s1);
-        s2 = warp_sum(s2);
-      }
-      if (lane == 0) s1_s[t] = s1, s2_s[t] = s2;
-    }
-  }
-  __syncthreads();
-  // coefficients and the Limber weight
-  for (int t = tid; t < cnt; t += HF_WARPS * 32) {
-    const int n = n0 + t;
-    const double a = A[n], g2 = g_s[t] * g_s[t];
-    double row[NROW64];
-    for (int i = 0; i < NROW64; ++i) row[i] = 0.0;
-    // background (background.py:122-126, 168, 196, 270-294)
-    const double ia = px_ddiv(1.0, a, px_rcp(px_hi(a)));
-    const double lna = (double)px_log2_d(a, T) * (0.69314718055994530942 / 144115188075855872.0);
-    const double fde = -3.0 * (1.0 + s[S_W0] + s[S_WA]) * lna + 3.0 * s[S_WA] * (a - 1.0);
-    const double ef = fde == 0.0 ? 1.0 : exp(fde);
-    const double ia2 = ia * ia, om3 = s[S_OMEGA_M] * (ia2 * ia), ode = s[S_OMEGA_DE] * ef;
-    const double e2 = om3 + s[S_OMEGA_K] * ia2 + ode;
-    const double ie2 = 1.0 / e2;
-    const double chi = chi_s[t], dchi = RH * ia2 * rsqrt(e2);
-    HfParams hp;
-    hp.knl = knl_s[t];
-    const double s1 = model == JCG_PK_LINEAR ? 0.0 : s1_s[t] * g2;
-    hp.neff = s1 - 3.0;  // power.py:138-139
-    hp.C = model == JCG_PK_LINEAR ? 0.0 : s1 * s1 + s2_s[t] * g2;
-    halofit_coefs64(om3 * ie2, ode * ie2, s[S_W0] + (1.0 - a) * s[S_WA], hp, row, model, T);
-    row[R_CHI] = chi;
-    row[R_G] = g_s[t];
-    row[R_LGKNL] = lgk_s[t];
-    row[R_LGCHIC] = log(fmax(chi, 1.0));
-    row[R_DCHI] = dchi;
-    row[R_U] = WS[n] * dchi / fmax(chi * chi, 1.0) * (1.0 / C2);
-    double* dst = it.rows64 + (size_t)n * NROW64;
-    for (int i = 0; i < NROW64; ++i) dst[i] = row[i];
-  }
-}
-
 void launch_halofit_rows(const Batch& b, const ConstTables* c, cudaStream_t st) {
   if (b.precision == JCG_FP32C) {
     dim3 grid((b.max_na + HF_NODES - 1) / HF_NODES, b.n_items);
@@ -668,10 +449,7 @@ void launch_halofit_rows(const Batch& b, const ConstTables* c, cudaStream_t st) 
     halofit_rows_kernel<<<grid, HF_WARPS * 32, 0, st>>>(b, c);
     return;
   }
-  // few CTAs: fewer nodes each, so that the batch spreads over the SMs
-  int nb = H64_NODES;
-  while (nb > 8 && (long long)b.n_items * ((b.max_na + nb - 1) / nb) < 2 * device_sm_count()) nb >>= 1;
-  halofit_rows64_kernel<<<dim3((b.max_na + nb - 1) / nb, b.n_items), HF_WARPS * 32, 0, st>>>(b, c, nb);
+  launch_rows64(b, c, st);
 }
 
 // ------------------------------------------------------ pointwise queries ---

@@ -854,6 +854,9 @@ __device__ __forceinline__ void ku_get_rec(const float4* rec, int& q, float& dx,
 
 void launch_tracer_kernels(const Batch& b, const ConstTables* c, cudaStream_t st);
 void launch_tracer64(const Batch& b, const ConstTables* c, cudaStream_t st);
+void launch_rows64(const Batch& b, const ConstTables* c, cudaStream_t st);
+// launch_halofit_rows and launch_tracer_kernels
+void launch_rows_tracers(const Batch& b, const ConstTables* c, cudaStream_t st);
 void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st);
 void launch_limber64(const Batch& b, const ConstTables* c, cudaStream_t st);
 // derivatives (jcg_grad.cu)

@@ -1,5 +1,5 @@
-// Tracer radial kernels of the plain method (precision "fp64") on the Limber
-// nodes (probes.py:16-129, 188-272): for a WeakLensing bin
+// Tracer radial kernels and halofit rows of the plain method (precision "fp64") on
+// the Limber nodes.  Rows: see there.  Kernels (probes.py:16-129, 188-272): for a WeakLensing bin
 //   q(z) = simps_{z' in [z, zmax], 256}[ n(z') clip(chi' - chi, 0) / clip(chi', 1) ] (1 + z) chi
 // times 3 H0^2 Omega_m / (2 c) and (1 + m), plus the NLA term; for a
 // NumberCounts bin n(z) b H(z).
@@ -22,6 +22,9 @@
 // 5 bins, 513 nodes, 4096 cosmologies: 30.6 -> 3.5 ms; one cosmology, 2 bins, 257
 // nodes: 82 -> 15 us; 5 + 5 bins, 513 nodes: 195 -> 28 us.
 #include "jcg_internal.cuh"
+#include "jcg_dual.cuh"
+#include "jcg_px_node.cuh"
+#include "jcg_rows.cuh"
 #include "jcg_wl64.cuh"
 
 namespace jcg {
@@ -96,19 +99,31 @@ __device__ __forceinline__ double tracer_value(const GeoHeader* geo, const Cosmo
 }
 
 // ------------------------------------------------- a warp per (item, node) --
-__global__ void __launch_bounds__(T64_WARPS * 32, 4)
-    tracer64_kernel(Batch bt, const ConstTables* __restrict__ c, int per) {
-  const Item it = batch_item(bt, blockIdx.y);
+struct Tracer64Smem {
+  float2 chi[NCHI], slope[NCHI];
+  float chi3[NCHI];
+  double atab[NCHI];
+  float2 runs[T64_WARPS][T64_RUNS][MAXTR];
+  int exps[T64_WARPS][MAXTR];
+  double accs[MAXTR][T64_NODES], chis[T64_NODES];
+};
+
+__device__ __forceinline__ void tracer64(const Batch& bt, const ConstTables* __restrict__ c, int per, int block, int item,
+                                         unsigned char* smem) {
+  const Item it = batch_item(bt, item);
   const GeoHeader* geo = it.geo;
   const int na = geo->na, n_tr = geo->n_tr;
-  const int n0 = blockIdx.x * per;
+  const int n0 = block * per;
   if (n0 >= na) return;
-  __shared__ float2 chi[NCHI], slope[NCHI];
-  __shared__ float chi3[NCHI];
-  __shared__ double atab[NCHI];
-  __shared__ float2 runs[T64_WARPS][T64_RUNS][MAXTR];
-  __shared__ int exps[T64_WARPS][MAXTR];
-  __shared__ double accs[MAXTR][T64_NODES], chis[T64_NODES];
+  Tracer64Smem& S = *reinterpret_cast<Tracer64Smem*>(smem);
+  auto& chi = S.chi;
+  auto& slope = S.slope;
+  auto& chi3 = S.chi3;
+  auto& atab = S.atab;
+  auto& runs = S.runs;
+  auto& exps = S.exps;
+  auto& accs = S.accs;
+  auto& chis = S.chis;
   const CosmoTab* ct = it.ctab;
   for (int i = threadIdx.x; i < NCHI; i += blockDim.x) {
     const F3 a = px3_of(ct->chi[i]);
@@ -206,6 +221,239 @@ __global__ void __launch_bounds__(T64_WARPS * 32, 4)
       dz = node_D(geo, ct, c, n, awl);
     it.kern[(size_t)t * na + n] = tracer_value(geo, ct, c, t, n, accs[t][i], chis[i], Z[n], om, hz, dz);
   }
+}
+
+__global__ void __launch_bounds__(T64_WARPS * 32, 4)
+    tracer64_kernel(Batch bt, const ConstTables* __restrict__ c, int per) {
+  __shared__ __align__(16) unsigned char smem[sizeof(Tracer64Smem)];
+  tracer64(bt, c, per, blockIdx.x, blockIdx.y, smem);
+}
+
+// ---------------------------------------------------------- halofit rows ----
+// The float64 rows, float64-class numbers on the FP32 pipe where the work is
+// (jcg_px.cuh).  Bound: issue.  The moments (power.py:121-136) take up to 257
+// exponentials per node, each 35 FP64 operations in float64 (9,000 per node, on
+// a pipe of 1/64 rate); a term in pairs is about 130 FP32 and integer
+// instructions.  Terms with y^2 > 60 are below 1e-20 of the sums and end the
+// loop (lanes walk k upwards).  The root find's decisions stay in float64.
+// Phases: a thread per node (growth, chi, root find), a warp per node (the
+// moments), a thread per node (coefficients, Limber weight; exponentials and
+// logarithms by the pair functions, sums in float64: 230 FP64 operations where
+// float64 functions made it 600).
+//   4096 cosmologies x 513 nodes: 52.3 -> 3.5 ms; one cosmology: 241 -> 17 us.
+constexpr int H64_NODES = 64;
+
+// exp(v) and log of positive v by the pair functions, as doubles
+__device__ __forceinline__ double px_expd(double v, const PxTab& T) {
+  return px_join(px_exp2(__double2ll_rn(v * (D_LOG2E * 9007199254740992.0)), T));
+}
+
+// halofit coefficients (power.py:177-244) into a row, as halofit_coefs
+__device__ void halofit_coefs64(double om_m, double om_de, double w, const HfParams& hp, double* row, int model,
+                                const PxTab& T) {
+  const double n = hp.neff, C = hp.C;
+  row[R_KNL] = hp.knl;
+  row[R_NEFF] = n;
+  row[R_C] = C;
+  row[R_OMM] = om_m;
+  row[R_OMDE] = om_de;
+  row[R_W] = w;
+  if (model != JCG_PK_TAKAHASHI2012) {
+    const HfCoef<double> h = hf_coefs<double>(model, n, C, om_m, om_de, w);
+    row[R_AN] = h.an, row[R_BN] = h.bn, row[R_CN] = h.cn, row[R_GAMMAN] = h.gam, row[R_ALPHAN] = h.alpha;
+    row[R_BETAN] = h.beta, row[R_NUN] = h.nu, row[R_MUN] = h.mu, row[R_F1] = h.f1, row[R_F2] = h.f2;
+    row[R_F3] = h.f3, row[R_LGCF3] = h.lcf3;
+    return;
+  }
+  constexpr double L10 = 2.302585092994046;
+  const double dw = om_de * (1.0 + w);
+  const double e_an = 1.5222 + n * (2.8553 + n * (2.3706 + n * (0.9903 + n * 0.2250))) - 0.6038 * C + 0.1749 * dw;
+  const double e_bn = -0.5642 + n * (0.5864 + n * 0.5716) - 1.5474 * C + 0.2279 * dw;
+  const double e_cn = 0.3698 + n * (2.0404 + n * 0.8161) + 0.5869 * C;
+  row[R_AN] = px_expd(L10 * e_an, T);
+  row[R_BN] = px_expd(L10 * e_bn, T);
+  row[R_CN] = px_expd(L10 * e_cn, T);
+  row[R_NUN] = px_expd(L10 * (5.2105 + 3.6902 * n), T);
+  row[R_GAMMAN] = 0.1971 - 0.0843 * n + 0.8460 * C;
+  row[R_ALPHAN] = fabs(6.0835 + n * (1.3373 - n * 0.1959) - 5.5274 * C);
+  row[R_BETAN] = 2.0379 + n * (-0.7354 + n * (0.3157 + n * (1.2490 + n * 0.3980))) - 0.1682 * C;
+  row[R_MUN] = 0.0;
+  // Omega_m^e, e = -0.0307, -0.0585, 0.0743, which scale exponents of P(k):
+  // e^x in float64 by its Taylor polynomial for |x| < 0.25 (Omega_m > 0.035)
+  const double lom = (double)px_log2_d(om_m, T) * (0.69314718055994530942 / 144115188075855872.0);
+  const double ex[3] = {-0.0307 * lom, -0.0585 * lom, 0.0743 * lom};
+  double f[3];
+  const bool small = om_m > 0.035 && om_m < 28.0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double x = ex[q];
+    double p = 1.0 / 479001600.0;
+    p = fma(p, x, 1.0 / 39916800.0);
+    p = fma(p, x, 1.0 / 3628800.0);
+    p = fma(p, x, 1.0 / 362880.0);
+    p = fma(p, x, 1.0 / 40320.0);
+    p = fma(p, x, 1.0 / 5040.0);
+    p = fma(p, x, 1.0 / 720.0);
+    p = fma(p, x, 1.0 / 120.0);
+    p = fma(p, x, 1.0 / 24.0);
+    p = fma(p, x, 1.0 / 6.0);
+    p = fma(p, x, 0.5);
+    p = fma(p, x, 1.0);
+    f[q] = fma(p, x, 1.0);
+  }
+  if (!small) {
+    const double l = log(om_m);
+    f[0] = exp(-0.0307 * l), f[1] = exp(-0.0585 * l), f[2] = exp(0.0743 * l);
+  }
+  row[R_F1] = f[0];
+  row[R_F2] = f[1];
+  row[R_F3] = f[2];
+  row[R_LGCF3] = L10 * e_cn + (small ? ex[2] : log(f[2]));
+}
+
+struct Rows64Smem {
+  PxTab T;
+  double sig[NRT], s[NSCAL];
+  float2 wpk[NKH], kh2[NKH];
+  double knl_s[H64_NODES], inv_s[H64_NODES], lgk_s[H64_NODES], g_s[H64_NODES], chi_s[H64_NODES], s1_s[H64_NODES],
+      s2_s[H64_NODES];
+  int wide;
+};
+
+__device__ __forceinline__ void rows64(const Batch& bt, const ConstTables* __restrict__ c, int nb, int block, int item,
+                                       unsigned char* smem) {
+  const Item it = batch_item(bt, item);
+  const GeoHeader* geo = it.geo;
+  const int na = geo->na, n0 = block * nb;
+  if (n0 >= na) return;
+  const int cnt = min(na - n0, nb);
+  const int model = pk_model(it.physics);
+  const CosmoTab* ct = it.ctab;
+  Rows64Smem& S = *reinterpret_cast<Rows64Smem*>(smem);
+  PxTab& T = S.T;
+  double *sig = S.sig, *s = S.s, *knl_s = S.knl_s, *inv_s = S.inv_s, *lgk_s = S.lgk_s, *g_s = S.g_s, *chi_s = S.chi_s,
+         *s1_s = S.s1_s, *s2_s = S.s2_s;
+  float2 *wpk = S.wpk, *kh2 = S.kh2;
+  int& wide = S.wide;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < (int)(sizeof(PxTab) / 16); i += T64_WARPS * 32)
+    reinterpret_cast<uint4*>(&T)[i] = reinterpret_cast<const uint4*>(&c->px)[i];
+  for (int i = tid; i < NRT; i += T64_WARPS * 32) sig[i] = ct->sig[i];
+  for (int i = tid; i < NSCAL; i += T64_WARPS * 32) s[i] = ct->s[i];
+  if (tid == 0) wide = 0;
+  __syncthreads();
+  for (int i = tid; i < NKH; i += T64_WARPS * 32) {
+    const float2 w = ct->rtay[0][i];  // w_i P(k_i) k_i^3 / (2 pi^2), written by the float64 table stage
+    wpk[i] = w;
+    kh2[i] = make_float2(c->kh2_hi[i], c->kh2_lo[i]);
+    if (!(w.x > 1e-28f && w.x < 1e28f)) wide = 1;  // outside what the pairs below hold: float64 terms
+  }
+  const double* A = geo_ptr<double>(geo, geo->off_a);
+  const double* WS = geo_ptr<double>(geo, geo->off_wsimp);
+  const int64_t* SC = geo_ptr<int64_t>(geo, geo->off_seg_chi);
+  const int64_t* SG = geo_ptr<int64_t>(geo, geo->off_seg_grow);
+  // growth, chi and the root find (power.py:96-118)
+  for (int t = tid; t < cnt; t += T64_WARPS * 32) {
+    const int n = n0 + t;
+    const double a = A[n];
+    const int2 sg = unpack_seg(SG[n]);
+    const double sl = (ct->g[sg.y] - ct->g[sg.x]) * c->grow_ida[min(sg.x, sg.y)] * (sg.y > sg.x ? 1.0 : -1.0);
+    const double g = clip_lohi(ct->g[sg.x] + sl * (a - c->atab_grow[sg.x]), 0.0, 1.0);
+    const double g2 = g * g;
+    int ind, j2;
+    root_segment(sig, g2, ind, j2);
+    const double xp = sig[ind] * g2;
+    double root = c->logr[ind] + (c->logr[j2] - c->logr[ind]) / (sig[j2] * g2 - xp) * (1.0 - xp);
+    double R = exp(root);
+    if (!(R >= 1e-6)) R = R < 1e-6 ? 1e-6 : R, root = log(R);  // power.py:113-115
+    g_s[t] = g;
+    inv_s[t] = R;
+    knl_s[t] = 1.0 / R;
+    lgk_s[t] = -root;
+    chi_s[t] = chi_at(ct, c, a, unpack_seg(SC[n]));
+    if (!(R < 1e6)) wide = 1;
+  }
+  __syncthreads();
+  // the moments
+  if (model != JCG_PK_LINEAR) {
+    for (int t = warp; t < cnt; t += T64_WARPS) {
+      double s1, s2;
+      const double R = inv_s[t];
+      if (!wide) {
+        const FF R2 = px_split(R * R);
+        FF a1{0.f, 0.f}, a2{0.f, 0.f};  // at most 9 terms per lane
+        for (int i = lane; i < NKH; i += 32) {
+          const FF y2 = px_mul(R2, px_f2(kh2[i]));
+          if (y2.hi > 60.f) break;
+          const FF e = px_exp2(-px_fix53(px_mul(y2, pxc(D_LOG2E))), T);
+          const FF r = px_mul(px_mul(px_f2(wpk[i]), e), y2);
+          a1 = px_add(a1, r);
+          a2 = px_add(a2, px_mul(r, px_1p(FF{-y2.hi, -y2.lo})));
+        }
+        __syncwarp();
+        s1 = 2.0 * warp_sum(px_join(a1));
+        s2 = 4.0 * warp_sum(px_join(a2));
+      } else {
+        s1 = s2 = 0.0;
+        for (int i = lane; i < NKH; i += 32) {
+          const double y = c->kh[i] * R, y2 = y * y;
+          const double r = ct->pk3[i] * exp(-y2) / TWO_PI2;
+          s1 += c->simpson_kh[i] * (2 * r * y2);
+          s2 += c->simpson_kh[i] * (4 * r * (y2 - y2 * y2));
+        }
+        s1 = warp_sum(s1);
+        s2 = warp_sum(s2);
+      }
+      if (lane == 0) s1_s[t] = s1, s2_s[t] = s2;
+    }
+  }
+  __syncthreads();
+  // coefficients and the Limber weight
+  for (int t = tid; t < cnt; t += T64_WARPS * 32) {
+    const int n = n0 + t;
+    const double a = A[n], g2 = g_s[t] * g_s[t];
+    double row[NROW64];
+    for (int i = 0; i < NROW64; ++i) row[i] = 0.0;
+    // background (background.py:122-126, 168, 196, 270-294)
+    const double ia = px_ddiv(1.0, a, px_rcp(px_hi(a)));
+    const double lna = (double)px_log2_d(a, T) * (0.69314718055994530942 / 144115188075855872.0);
+    const double fde = -3.0 * (1.0 + s[S_W0] + s[S_WA]) * lna + 3.0 * s[S_WA] * (a - 1.0);
+    const double ef = fde == 0.0 ? 1.0 : exp(fde);
+    const double ia2 = ia * ia, om3 = s[S_OMEGA_M] * (ia2 * ia), ode = s[S_OMEGA_DE] * ef;
+    const double e2 = om3 + s[S_OMEGA_K] * ia2 + ode;
+    const double ie2 = 1.0 / e2;
+    const double chi = chi_s[t], dchi = RH * ia2 * rsqrt(e2);
+    HfParams hp;
+    hp.knl = knl_s[t];
+    const double s1 = model == JCG_PK_LINEAR ? 0.0 : s1_s[t] * g2;
+    hp.neff = s1 - 3.0;  // power.py:138-139
+    hp.C = model == JCG_PK_LINEAR ? 0.0 : s1 * s1 + s2_s[t] * g2;
+    halofit_coefs64(om3 * ie2, ode * ie2, s[S_W0] + (1.0 - a) * s[S_WA], hp, row, model, T);
+    row[R_CHI] = chi;
+    row[R_G] = g_s[t];
+    row[R_LGKNL] = lgk_s[t];
+    row[R_LGCHIC] = log(fmax(chi, 1.0));
+    row[R_DCHI] = dchi;
+    row[R_U] = WS[n] * dchi / fmax(chi * chi, 1.0) * (1.0 / C2);
+    double* dst = it.rows64 + (size_t)n * NROW64;
+    for (int i = 0; i < NROW64; ++i) dst[i] = row[i];
+  }
+}
+
+__global__ void __launch_bounds__(T64_WARPS * 32, 5)
+    halofit_rows64_kernel(Batch bt, const ConstTables* __restrict__ c, int nb) {
+  __shared__ __align__(16) unsigned char smem[sizeof(Rows64Smem)];
+  rows64(bt, c, nb, blockIdx.x, blockIdx.y, smem);
+}
+
+// Rows and kernels need the tables only: few cosmologies run both in one launch,
+// CTAs of either kind side by side.
+__global__ void __launch_bounds__(T64_WARPS * 32, 4)
+    rows_tracer64_kernel(Batch bt, const ConstTables* __restrict__ c, int nb, int per, int row_ctas) {
+  __shared__ __align__(16) unsigned char
+      smem[sizeof(Tracer64Smem) > sizeof(Rows64Smem) ? sizeof(Tracer64Smem) : sizeof(Rows64Smem)];
+  if ((int)blockIdx.x < row_ctas) rows64(bt, c, nb, blockIdx.x, blockIdx.y, smem);
+  else tracer64(bt, c, per, (int)blockIdx.x - row_ctas, blockIdx.y, smem);
 }
 
 // --------------------------------------------- lanes over 32 cosmologies ----
@@ -381,6 +629,32 @@ void launch_tracer64(const Batch& b, const ConstTables* c, cudaStream_t st) {
   }
   const int per = t64_nodes(b.max_na, b.n_items);
   tracer64_kernel<<<dim3((b.max_na + per - 1) / per, b.n_items), T64_WARPS * 32, 0, st>>>(b, c, per);
+}
+
+// rows per CTA: as many as pay for the tables; fewer while the CTAs do not fill the SMs
+static int rows64_nodes(const Batch& b) {
+  int nb = H64_NODES;
+  while (nb > 8 && (long long)b.n_items * ((b.max_na + nb - 1) / nb) < 2 * device_sm_count()) nb >>= 1;
+  return nb;
+}
+void launch_rows64(const Batch& b, const ConstTables* c, cudaStream_t st) {
+  const int nb = rows64_nodes(b);
+  halofit_rows64_kernel<<<dim3((b.max_na + nb - 1) / nb, b.n_items), T64_WARPS * 32, 0, st>>>(b, c, nb);
+}
+
+void launch_rows_tracers(const Batch& b, const ConstTables* c, cudaStream_t st) {
+  if (b.precision != JCG_FP32C) {
+    const int nb = rows64_nodes(b), per = t64_nodes(b.max_na, b.n_items);
+    const int rows = (b.max_na + nb - 1) / nb, tr = (b.max_na + per - 1) / per;
+    // while all CTAs fit the SMs at once, two each (257 nodes, 2 bins: 17 us
+    // against 17 + 16; 513 nodes, 10 tracers: 34 against 22 + 27)
+    if ((long long)b.n_items * (rows + tr) <= 2 * device_sm_count()) {
+      rows_tracer64_kernel<<<dim3(rows + tr, b.n_items), T64_WARPS * 32, 0, st>>>(b, c, nb, per, rows);
+      return;
+    }
+  }
+  launch_halofit_rows(b, c, st);
+  launch_tracer_kernels(b, c, st);
 }
 
 }  // namespace jcg

@@ -1,4 +1,4 @@
-// What the float64 lensing integrals (jcg_tracer64.cu, jcg_gradkern64.cu) share:
+// What the float64 lensing integrals (jcg_tracer64.cu, jcg_gradfront64.cu) share:
 // pairs of signed and scaled doubles, and comoving distances from the node.
 #pragma once
 
