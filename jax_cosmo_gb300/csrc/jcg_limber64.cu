@@ -9,7 +9,7 @@
 // FP64 (the sums that pairs would round most), which keeps both pipes busy: FP64
 // 70%, issue slots 58% (608 cosmologies).  5 lensing bins, 100 ell, 513
 // nodes: 4096 cosmologies 171.8 -> 16.5 ms; one cosmology, 2 bins, 50 ell, 257
-// nodes 894 -> 29 us (clusters: seven times the CTAs).  Against 80-bit arithmetic
+// nodes 894 -> 26 us (clusters: seven times the CTAs).  Against 80-bit arithmetic
 // on the same rows the C_ell are off by 0.6e-15 rms (float64: 0.5e-15), below
 // what the tables upstream leave.
 //
@@ -358,7 +358,14 @@ static void launch_limber64_t(const Batch& b, const ConstTables* c, cudaStream_t
   const long long ctas = (long long)b.n_items * ((b.max_ell + lt - 1) / lt);
   if (ctas < 2 * sms) {
     R = nblk < PX_MAXCL ? nblk : PX_MAXCL;
-    while (lt > 8 && (long long)b.n_items * ((b.max_ell + lt - 1) / lt) * R < 2 * sms) lt = even((lt + 1) / 2);
+    const int bsz = (b.max_na + nblk - 1) / nblk;
+    auto count = [&](int l) { return (long long)b.n_items * ((b.max_ell + l - 1) / l) * R; };
+    while (lt > 8 && count(lt) < 2 * sms) lt = even((lt + 1) / 2);
+    // a node per thread in each block where clusters are small and the CTAs still fit
+    // at once (50 ell, 257 nodes, clusters of 4: lt 7 29 us, 3 25.8; 513 nodes, of 8:
+    // 31.4 and 34.5, so not there)
+    const int one = even(PX_THREADS / bsz > 1 ? PX_THREADS / bsz : 1);
+    if (R < PX_MAXCL && one < lt && lt <= 8 && count(one) <= 2 * sms) lt = one;
     const int slots = (nblk + R - 1) / R;
     if (px_layout(b.max_cls, lt, slots).total > 220 * 1024) R = 1;
   }
