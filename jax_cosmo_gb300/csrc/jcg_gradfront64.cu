@@ -174,20 +174,24 @@ __device__ __forceinline__ void rowfin64(const GradBatch& gb, const ConstTables*
   const int na = geo->na;
   const int idx = block * 64 + threadIdx.x, n_raw = idx / NG, grp = idx % NG;
   const bool live = n_raw < na;
-  const int n = live ? n_raw : na - 1;  // the rest of the last warp evaluates a valid node, writes nothing
+  const int n = live ? n_raw : na - 1;  // the rest of the last warp reads and writes no row
   constexpr int ND = NDIR / NG;
   const int d0 = grp * ND;
   const int model = pk_model(geo->physics);
   double* row = gi.rowd + (size_t)n * NROWD;
-  double S1 = row[0], S2 = row[NPW + 1], S3 = row[GR64_SUMS - 1], S1d[ND], S2d[ND];
+  double S1 = 0.0, S2 = 0.0, S3 = 0.0, g = 0.0, S1d[ND], S2d[ND];
+  int seg = 0;
+  if (live) {
+    S1 = row[0], S2 = row[NPW + 1], S3 = row[GR64_SUMS - 1];
 #pragma unroll
-  for (int q = 0; q < ND; ++q) {
-    const int d = d0 + q;
-    S1d[q] = d < NPW ? row[1 + d] : 0.0;
-    S2d[q] = d < NPW ? row[NPW + 2 + d] : 0.0;
+    for (int q = 0; q < ND; ++q) {
+      const int d = d0 + q;
+      S1d[q] = d < NPW ? row[1 + d] : 0.0;
+      S2d[q] = d < NPW ? row[NPW + 2 + d] : 0.0;
+    }
+    seg = (int)row[GR64_SUMS];
+    g = row[GR64_SUMS + 1];
   }
-  const int seg = (int)row[GR64_SUMS];
-  const double g = row[GR64_SUMS + 1];
   __syncwarp();
   if (!live) return;
   const double* s = tb->sv;

@@ -198,43 +198,50 @@ __global__ void __launch_bounds__(GXP_THREADS) grad_pack64_kernel(GradBatch gb, 
   const PxTab& T = c->px;
   const int lane = threadIdx.x & 31, dir = lane & 7;
   const int n_raw = ((int)blockIdx.x * (GXP_THREADS / 32) + (threadIdx.x >> 5)) * 4 + (lane >> 3);
-  const int n = min(n_raw, na - 1);
-  double* R = gi.rowd + (size_t)n * NROWD;
+  const bool live = n_raw < na;  // a slot past the last node reads and writes nothing
+  double* R = gi.rowd + (size_t)min(n_raw, na - 1) * NROWD;
   const bool lin = pk_model(geo->physics) == JCG_PK_LINEAR;
   double v[NA_IN], d[NA_IN];
 #pragma unroll
-  for (int i = 0; i < NA_IN; ++i) v[i] = R[i], d[i] = R[NA_IN * (1 + dir) + i];
+  for (int i = 0; i < NA_IN; ++i) v[i] = live ? R[i] : 1.0, d[i] = live ? R[NA_IN * (1 + dir) + i] : 0.0;
   __syncwarp();
   const double fc = tb->sv[S_TFNW] != 0.0 ? 1.0 : tb->sv[S_FC];
   const double pn = tb->sv[S_PKNORM], g = v[A_G], chic = v[A_CHIC];
-  if (n_raw < na) {
-    long long* row = reinterpret_cast<long long*>(R);
-    float2* rf = reinterpret_cast<float2*>(R);
-    auto in = [&](double x, double lo, double hi) {
-      bad |= !(x > lo && x < hi);
-      return x;
-    };
-    auto pair = [&](int i, double x) {
-      bad |= !(fabs(x) < 1e15);
-      const FF f = px_of(x);
-      rf[i] = make_float2(f.hi, f.lo);
-    };
-    // one logarithm and one exponent per lane
-    double lx = 1.0, ex = 0.0;
+  auto in = [&](double x, double lo, double hi) {
+    bad |= !(x > lo && x < hi);
+    return x;
+  };
+  // one logarithm per lane; ln k_nl goes from dir 5 to dir 1, all 32 lanes taking part
+  double lx = 1.0;
+  if (live) {
     if (dir == 0 || dir == 1) lx = in(chic, 1e-9, 1e9);
     if (dir == 4) lx = in(g * g * pn * (fc * fc * (1.0 / (2.0 * (PI * PI)))), 1e-18, 1e18);
     if (!lin) {
       if (dir == 2) lx = in(v[A_AN], 1e-18, 1e18);
       if (dir == 3) lx = in(v[A_BN], 1e-18, 1e18);
       if (dir == 5) lx = in(v[A_KNL], 1e-9, 1e9);
+    }
+  }
+  const long long lg = px_log2_d(lx, T);
+  const long long lknl = __shfl_down_sync(0xffffffffu, lg, 4);
+  if (live) {
+    long long* row = reinterpret_cast<long long*>(R);
+    float2* rf = reinterpret_cast<float2*>(R);
+    auto pair = [&](int i, double x) {
+      bad |= !(fabs(x) < 1e15);
+      const FF f = px_of(x);
+      rf[i] = make_float2(f.hi, f.lo);
+    };
+    // one exponent per lane
+    double ex = 0.0;
+    if (!lin) {
       if (dir == 0) ex = in(v[A_BETA], -7.9, 7.9);
       if (dir == 1) ex = in(3.0 * v[A_F1], -7.9, 7.9);
       if (dir == 2) ex = in(v[A_F2], -7.9, 7.9);
       if (dir == 3) ex = in(3.0 - v[A_GAM], -7.9, 7.9);
       if (dir == 4) ex = in(v[A_LCF3] * D_LOG2E, -30.0, 30.0) * 0.125;  // 2^-57 units
     }
-    const long long lg = px_log2_d(lx, T), fx = __double2ll_rn(ex * P2_60);
-    const long long lknl = __shfl_down_sync(__activemask(), lg, 4);  // to dir 1 from dir 5
+    const long long fx = __double2ll_rn(ex * P2_60);
     if (dir == 0) row[GR_L2C] = lg, row[GR_BETA] = fx;
     if (dir == 1) row[GR_L2Y] = lg + lknl, row[GR_E1] = fx;
     if (dir == 2) row[GR_A0] = lg >> 4, row[GR_E2] = fx;
