@@ -25,6 +25,7 @@ import ctypes
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from jax_cosmo_gb300 import _geometry, _lib
 
@@ -151,6 +152,20 @@ def _cov_index(n_tr, device):
     return blocks[:, 0], blocks[:, 1], blocks[:, 2], blocks[:, 3]
 
 
+def _values_only(g):
+    """Whether cotangent ``g`` can be handed to libjcg by its address: a tensor of
+    values alone, with no graph of the gradient asked for (``create_graph``), not a
+    batch of cotangents (``is_grads_batched``, a vectorised Jacobian), no forward
+    tangent.  The others are left to torch operations, which carry them on."""
+    if torch.is_grad_enabled() and g.requires_grad:
+        return False
+    try:
+        g.data_ptr()
+    except RuntimeError:  # a batched tensor has no storage of its own
+        return False
+    return forward_ad.unpack_dual(g).tangent is None
+
+
 class _Covariance(torch.autograd.Function):
     @staticmethod
     def forward(ctx, cl_signal, ell_t, n_tr, cl_noise, tracer_noise, f_sky, sparse):
@@ -168,7 +183,7 @@ class _Covariance(torch.autograd.Function):
         s3 = sig if batched else sig[None]
         g = gcov if batched else gcov[None]
         B, n_cls, n_ell = s3.shape
-        if not (torch.is_grad_enabled() and g.requires_grad):
+        if _values_only(g):
             cn = None
             if cl_noise is not None:
                 cn = torch.as_tensor(cl_noise, dtype=torch.float64).to(ell_t.device).expand(n_cls, n_ell).contiguous()
@@ -181,7 +196,6 @@ class _Covariance(torch.autograd.Function):
                       _lib.stream_of(ell_t.device))
             go = go.to(device=sig.device, dtype=sig.dtype)
             return (go if batched else go[0]), None, None, None, None, None, None
-        # a graph of the gradient is asked for: in torch operations
         if not sparse:  # the entries that depend on C_ell: the per-ell diagonals of each block
             g4 = g.reshape(B, n_cls, n_ell, n_cls, n_ell)
             idx = torch.arange(n_ell, device=g.device)
@@ -239,7 +253,7 @@ class _LogLike(torch.autograd.Function):
         g_C = None
         if ctx.needs_input_grad[2]:
             B = alpha.shape[0]
-            if sparse and not (torch.is_grad_enabled() and gout.requires_grad):
+            if sparse and _values_only(gout):
                 g_C = _sparse_inv_batched(C) if include_logdet else torch.empty_like(C)
                 _lib.call("jcg_gaussian_loglike_cov_grad", _lib.ptr(alpha), _lib.ptr(g_C) if include_logdet else None,
                           _lib.ptr(go.contiguous()), B, n_cls, n_ell, _lib.ptr(g_C), _lib.stream_of(C.device))
