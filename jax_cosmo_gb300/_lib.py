@@ -193,10 +193,18 @@ def call(name, *args):
 
 
 def ptr(t):
-    """Device pointer of a tensor (or None)."""
+    """Device pointer of a tensor (or None).
+
+    The pointer holds the tensor, so that an expression's temporary
+    (``ptr(x.contiguous())``) lives until the call it is passed to has returned:
+    freed before its kernels are queued, its memory could go to another thread that
+    allocates on the same stream meanwhile (a call releases the GIL).
+    """
     if t is None:
         return None
-    return ctypes.c_void_p(t.data_ptr())
+    p = ctypes.c_void_p(t.data_ptr())
+    p.tensor = t
+    return p
 
 
 def stream_of(device):
