@@ -91,6 +91,25 @@ static int const_tables(ConstTables** out) {
   return JCG_OK;
 }
 
+// ------------------------------------------------ shared-memory limits ------
+namespace jcg {
+void allow_smem(const void* kernel, size_t bytes) {
+  constexpr int KERNELS = 256, DEVICES = 64;  // instantiations of the library, as const_tables
+  static std::mutex mu;
+  static const void* known[KERNELS];
+  static size_t granted[KERNELS][DEVICES];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= DEVICES) return;  // the launch reports it
+  std::lock_guard<std::mutex> lk(mu);
+  int i = 0;
+  while (i < KERNELS - 1 && known[i] && known[i] != kernel) ++i;
+  known[i] = kernel;
+  if (granted[i][dev] >= bytes) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+    granted[i][dev] = bytes;
+}
+}  // namespace jcg
+
 // ------------------------------------------------ pinned staging ring -------
 // Small host tables (the item arrays of ragged requests) reach the device
 // through pinned host memory: a copy from pageable memory may wait for the

@@ -1527,7 +1527,7 @@ void launch_grad_front(const GradBatch& gb, const ConstTables* c, cudaStream_t s
   }
   if (gb.precision == JCG_FP32C) {
     const size_t smt = grad_tables_smem();
-    cudaFuncSetAttribute(grad_tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
+    allow_smem(grad_tables_kernel, smt);
     cudaFuncSetAttribute(grad_tables_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);  // four CTAs per SM
     grad_tables_kernel<<<gb.n_items, 128, smt, st>>>(gb, c);
@@ -1565,7 +1565,7 @@ void launch_grad(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
     launch_grad_front64(gb, c, st, 1, 1, 1);
     const int lt = grad_limber_tile(gb.n_ell, gb.n_cls);
     const size_t sml = grad_limber_smem(gb.n_cls, lt);
-    cudaFuncSetAttribute(grad_limber_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sml);
+    allow_smem(grad_limber_kernel, sml);
     dim3 gl((gb.n_ell + lt - 1) / lt, gb.n_split, gb.n_items);
     grad_limber_kernel<<<gl, GL_THREADS, sml, st>>>(gb, c, lt);
   }

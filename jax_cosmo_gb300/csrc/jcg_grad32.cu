@@ -480,10 +480,10 @@ void launch_grad_limber32(const GradBatch& gb, const ConstTables* c, cudaStream_
   const size_t smem = sizeof(float) * limber32_smem_floats(gb.n_cls, gb.n_tr, lt, ta);
   dim3 grid((gb.n_ell + lt - 1) / lt, gb.n_split, gb.n_items);
   if (gb.physics_or != 0) {
-    cudaFuncSetAttribute(grad_limber32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(grad_limber32_kernel<true>, smem);
     grad_limber32_kernel<true><<<grid, L32_THREADS, smem, st>>>(gb, c, lt, ta);
   } else {
-    cudaFuncSetAttribute(grad_limber32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(grad_limber32_kernel<false>, smem);
     grad_limber32_kernel<false><<<grid, L32_THREADS, smem, st>>>(gb, c, lt, ta);
   }
 }

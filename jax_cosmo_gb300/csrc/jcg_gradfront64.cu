@@ -636,14 +636,14 @@ void launch_grad_front64(const GradBatch& gb, const ConstTables* c, cudaStream_t
   // 83 in four launches); the cosmologies out of range (a rare case) always so
   if (only_wide || (rows && kern && gb.n_items * (long long)(mom + wl) <= 2 * sms)) {
     const size_t sm = sizeof(Gr64Smem) > sizeof(GkSmem) ? sizeof(Gr64Smem) : sizeof(GkSmem);
-    cudaFuncSetAttribute(grad_front64a_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(grad_front64a_kernel, sm);
     grad_front64a_kernel<<<dim3(wl + mom, gb.n_items), GK_WARPS * 32, sm, st>>>(gb, c, nb, per, wl, only_wide);
     const int rf = (gb.na * 4 + 63) / 64;
     grad_front64b_kernel<<<dim3(rf + kf * gb.n_tr, gb.n_items), GKF_THREADS, 0, st>>>(gb, c, rf, kf, only_wide);
     return;
   }
   if (rows) {
-    cudaFuncSetAttribute(grad_moments64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Gr64Smem));
+    allow_smem(grad_moments64_kernel, sizeof(Gr64Smem));
     grad_moments64_kernel<<<dim3(mom, gb.n_items), GR64_WARPS * 32, sizeof(Gr64Smem), st>>>(gb, c, nb);
     // two directions a thread while that leaves SMs idle (513 nodes: 26 us against 60
     // for all eight), all eight from there on (61 cosmologies: 128 us against 228)
@@ -654,7 +654,7 @@ void launch_grad_front64(const GradBatch& gb, const ConstTables* c, cudaStream_t
   }
   if (kern) {
     if (wl) {
-      cudaFuncSetAttribute(grad_wlsum64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GkSmem));
+      allow_smem(grad_wlsum64_kernel, sizeof(GkSmem));
       grad_wlsum64_kernel<<<dim3(wl, gb.n_items), GK_WARPS * 32, sizeof(GkSmem), st>>>(gb, c, per);
     }
     grad_kernfin64_kernel<<<dim3(kf, gb.n_tr, gb.n_items), GKF_THREADS, 0, st>>>(gb, c);

@@ -512,7 +512,7 @@ template <bool GEN>
 static void launch_limber64g(const GradBatch& gb, const ConstTables* c, cudaStream_t st) {
   const int lt = grad_limber64_tile(gb.n_ell, gb.n_cls);
   const size_t sm = gx_layout(gb.n_cls, gb.n_tr, lt).total;
-  cudaFuncSetAttribute(grad_limber64_kernel<GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  allow_smem(grad_limber64_kernel<GEN>, sm);
   grad_limber64_kernel<GEN><<<dim3((gb.n_ell + lt - 1) / lt, gb.n_split, gb.n_items), GX_THREADS, sm, st>>>(gb, c, lt);
 }
 

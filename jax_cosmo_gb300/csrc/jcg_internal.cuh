@@ -46,6 +46,15 @@ inline int device_sm_count() {
   return n;
 }
 
+// Lets launches of `kernel` ask for `bytes` of dynamic shared memory.  The limit is an
+// attribute of the kernel that all host threads share: it is only ever raised, so a
+// thread cannot take it below what another is about to launch with.
+void allow_smem(const void* kernel, size_t bytes);
+template <class F>
+inline void allow_smem(F* kernel, size_t bytes) {
+  allow_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 struct ConstTables {
   double atab_chi[NCHI];   // logspace(-3, 0, 256)
   double lna_chi[NCHI];    // log(atab_chi): the RK4 abscissae of background.py:231

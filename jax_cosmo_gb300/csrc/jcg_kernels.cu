@@ -264,8 +264,7 @@ __global__ void __launch_bounds__(256)
 template <int NW>
 static void launch_tu(const Batch& b, const ConstTables* c, cudaStream_t st) {
   const size_t smem = tu_smem(NCHI - b.chi_wbase, NW);
-  cudaFuncSetAttribute(tracer32_uniform_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+  allow_smem(tracer32_uniform_kernel<NW>, smem);
   dim3 grid((b.max_na + TU_NODES - 1) / TU_NODES, (b.n_items + 31) / 32);
   tracer32_uniform_kernel<NW><<<grid, 256, smem, st>>>(b, c);
 }

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(LB_THREADS, MAXU <= 1 ? 6 : (MAXU <= 3 ? 3 : 2
 template <int MAXU, bool GEN = false>
 static void launch_limber32_t(const Batch& b, const ConstTables* c, int lt, cudaStream_t st) {
   const L32Layout L = l32_layout(b.max_tr, b.max_cls, lt);
-  cudaFuncSetAttribute(limber32_kernel<MAXU, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+  allow_smem(limber32_kernel<MAXU, GEN>, L.total);
   dim3 grid((b.max_ell + lt - 1) / lt, b.n_items);
   limber32_kernel<MAXU, GEN><<<grid, LB_THREADS, L.total, st>>>(b, c, lt);
 }

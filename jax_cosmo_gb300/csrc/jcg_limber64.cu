@@ -371,7 +371,7 @@ static void launch_limber64_t(const Batch& b, const ConstTables* c, cudaStream_t
   }
   const int slots = R > 1 ? (nblk + R - 1) / R : 1;
   const PxLayout L = px_layout(b.max_cls, lt, slots);
-  cudaFuncSetAttribute(limber64_kernel<GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+  allow_smem(limber64_kernel<GEN>, L.total);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(R, (b.max_ell + lt - 1) / lt, b.n_items);
   cfg.blockDim = dim3(PX_THREADS);

@@ -504,7 +504,7 @@ void launch_loglike(const double* data, const double* mu, const double* cov, int
   const size_t smem = (5 * (size_t)n_cls + 3 + (alpha ? elems : 0)) * sizeof(double);
   const dim3 grid(n_ell, n_cosmo);
   auto run = [&](auto kernel, int threads) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kernel, smem);
     kernel<<<grid, threads, smem, st>>>(data, mu, cov, n_cls, n_ell, dense, dense ? structure : nullptr, partial, status,
                                         alpha);
   };
@@ -722,7 +722,7 @@ static size_t sparse_gj_smem(int n) { return (size_t)n * n * sizeof(double); }
 
 void launch_sparse_inv(const double* sp, int n_batch, int n, int nd, double* out, cudaStream_t st) {
   const size_t smem = sparse_gj_smem(n);
-  cudaFuncSetAttribute(sparse_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(sparse_gj_kernel, smem);
   const dim3 grid(nd, n_batch);
   const int elems = n * (n + 1) / 2;
   const size_t sym = 3 * (size_t)n * sizeof(double);
@@ -737,7 +737,7 @@ void launch_sparse_inv(const double* sp, int n_batch, int n, int nd, double* out
 void launch_sparse_slogdet(const double* sp, int n, int nd, double* sign_part, double* ld_part,
                            double* sign_out, double* ld_out, cudaStream_t st) {
   const size_t smem = sparse_gj_smem(n);
-  cudaFuncSetAttribute(sparse_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(sparse_gj_kernel, smem);
   sparse_gj_kernel<<<dim3(nd, 1), 256, smem, st>>>(sp, n, nd, 1, nullptr, sign_part, ld_part);
   sparse_slogdet_reduce<<<1, 32, 0, st>>>(sign_part, ld_part, nd, sign_out, ld_out);
 }

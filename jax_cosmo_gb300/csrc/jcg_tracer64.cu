@@ -604,7 +604,7 @@ static int t64_nodes(int na, int rows) {
 template <int NW>
 static void launch_t64u(const Batch& b, const ConstTables* c, cudaStream_t st) {
   const size_t smem = t64_tab_bytes(NCHI - b.chi_wbase) + sizeof(T64Rec<NW>) * T64_WARPS * 32;
-  cudaFuncSetAttribute(tracer64_uniform_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(tracer64_uniform_kernel<NW>, smem);
   const int groups = (b.n_items + 31) / 32;
   const int per = t64_nodes(b.max_na, groups);
   tracer64_uniform_kernel<NW><<<dim3((b.max_na + per - 1) / per, groups), T64_WARPS * 32, smem, st>>>(b, c, per);

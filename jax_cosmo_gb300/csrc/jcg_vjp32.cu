@@ -1100,12 +1100,12 @@ static void launch_ku(const GradBatch& gb, cudaStream_t st, bool rev) {
   const int wn = NCHI - gb.krev_wbase;
   if (rev) {
     const size_t smem = ku_rev_smem(wn, NW);
-    cudaFuncSetAttribute(grad_kernrev32u_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(grad_kernrev32u_kernel<NW>, smem);
     dim3 grid(kv_chunks(gb.na), (gb.n_items + 31) / 32);
     grad_kernrev32u_kernel<NW><<<grid, 256, smem, st>>>(gb);
   } else {
     const size_t smem = ku_val_smem(wn, NW);
-    cudaFuncSetAttribute(grad_kernval32u_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(grad_kernval32u_kernel<NW>, smem);
     dim3 grid((gb.na + KU_NODES - 1) / KU_NODES, (gb.n_items + 31) / 32);
     grad_kernval32u_kernel<NW><<<grid, 256, smem, st>>>(gb);
   }
@@ -1153,7 +1153,7 @@ static void launch_vjp_t(const GradBatch& gb, cudaStream_t st) {
   // (a listed batch's sizes are maxima: its items take the global sums)
   const int ncacc = (FWD || gb.vjp_cl) && !gb.listed ? vj_cacc(gb.n_cls, gb.n_ell, LT, G) : 0;
   const size_t smem = vj_layout(gb.n_tr, gb.n_cls, LT, ncacc).total;
-  cudaFuncSetAttribute(grad_vjp32_kernel<GEN, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(grad_vjp32_kernel<GEN, FWD>, smem);
   if ((FWD || gb.vjp_cl) && !ncacc) cudaMemsetAsync(gb.cl_count, 0, sizeof(unsigned) * (size_t)gb.n_items, st);
   dim3 grid(G, gb.n_items);
   grad_vjp32_kernel<GEN, FWD><<<grid, VJ_THREADS, smem, st>>>(gb, LT, G);
