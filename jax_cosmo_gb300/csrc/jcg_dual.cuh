@@ -485,6 +485,23 @@ __device__ __forceinline__ void growth_qrT(const BgT<T>& b, double x, T& q, T& r
   r = 1.5 * omm / x / x;
 }
 
+// G(y) of Eisenstein & Hu 1998 eq. 15 (transfer.py:134-137), x = sqrt(1 + y):
+//   y (-6 x + (2 + 3 y) log((x + 1) / (x - 1)))
+// cancels to 1/150 of its terms at y = 3 (alpha_b would be off by 3e-14).  With
+// log((x + 1) / (x - 1)) = 2 atanh(1 / x) and y = x^2 - 1 the terms in x cancel
+// exactly and what is left is a positive series in w = 1 / x^2:
+//   G = y / x sum_{m >= 2} (8 m - 8) / (4 m^2 - 1) w^(m - 1),
+// 42 terms of it for w <= 0.4.
+template <class T>
+__device__ __forceinline__ T eh_G(const T& y, const T& x, const T& lg) {
+  if (!(val(y) >= 1.5)) return y * (-6.0 * x + (2.0 + 3.0 * y) * lg);
+  const T w = 1.0 / (1.0 + y);
+  T p = w * 0.0;
+#pragma unroll
+  for (int m = 43; m >= 2; --m) p = p * w + (8.0 * m - 8.0) / (4.0 * m * m - 1.0);
+  return y / x * (p * w);
+}
+
 // transfer.py:47-142, core.py:145-162 (cosmo_scalars of jcg_tables.cu)
 template <class T>
 __device__ void cosmo_scalarsT(const T* p, T* s, bool nowiggle) {
@@ -527,7 +544,7 @@ __device__ void cosmo_scalarsT(const T* p, T* s, bool nowiggle) {
   beta_c = 1.0 / beta_c;
   const T y = (1.0 + z_eq) / (1.0 + z_d);
   const T x = xsqrt(1.0 + y);
-  const T G = y * (-6.0 * x + (2.0 + 3.0 * y) * xlog((x + 1.0) / (x - 1.0)));
+  const T G = eh_G(y, x, xlog((x + 1.0) / (x - 1.0)));
   const T alpha_b = 2.07 * k_eq * sh_d * xpow(1.0 + R_d, -0.75) * G;
   const T beta_node = 8.41 * xpow(w_m, 0.435);
   const T beta_b = 0.5 + fb + (3.0 - 2.0 * fb) * xsqrt((17.2 * w_m) * (17.2 * w_m) + 1.0);
@@ -553,23 +570,6 @@ __device__ void cosmo_scalarsT(const T* p, T* s, bool nowiggle) {
   s[S_TFNW] = T(p[0] * 0.0 + (nowiggle ? 1.0 : 0.0));
 }
 
-// G(y) of Eisenstein & Hu 1998 eq. 15 (transfer.py:134-137), x = sqrt(1 + y):
-//   y (-6 x + (2 + 3 y) log((x + 1) / (x - 1)))
-// cancels to 1/150 of its terms at y = 3 (alpha_b would be off by 3e-14).  With
-// log((x + 1) / (x - 1)) = 2 atanh(1 / x) and y = x^2 - 1 the terms in x cancel
-// exactly and what is left is a positive series in w = 1 / x^2:
-//   G = y / x sum_{m >= 2} (8 m - 8) / (4 m^2 - 1) w^(m - 1),
-// 42 terms of it for w <= 0.4.
-template <class T>
-__device__ __forceinline__ T eh_G(const T& y, const T& x, const T& lg) {
-  if (!(val(y) >= 1.5)) return y * (-6.0 * x + (2.0 + 3.0 * y) * lg);
-  const T w = 1.0 / (1.0 + y);
-  T p = w * 0.0;
-#pragma unroll
-  for (int m = 43; m >= 2; --m) p = p * w + (8.0 * m - 8.0) / (4.0 * m * m - 1.0);
-  return y / x * (p * w);
-}
-
 // Shuffles of a double or a Dual<1> within a 16-lane half warp (every lane
 // of the warp executes them).
 __device__ __forceinline__ double shfl_t(double x, int src) { return __shfl_sync(0xffffffffu, x, src, 16); }
@@ -582,7 +582,7 @@ __device__ __forceinline__ Dual<1> shfl_t(const Dual<1>& x, int src) {
 
 // The scalars of transfer.py:47-142 and core.py:145-162 for a 16-lane half
 // warp (lane in [0, 16); both halves of the warp execute it, converged): the
-// formulas and calls of the reference's order (cosmo_scalarsT), but the
+// formulas and calls of cosmo_scalarsT, but the
 // independent pow / sqrt / log calls of each level run on different lanes at
 // once (one call site per function and level, lane-selected arguments,
 // results broadcast by shuffles).  The chain's latency is that of 5 levels

@@ -268,4 +268,10 @@ __device__ __forceinline__ DualFF<NDIR> ff8_of(double v, const double* d, int st
   return r;
 }
 
+// The closed form: fp32c's tangents are float, far above what it cancels
+template <int N>
+__device__ __forceinline__ DualFF<N> eh_G(const DualFF<N>& y, const DualFF<N>& x, const DualFF<N>& lg) {
+  return y * (-6.0 * x + (2.0 + 3.0 * y) * lg);
+}
+
 }  // namespace jcg
