@@ -350,6 +350,13 @@ __global__ void __launch_bounds__(GX_THREADS, 2)
   float2* Ms = reinterpret_cast<float2*>(smem + L.M);    // [mb][n_cls][9]
   float* tot = reinterpret_cast<float*>(smem + L.tot);   // [27][lt n_cls]
   const int tid = threadIdx.x;
+  // a cosmology that is left to the float64 kernels already (one thread reads the
+  // flag: other CTAs may set it meanwhile): with narrow bins far apart the integral
+  // in pairs would be 5% of the call, for nothing (16 cosmologies, 3 + 3 bins)
+  __shared__ int left;
+  if (tid == 0) left = tb->wide;
+  __syncthreads();
+  if (left) return;
   const double* ELL = geo_ptr<double>(geo, geo->off_ell);
   const double* EF = geo_ptr<double>(geo, geo->off_ellfac);
   const GxScratch* sc = gx_scratch(tb);
