@@ -616,8 +616,9 @@ __global__ void __launch_bounds__(GR32_THREADS, 3) grad_rows32_kernel(GradBatch 
     }
   }
   const int ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-  const double xpi = tb->sigv[ind] * g2v;
-  const double xc = fmin(fmax(1.0, tb->sigv[1] * g2v), tb->sigv[NRT - 2] * g2v);
+  // (rounded products: see root_segment)
+  const double xpi = __dmul_rn(tb->sigv[ind], g2v);
+  const double xc = fmin(fmax(1.0, __dmul_rn(tb->sigv[1], g2v)), __dmul_rn(tb->sigv[NRT - 2], g2v));
   const int j2 = ind + ((xc - xpi >= 0.0) ? 1 : -1);
   const FF8 xp0 = ff8_of(tb->sigF[ind], tb->sigdF[ind]) * g2;
   const FF8 xp1 = ff8_of(tb->sigF[j2], tb->sigdF[j2]) * g2;

@@ -56,8 +56,9 @@ __device__ HfParams halofit_params_warp(const double* sig, const double* pk3, do
   const double g2 = g * g;
   const int best = root_argmin_warp(sig, g2, lane);
   const int ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-  const double xp_ind = sig[ind] * g2;
-  const double lo = sig[1] * g2, hi = sig[NRT - 2] * g2;
+  // (rounded products: see root_segment)
+  const double xp_ind = __dmul_rn(sig[ind], g2);
+  const double lo = __dmul_rn(sig[1], g2), hi = __dmul_rn(sig[NRT - 2], g2);
   const double xc = fmin(fmax(1.0, lo), hi);  // clip(x, xp[1], xp[-2])
   const int s = (xc - xp_ind >= 0.0) ? 1 : -1;
   const int j2 = ind + s;

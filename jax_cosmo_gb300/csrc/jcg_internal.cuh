@@ -388,8 +388,11 @@ __device__ __forceinline__ void root_segment(const double* sig, double g2, int& 
     }
   }
   ind = best < 1 ? 1 : (best > NRT - 2 ? NRT - 2 : best);
-  const double xc = fmin(fmax(1.0, sig[1] * g2), sig[NRT - 2] * g2);  // clip(x, xp[1], xp[-2])
-  j2 = ind + ((xc - sig[ind] * g2 >= 0.0) ? 1 : -1);
+  // rounded products: past the table's end (k_nl below 0.1 h/Mpc) clip(..) is v_ind
+  // itself, and a product fused into the subtraction would leave its rounding there
+  const double v = __dmul_rn(sig[ind], g2);
+  const double xc = fmin(fmax(1.0, __dmul_rn(sig[1], g2)), __dmul_rn(sig[NRT - 2], g2));  // clip(x, xp[1], xp[-2])
+  j2 = ind + ((xc - v >= 0.0) ? 1 : -1);
 }
 
 // jnp.clip(x, lo) / jnp.clip(x, lo, hi)
