@@ -1,11 +1,9 @@
 // Forward-mode (tangent) arithmetic for the derivative kernels, and the FP64
 // physics of the tables written once for a number type T (double or Dual<N>).
 //
-// Dual<N> carries a value and N tangents.  The derivative kernels use it two
-// ways: Dual<1> with one tangent direction per lane (8 lanes = the 8 Cosmology
-// leaves of core.py:98-108; register use stays that of plain FP64), and
-// Dual<8> for short per-term loops (spectral moments, lensing integrand) where
-// the value part is shared by the 8 directions.
+// Dual<N> carries a value and N tangents.  The derivative kernels use Dual<1>, one
+// tangent direction per thread or lane (the 8 Cosmology leaves of core.py:98-108;
+// register use stays that of plain FP64).
 //
 // Derivative conventions follow JAX's for the reference's operations:
 // max(x, c) / min(x, c) pass the tangent of x where x is the selected branch;
@@ -193,215 +191,6 @@ __device__ __forceinline__ Dual<N> xfmin(const Dual<N>& a, double c) {
   return a.v <= c ? a : dconst<N>(c);
 }
 
-// ---------------------------------------------------------------- DualF ----
-// Value in FP64, N tangents in FP32 (the fp32c Jacobian's table and row
-// stages): the value arithmetic is exactly that of double, each tangent
-// update is one FP32 operation with a factor rounded from FP64.
-template <int N>
-struct DualF {
-  double v;
-  float d[N];
-};
-
-template <int N>
-__device__ __forceinline__ DualF<N> fconst(double v) {
-  DualF<N> r;
-  r.v = v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = 0.f;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ double val(const DualF<N>& x) {
-  return x.v;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator+(const DualF<N>& a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a.v + b.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a.d[i] + b.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator-(const DualF<N>& a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a.v - b.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a.d[i] - b.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator*(const DualF<N>& a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a.v * b.v;
-  const float av = (float)a.v, bv = (float)b.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = fmaf(a.d[i], bv, av * b.d[i]);
-  return r;
-}
-// The tangent factors of division and the elementary functions are formed
-// in FP32 from the rounded value (one float64 division per operation, not
-// two): the tangents are FP32 anyway.
-template <int N>
-__device__ __forceinline__ DualF<N> operator/(const DualF<N>& a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a.v / b.v;
-  const float ib = 1.f / (float)b.v, rv = (float)r.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = (a.d[i] - rv * b.d[i]) * ib;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator-(const DualF<N>& a) {
-  DualF<N> r;
-  r.v = -a.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = -a.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator+(const DualF<N>& a, double b) {
-  DualF<N> r = a;
-  r.v = a.v + b;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator+(double a, const DualF<N>& b) {
-  return b + a;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator-(const DualF<N>& a, double b) {
-  DualF<N> r = a;
-  r.v = a.v - b;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator-(double a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a - b.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = -b.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator*(const DualF<N>& a, double b) {
-  DualF<N> r;
-  r.v = a.v * b;
-  const float bf = (float)b;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * bf;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator*(double a, const DualF<N>& b) {
-  return b * a;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator/(const DualF<N>& a, double b) {
-  DualF<N> r;
-  r.v = a.v / b;
-  const float ib = (float)(1.0 / b);
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * ib;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> operator/(double a, const DualF<N>& b) {
-  DualF<N> r;
-  r.v = a / b.v;
-  const float s = -(float)r.v / (float)b.v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = s * b.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> scale_f(double v, double s, const DualF<N>& a) {
-  DualF<N> r;
-  r.v = v;
-  const float sf = (float)s;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = sf * a.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xexp(const DualF<N>& a) {
-  const double e = exp(a.v);
-  return scale_f(e, e, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> scale_ff(double v, float s, const DualF<N>& a) {
-  DualF<N> r;
-  r.v = v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = s * a.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xlog(const DualF<N>& a) {
-  return scale_ff(log(a.v), 1.f / (float)a.v, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xsqrt(const DualF<N>& a) {
-  const double s = sqrt(a.v);
-  return scale_ff(s, 0.5f / (float)s, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xcbrt(const DualF<N>& a) {
-  const double c = cbrt(a.v);
-  return scale_ff(c, (float)c / (3.f * (float)a.v), a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xsin(const DualF<N>& a) {
-  double sn, cs;
-  sincos(a.v, &sn, &cs);
-  return scale_f(sn, cs, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xcos(const DualF<N>& a) {
-  double sn, cs;
-  sincos(a.v, &sn, &cs);
-  return scale_f(cs, -sn, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xfabs(const DualF<N>& a) {
-  return a.v < 0.0 ? -a : a;
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xpow(const DualF<N>& a, double e) {
-  const double p = pow(a.v, e);
-  return scale_f(p, e * p / a.v, a);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xpow(const DualF<N>& a, const DualF<N>& e) {
-  return xexp(e * xlog(a));
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xfmax(const DualF<N>& a, double c) {
-  return a.v >= c ? a : fconst<N>(c);
-}
-template <int N>
-__device__ __forceinline__ DualF<N> xfmin(const DualF<N>& a, double c) {
-  return a.v <= c ? a : fconst<N>(c);
-}
-
-// value of lane `src` of a warp for a Dual<1> (the tangent of direction src)
-__device__ __forceinline__ Dual<1> shfl_d1(const Dual<1>& x, int src) {
-  Dual<1> r;
-  r.v = __shfl_sync(0xffffffffu, x.v, src);
-  r.d[0] = __shfl_sync(0xffffffffu, x.d[0], src);
-  return r;
-}
-
-// Gather the 8 directions held by lanes 0..7 (one Dual<1> each) into a Dual<8>.
-__device__ __forceinline__ Dual<NDIR> gather8(const Dual<1>& x) {
-  Dual<NDIR> r;
-  r.v = __shfl_sync(0xffffffffu, x.v, 0);
-#pragma unroll
-  for (int i = 0; i < NDIR; ++i) r.d[i] = __shfl_sync(0xffffffffu, x.d[0], i);
-  return r;
-}
-
 // ------------------------------------------------------- templated physics --
 // The float64 formulas of jcg_internal.cuh / jcg_tables.cu / jcg_halofit.cu
 // written for a number type T; grid abscissae (a, k) stay double.
@@ -440,49 +229,10 @@ __device__ __forceinline__ void omT(const BgT<T>& c, double a, double lna, T& om
   omm = c.Om * (ia * ia * ia) / e2;
   omde = c.Ode * ef / e2;
 }
-// background.py:294
-template <class T>
-__device__ __forceinline__ T dchioverdaT(const BgT<T>& c, double a, double lna) {
-  return RH / ((a * a) * xsqrt(esqrT(c, a, lna, (T*)nullptr)));
-}
 // background.py:53
 template <class T>
 __device__ __forceinline__ T wT(const BgT<T>& c, double a) {
   return c.w0 + (1.0 - a) * c.wa;
-}
-// dchi/dln a = R_H / (a sqrt(E^2(a))) with ln a and 1 / a given (background.py:227-229, 294)
-template <class T>
-__device__ __forceinline__ T dchi_dlna_cT(const BgT<T>& c, double a, double lna, double ia) {
-  const T f = -3.0 * (1.0 + c.w0 + c.wa) * lna + 3.0 * c.wa * (a - 1.0);
-  const T ef = xexp(f);
-  const double ia2 = ia * ia;
-  const T e2 = c.Om * (ia2 * ia) + c.Ok * ia2 + c.Ode * ef;
-  return (RH * ia) / xsqrt(e2);
-}
-// growth ODE coefficients with ln x and 1 / x given (background.py:96-106)
-template <class T>
-__device__ __forceinline__ void growth_qr_cT(const BgT<T>& b, double x, double lnx, double ix, T& q, T& r) {
-  const T f = -3.0 * (1.0 + b.w0 + b.wa) * lnx + 3.0 * b.wa * (x - 1.0);
-  const T ef = xexp(f);
-  const double ix2 = ix * ix, ix3 = ix2 * ix;
-  const T ie2 = 1.0 / (b.Om * ix3 + b.Ok * ix2 + b.Ode * ef);
-  const T omm = b.Om * ix3 * ie2, omde = b.Ode * ef * ie2;
-  q = (2.0 - 0.5 * (omm + (1.0 + 3.0 * wT(b, x)) * omde)) * ix;
-  r = 1.5 * omm * ix2;
-}
-// background.py:227-229
-template <class T>
-__device__ __forceinline__ T dchi_dlnaT(const BgT<T>& c, double x) {
-  const double xa = exp(x);
-  return dchioverdaT(c, xa, x) * xa;
-}
-// background.py:96-106
-template <class T>
-__device__ __forceinline__ void growth_qrT(const BgT<T>& b, double x, T& q, T& r) {
-  T omm, omde;
-  omT(b, x, log(x), omm, omde);
-  q = (2.0 - 0.5 * (omm + (1.0 + 3.0 * wT(b, x)) * omde)) / x;
-  r = 1.5 * omm / x / x;
 }
 
 // G(y) of Eisenstein & Hu 1998 eq. 15 (transfer.py:134-137), x = sqrt(1 + y):
@@ -758,56 +508,6 @@ __device__ void cosmo_scalars_warpT(const T* p, T* s, int lane, bool nowiggle) {
   s[S_AGAM] = 1.0 - shfl_t(Q5, 3) + 0.38 * lg223 * (fb * fb);
   s[S_NWQ] = nwq;
   s[S_TFNW] = T(p[0] * 0.0 + (nowiggle ? 1.0 : 0.0));
-}
-
-// transfer.py:88-105, type "eisenhu", at a fixed wavenumber k; not inlined,
-// so that the oscillating fit's callers keep their registers
-template <class T>
-__device__ __noinline__ T eh_nowiggleT(T sh_d, T ag, T nwq, double k) {
-  const T x = 0.43 * k * sh_d, x2 = x * x;
-  const T q = k * nwq / (ag + (1.0 - ag) / (1.0 + x2 * x2));
-  const T L = xlog(2.0 * EULER_E + 1.8 * q);
-  const T C = 14.2 + 731.0 / (1.0 + 62.5 * q);
-  return L / (L + C * q * q);
-}
-
-// transfer.py:107-153 at a fixed wavenumber k (lk = log k); type "eisenhu"
-// (S_TFNW set) by eh_nowiggleT unless NW = false (scalars known to be of type
-// "eisenhu_osc")
-template <bool NW = true, class T>
-__device__ __forceinline__ T eh_transferT(const T* s, double k, double lk) {
-  const T k_eq = s[S_K_EQ], sh_d = s[S_SH_D];
-  if (NW && val(s[S_TFNW]) != 0.0) return eh_nowiggleT(sh_d, s[S_AGAM], s[S_NWQ], k);
-  const T q = k / (13.41 * k_eq);
-  const T q108 = xexp(1.08 * (lk - s[S_LGQ]));
-  const T Cb = 386.0 / (1.0 + 69.9 * q108);
-  const T qq = q * q;
-  const T L1 = xlog(EULER_E + 1.8 * s[S_BETA_C] * q);
-  const T L2 = xlog(EULER_E + 1.8 * q);
-  const T Ta = L1 / (L1 + (14.2 + Cb) * qq);
-  const T Tb = L1 / (L1 + (14.2 / s[S_ALPHA_C] + Cb) * qq);
-  const T Tn = L2 / (L2 + (14.2 + Cb) * qq);
-  const T ksh = k * sh_d;
-  const T x54 = ksh / 5.4, x54s = x54 * x54;
-  const T f = 1.0 / (1.0 + x54s * x54s);
-  const T Tc = f * Ta + (1.0 - f) * Tb;
-  const T bn = s[S_BETA_NODE] / ksh;
-  const T tilde_s = sh_d / xcbrt(1.0 + bn * bn * bn);
-  const T x52 = ksh / 5.2;
-  const T bb = s[S_BETA_B] / ksh;
-  const T silk = xexp(-xexp(1.4 * (lk - s[S_LGKSILK])));
-  const T arg = k * tilde_s;
-  const T sinc = xsin(arg) / arg;
-  const T Tbar = (Tn / (1.0 + x52 * x52) + s[S_ALPHA_B] / (1.0 + bb * bb * bb) * silk) * sinc;
-  return s[S_FB] * Tbar + s[S_FC] * Tc;
-}
-
-// power.py:42-53 at a fixed wavenumber
-template <bool NW = true, class T>
-__device__ __forceinline__ T pk_linearT(const T* s, double k, double lk, const T& g) {
-  const T t = eh_transferT<NW>(s, k, lk);
-  const T pk = xexp(s[S_NS] * lk) * (t * t) * (g * g);
-  return pk * s[S_PKNORM];
 }
 
 // Halofit coefficients at one scale factor from n_eff, C, Omega_m(a),

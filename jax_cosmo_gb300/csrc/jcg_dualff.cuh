@@ -1,13 +1,10 @@
 // Forward-mode tangents with a float-pair value: DualFF<N> carries the value
 // as a float pair (about 48 bits, FP32 pipe; jcg_ff.cuh) and N tangents in
-// FP32.  It replaces DualF<N> (value in FP64) in the fp32c Jacobian's table
-// stages, where the value arithmetic of the per-node evaluations (ODE
-// right-hand sides, Eisenstein-Hu at the Romberg and P(k) nodes) bound the
-// stage on the 1/64-rate FP64 pipe.  The interface is DualF's, so the
-// templated physics of jcg_dual.cuh instantiates with it unchanged; double
-// operands (grid abscissae, constants) become pairs (constants at compile
-// time).  Tangent factors are formed in FP32 from the value's high part, as
-// DualF forms them from the rounded FP64 value.
+// FP32: the numbers of the fp32c Jacobian's table and row stages, whose value
+// arithmetic would bind them to the 1/64-rate FP64 pipe.  The interface is Dual's,
+// so the templated physics of jcg_dual.cuh instantiates with it; double operands
+// (grid abscissae, constants) become pairs (constants at compile time).  Tangent
+// factors are formed in FP32 from the value's high part.
 #pragma once
 
 #include "jcg_dual.cuh"

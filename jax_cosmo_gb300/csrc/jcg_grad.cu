@@ -1,14 +1,15 @@
 // Derivatives of C_ell with respect to the 8 Cosmology leaves (core.py:98-108):
-// the Jacobian dC_ij(l)/dtheta of angular_cl (angular_cl.py:49-98), FP64.
+// the Jacobian dC_ij(l)/dtheta of angular_cl (angular_cl.py:49-98).
 //
 // Tables (background ODEs, sigma8, sigma^2(R), P(k) k^3), per-node halofit
 // parameters and radial kernels are differentiated forward: value + 8
-// tangents.  Scalar chains run with one tangent direction per lane (lanes 0-7
-// of a warp each carry Dual<1>), per-term loops with Dual<8>.  The Limber
-// integrand, evaluated n_ell x Na times, is differentiated backward by a
-// hand-written reverse sweep (node_fb) that returns dP/d(inputs); contracting
-// with the inputs' tangents gives dP/dtheta, and
+// tangents.  The Limber integrand, evaluated n_ell x Na times, is differentiated
+// backward by a hand-written reverse sweep that returns dP/d(inputs);
+// contracting with the inputs' tangents gives dP/dtheta, and
 //   dC_ij(l)/dtheta = ef_ij(l) sum_a [dP(l,a)/dtheta M_ij(a) + P(l,a) dM_ij(a)/dtheta].
+// This file has the scalars, the fp32c tables and rows, the float64 integral of the
+// cosmologies that leave the range of float pairs (node_fb), and the launches;
+// the FP64 stages are in jcg_grad64.cu, jcg_gradfront64.cu and jcg_gradlim64.cu.
 // The tables are recomputed here from the parameters, not taken from a
 // forward pass.  Derivative conventions are JAX's for the reference's
 // operations (max/min pass the tangent of the selected branch; the
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(128, 4) grad_tables_kernel(GradBatch gb, const
     // the three sequential scans as parallel scans (128 threads).
     // Growth: one RK4 step is linear in y = (D, dD/da), y_i = M_i y_{i-1};
     // thread i forms M_i (FP64) and its tangents dM_i (FP32) by running the
-    // step on the unit vectors in DualF<8>.
+    // step on the unit vectors in DualFF<8>.
     double m4[4] = {1.0, 0.0, 0.0, 1.0};
     float dm4[4][NDIR];
 #pragma unroll
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(128, 4) grad_tables_kernel(GradBatch gb, const
   // P(k_i, a = 1) k_i^3 on the halofit grid
   {
     // the node values exp(n_s ln k) T(k)^2 from grad_nodes_kernel, in
-    // pk_linearT's order: ((u g^2) pknorm), then k^3
+    // the order ((u g^2) pknorm), then k^3
     const FF8 g1f = ff8_of(g1s[0], g1s + 1, 1);
     const FF8 g1sq = g1f * g1f;
     const FF8 pkn = ff8_of(sv[S_PKNORM], sd + S_PKNORM, NSCAL);
@@ -492,16 +493,8 @@ __global__ void __launch_bounds__(NRT) grad_moments32_kernel(GradBatch gb, const
 size_t grad_tables_smem() { return sizeof(double) * (NSCAL * (1 + NDIR) + GNODE_U + NDIR + 1); }
 
 // ------------------------------------------------------- fp32c rows -------
-__device__ __forceinline__ F8 interp_f8(double x, const double* xp, const double* fv, const double* fd,
-                                        int stride, int2 sg) {
-  const F8 f0 = f8_of(fv[sg.x], fd + sg.x, stride), f1 = f8_of(fv[sg.y], fd + sg.y, stride);
-  const F8 a = (f1 - f0) / (xp[sg.y] - xp[sg.x]);
-  const F8 b = f0 - a * xp[sg.x];
-  return a * x + b;
-}
-
-// fp32c Jacobian rows: one node per thread in DualF<8> (value FP64, the 8
-// tangents FP32), the operations: root
+// fp32c Jacobian rows: one node per thread in DualFF<8> (value a float
+// pair, the 8 tangents FP32): root
 // find, moments (exp terms for y^2 in [1, 60], Taylor prefix tables below),
 // takahashi2012 coefficients, Limber weight; the row is written as computed.
 // interpolation on the segment sg of a table with tangents, by the segment's
@@ -631,13 +624,13 @@ __global__ void __launch_bounds__(GR32_THREADS, 3) grad_rows32_kernel(GradBatch 
   row[F_LG2KNL] = (ff_log(knl.v) * ffc(1.4426950408889634)).hi;
   row[F_INVKNL] = inv.v.hi;
   put_t(T_KNL, knl, 1.f);
-  // moments: the exp terms for y^2 in [Y2_TAYLOR, Y2_SKIP] in FP32 from a
-  // float-pair y^2 (values summed in float pairs), below Y2_TAYLOR the Taylor
+  // moments: the exp terms for y^2 in [1, 60] in FP32 from a
+  // float-pair y^2 (values summed in float pairs), below 1 the Taylor
   // series from the float-pair tables (Horner with derivatives); the
   // derivatives with respect to R and the tangents in FP32
   const float iR = knl.v.hi;
   const float linv = LN2_F * lg2f(inv.v.hi);
-  constexpr float HLY2T = 0.0f, HLY2S = 2.0471425f;  // 0.5 log(Y2_TAYLOR), 0.5 log(Y2_SKIP)
+  constexpr float HLY2T = 0.0f, HLY2S = 2.0471425f;  // 0.5 log(1), 0.5 log(60)
   int ilo = (int)floorf((HLY2T - linv - (float)LOG_KMIN) * (float)(1.0 / DLOGK));
   int ihi = (int)ceilf((HLY2S - linv - (float)LOG_KMIN) * (float)(1.0 / DLOGK));
   ilo = max(0, min(ilo, NKH));
@@ -1280,10 +1273,9 @@ int grad_limber_tile(int n_ell, int n_cls) {
 }
 
 // The per-node physics of the fp32c table stage with the abscissae as float
-// pairs (ConstTables' *_ff grids): dchi_dlna_cT, growth_qr_cT and
-// eh_transferT / eh_nowiggleT of jcg_dual.cuh with FF in place of their
-// double arguments, the same operations in the same order, so that no
-// operand is converted from float64 at run time.
+// pairs (ConstTables' *_ff grids): chi's and the growth's right-hand sides
+// (background.py:96-106, 227-229) and the transfer function, so that no operand
+// is converted from float64 at run time.
 __device__ __forceinline__ FF8 dchi_dlna_f8(const BgT<FF8>& c, FF a, FF lna, FF ia) {
   const FF8 f = -3.0 * (1.0 + c.w0 + c.wa) * lna + 3.0 * c.wa * (a - ffc(1.0));
   const FF8 ef = xexp(f);

@@ -7,7 +7,6 @@
 namespace jcg {
 
 typedef Dual<1> D1;
-typedef Dual<NDIR> D8;
 
 __device__ __forceinline__ D1 mk1(double v, double d) {
   D1 r;
@@ -15,8 +14,6 @@ __device__ __forceinline__ D1 mk1(double v, double d) {
   r.d[0] = d;
   return r;
 }
-
-typedef DualF<NDIR> F8;
 
 // interpolation (scipy/interpolate.py:55-59) with a dual table fp
 __device__ __forceinline__ D1 interp_d1(double x, const double* xp, const double* fv, const double* fd,
@@ -28,15 +25,6 @@ __device__ __forceinline__ D1 interp_d1(double x, const double* xp, const double
 }
 
 
-
-// DualF<8> from a value and 8 double tangents at stride `stride`
-__device__ __forceinline__ F8 f8_of(double v, const double* d, int stride) {
-  F8 r;
-  r.v = v;
-#pragma unroll
-  for (int i = 0; i < NDIR; ++i) r.d[i] = (float)d[i * stride];
-  return r;
-}
 
 constexpr double TWO_PI2_G = 2.0 * (PI * PI);
 constexpr double C2_G = C_KMS * C_KMS;

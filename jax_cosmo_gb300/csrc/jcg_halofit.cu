@@ -320,11 +320,11 @@ __global__ void __launch_bounds__(HF_WARPS * 32, 8)
     if (model == JCG_PK_LINEAR) {
       ihi = -1;  // linear_matter_power: the halofit moments are not used
     } else {
-      // exp only for y^2 in [Y2_TAYLOR, Y2_SKIP] (the split point only needs
+      // exp only for y^2 in [1, 60] (the split point only needs
       // to be consistent, so it is found in FP32); y^2 = kh^2 inv^2 with
       // inv^2 as a float pair for the FP32 terms
       const float linv = LN2_F * lg2f((float)inv);
-      constexpr float HLY2T = 0.0f, HLY2S = 2.0471425f;  // 0.5 log(Y2_TAYLOR), 0.5 log(Y2_SKIP)
+      constexpr float HLY2T = 0.0f, HLY2S = 2.0471425f;  // 0.5 log(1), 0.5 log(60)
       ilo = (int)floorf((HLY2T - linv - (float)LOG_KMIN) * (float)(1.0 / DLOGK));
       ihi = (int)ceilf((HLY2S - linv - (float)LOG_KMIN) * (float)(1.0 / DLOGK));
       ilo = max(0, min(ilo, NKH));

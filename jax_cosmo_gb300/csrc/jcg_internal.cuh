@@ -21,7 +21,6 @@ constexpr int NRT = 256;     // power.py:93        log R nodes of the sigma^2(R)
 constexpr int NKH = 257;     // power.py:111,136   simps(..., 256) over ln k
 constexpr int NROMB = 129;   // power.py:77        romb(divmax=7): 2 + 1 + 2 + ... + 64
 constexpr int NZP = 257;     // probes.py:51       simps(integrand, z, zmax, 256)
-constexpr int NNORM = 257;   // redshift.py:30     simps(pz_fn, 0, zmax, 256)
 constexpr int MAXTR = JCG_MAX_TRACERS;
 constexpr int MAXPAIR = JCG_MAX_PAIRS;
 
@@ -136,8 +135,6 @@ constexpr int NSCAL = 40;
 // ln k grid of the spectral moments: simps over [ln 1e-4, ln 1e4], 256 intervals (power.py:136)
 constexpr double LOG_KMIN = -0x1.26bb1bbb55515p+3;  // np.log(1e-4)
 constexpr double DLOGK = (0x1.26bb1bbb55516p+3 - -0x1.26bb1bbb55515p+3) / 256.0;
-constexpr double Y2_TAYLOR = 1.0;   // below: exp(-y^2) by its Taylor series (NTAYLOR terms)
-constexpr double Y2_SKIP = 60.0;    // above: exp(-y^2) y^4 P k^3 < 1e-20 of the sum
 constexpr int PAD_CT = 7;        // keeps sizeof(CosmoTab) a multiple of 64
 static_assert(S_NSCALAR <= NSCAL, "scalar block too small");
 
@@ -395,8 +392,7 @@ __device__ __forceinline__ void root_segment(const double* sig, double g2, int& 
   j2 = ind + ((xc - v >= 0.0) ? 1 : -1);
 }
 
-// jnp.clip(x, lo) / jnp.clip(x, lo, hi)
-__device__ __forceinline__ double clip_lo(double x, double lo) { return fmax(x, lo); }
+// jnp.clip(x, lo, hi)
 __device__ __forceinline__ double clip_lohi(double x, double lo, double hi) {
   return fmin(fmax(x, lo), hi);
 }
@@ -476,31 +472,6 @@ __device__ __constant__ const double kExp2Tab64[64] = {
     0x1.ea4afa2a490dap+0, 0x1.efa1bee615a27p+0, 0x1.f50765b6e4540p+0, 0x1.fa7c1819e90d8p+0,
 };
 
-// exp(x) for -700 < x <= 0 by the table-driven method of P. T. P. Tang
-// ("Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic", ACM TOMS 15, 1989): x = (64 m + j) ln2/64 + r
-// with |r| <= ln2/128, exp(x) = 2^m 2^(j/64) e^r, e^r by its Taylor polynomial
-// of degree 6 (truncation < 3e-20 relative).  ln2/64 is split in a 40-bit
-// high part (exact products for |k| < 2^13) and the rest.  `tab` is a copy of
-// kExp2Tab64 in shared memory (lanes index it independently).
-__device__ __forceinline__ double exp_tang(double x, const double* tab) {
-  constexpr double INV_LN2_64 = 92.33248261689366;
-  constexpr double LN2_64_HI = 0x1.62e42fefa2000p-7;
-  constexpr double LN2_64_LO = 0x1.9ef35793c7673p-47;
-  const double kd = rint(x * INV_LN2_64);
-  const double r = fma(-kd, LN2_64_LO, fma(-kd, LN2_64_HI, x));
-  double p = 1.0 / 720.0;
-  p = fma(p, r, 1.0 / 120.0);
-  p = fma(p, r, 1.0 / 24.0);
-  p = fma(p, r, 1.0 / 6.0);
-  p = fma(p, r, 0.5);
-  p = fma(p, r, 1.0);
-  p = fma(p, r, 1.0);
-  const int k = (int)kd;
-  const double two_m = __hiloint2double(((k >> 6) + 1023) << 20, 0);
-  return tab[k & 63] * p * two_m;
-}
-
 // --------------------------------------------------------- background ------
 // background.py:25-196, 270-294 with the reference operation order.
 struct Bg {
@@ -520,7 +491,6 @@ __device__ __forceinline__ double bg_w(const Bg& c, double a) { return c.w0 + (1
 __device__ __forceinline__ double bg_fde_l(const Bg& c, double a, double lna) {
   return -3.0 * (1.0 + c.w0 + c.wa) * lna + 3.0 * c.wa * (a - 1.0);
 }
-__device__ __forceinline__ double bg_fde(const Bg& c, double a) { return bg_fde_l(c, a, log(a)); }
 // E^2(a) (background.py:122-126); a^-3, a^-2 by products of 1/a (no float64
 // pow), exp(f_de) skipped when f_de == 0 (w0 = -1, wa = 0), where it is 1.
 __device__ __forceinline__ double bg_esqr_l(const Bg& c, double a, double lna, double* efde) {
@@ -680,11 +650,6 @@ __device__ __forceinline__ double bg_omm(const Bg& c, double a) {
   double m, d;
   bg_om_l(c, a, log(a), &m, &d);
   return m;
-}
-__device__ __forceinline__ double bg_omde(const Bg& c, double a) {
-  double m, d;
-  bg_om_l(c, a, log(a), &m, &d);
-  return d;
 }
 // dchi/da = rh / (a^2 E(a)) (background.py:294)
 __device__ __forceinline__ double bg_dchioverda_l(const Bg& c, double a, double lna) {

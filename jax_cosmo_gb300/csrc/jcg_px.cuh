@@ -91,7 +91,6 @@ PX_FN FF px_of(double v) {
   const float h = (float)v;
   return FF{h, (float)(v - (double)h)};
 }
-PX_FN double px_d(FF a) { return (double)a.hi + (double)a.lo; }
 // a positive double between 2^-70 and 2^126 as a pair, and a pair (hi > 0) as a
 // double, by integer operations: conversions between float and double issue at
 // the FP64 rate (2 per clock and SM)
