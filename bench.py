@@ -311,7 +311,7 @@ def gpu_arm(args, rank, world, device):
     clocks.mark()
     t_fast, per = timed(lambda: step("fp32c"), args.steps, args.warmup)
     clk = clocks.stop()
-    # plain float64 method on the same workload (fewer steps: it is ~100x slower)
+    # plain float64 method on the same workload (fewer steps: it is about 7x slower)
     t64, per64 = timed(lambda: step("fp64"), max(1, min(args.steps, 2)), 1)
     # e2e through the public host-buffer entry (jcg_angular_cl_host): pinned
     # host params in, C_ell out to pinned host memory, both inside each step

@@ -401,8 +401,9 @@ int jcg_gaussian_loglike_cov_grad(const double* alpha_dev, const double* inv_dev
                                   int n_cosmo, int n_cls, int n_ell, double* cov_bar_dev, cudaStream_t stream);
 
 /* Gaussian log-likelihood with a covariance in the sparse block format
- * (likelihood.py:9-61; sparse.py:295-366): per-ell blocks factored by
- * Cholesky in float64.  data/mu [n_cosmo][n_cls*n_ell] (p*n_ell + l),
+ * (likelihood.py:9-61; sparse.py:295-366): per-ell blocks factored as
+ * L D L^T in float64; an infinite variance masks its data point (without the
+ * log-determinant, which it makes infinite).  data/mu [n_cosmo][n_cls*n_ell] (p*n_ell + l),
  * cov [n_cosmo][n_cls][n_cls][n_ell]; out [n_cosmo].  Returns
  * -0.5 * (r^T C^-1 r - logdet) when include_logdet, as likelihood.py:61.
  * status_dev [n_cosmo] (may be NULL): 0 ok, 2 a block is not positive
@@ -427,9 +428,11 @@ int jcg_gaussian_loglike_dense(const double* data_dev, const double* mu_dev, con
                                size_t workspace_bytes, cudaStream_t stream);
 
 /* sparse.inv / sparse.slogdet of (n, n, ndiag) block-diagonal matrices
- * (sparse.py:295-366), float64, one matrix; n <= JCG_SPARSE_MAX_N.  Each
- * diagonal's n x n matrix is inverted in place by Gauss-Jordan elimination
- * with partial pivoting. */
+ * (sparse.py:295-366), float64, one matrix; n <= JCG_SPARSE_MAX_N.  A diagonal's
+ * n x n matrix that is symmetric (bit for bit) and positive definite is inverted
+ * by the sweep operator on its lower triangle, any other by Gauss-Jordan
+ * elimination with partial pivoting.  out_dev must not overlap sparse_dev
+ * (JCG_ERR_ARG where they are the same). */
 #define JCG_SPARSE_MAX_N 160
 int jcg_sparse_inv(const double* sparse_dev, int n, int ndiag, double* out_dev, cudaStream_t stream);
 /* sparse.inv of n_batch matrices [n_batch][n][n][ndiag] in one launch (the

@@ -9,11 +9,15 @@ jax_cosmo differentiates its whole stack with ``jax.grad`` / ``jax.hessian``
   sweep weighted by the cotangent, so that fp32c never forms J; theta = the
   8 Cosmology leaves of core.py:98-108);
 * ``gaussian_cl_covariance``: the Knox formula (angular_cl.py:144-147) is a
-  product of two C_ell, its vector-Jacobian product is applied with index
-  additions on the device;
+  product of two C_ell; its vector-Jacobian product by
+  ``jcg_gaussian_covariance_vjp``;
 * ``gaussian_log_likelihood``: d logL / d mu = -C^-1 r (C^-1 r from the same
-  per-ell Cholesky as the value), d logL / d C = (C^-1 r r^T C^-1 + C^-1) / 2
-  with the reference's +0.5 logdet sign (likelihood.py:61).
+  per-ell factorisation as the value), d logL / d C = (C^-1 r r^T C^-1 + C^-1) / 2
+  with the reference's +0.5 logdet sign (likelihood.py:61), for the sparse form
+  by ``jcg_gaussian_loglike_cov_grad``.
+
+The last two take torch operations instead where the cotangent is more than its
+values: under ``create_graph``, as a batch of cotangents, with a forward tangent.
 
 ``angular_cl_jacobian`` returns J itself, and ``fisher_matrix`` the Gaussian
 Fisher matrix J^T C^-1 J of a C_ell data vector (the construction of the

@@ -1,12 +1,7 @@
-// Halofit parameters per Limber node (FP64) and pointwise table queries.
-//
-// Phase 1, one warp per scale-factor node: the sigma^2(R) root find of
-// power.py:96-118 and the spectral moments of power.py:121-139.
-// Phase 2, one thread per node: the takahashi2012 coefficients of
-// power.py:177-238 and the Limber weights.  (Scalar per-node work done by one
-// lane of a warp would hold the float64 pipe for all 32 lanes; GB300's FP64
-// rate is ~1/70 of its FP32 rate, so the per-node scalar work runs
-// thread-parallel instead.)
+// Halofit rows of the fp32c method (the root find of power.py:96-118, the spectral
+// moments of power.py:121-139, the coefficients of power.py:177-244 and the Limber
+// weight per scale-factor node) and pointwise queries of the float64 tables.  The
+// plain method's rows are in jcg_tracer64.cu.
 #include "jcg_fp32.cuh"
 #include "jcg_ff.cuh"
 #include "jcg_internal.cuh"
@@ -14,9 +9,6 @@
 #include "jcg_rows.cuh"
 
 namespace jcg {
-
-
-
 
 // argmin_j (1 - sig_j g2)^2 with the first index on ties (scipy/interpolate.py:47).
 // v_j = sig_j g2 is strictly decreasing, so (1 - v_j)^2 is unimodal and the

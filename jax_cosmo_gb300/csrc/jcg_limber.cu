@@ -335,6 +335,7 @@ static void launch_limber32_t(const Batch& b, const ConstTables* c, int lt, cuda
   limber32_kernel<MAXU, GEN><<<grid, LB_THREADS, L.total, st>>>(b, c, lt);
 }
 
+// lt: ell per CTA of the fp32c kernel (launch_limber64 chooses its own)
 void launch_limber(const Batch& b, const ConstTables* c, int lt, cudaStream_t st) {
   if (b.precision == JCG_FP32C) {
     // units per thread: the split path needs one, otherwise lt x ceil(n_cls / 4)

@@ -362,8 +362,11 @@ static void launch_limber64_t(const Batch& b, const ConstTables* c, cudaStream_t
     auto count = [&](int l) { return (long long)b.n_items * ((b.max_ell + l - 1) / l) * R; };
     while (lt > 8 && count(lt) < 2 * sms) lt = even((lt + 1) / 2);
     // a node per thread in each block where clusters are small and the CTAs still fit
-    // at once (50 ell, 257 nodes, clusters of 4: lt 7 29 us, 3 25.8; 513 nodes, of 8:
-    // 31.4 and 34.5, so not there)
+    // at once.  us with and without (50 ell, one cosmology): clusters of 1 24.8 and
+    // 28.8, of 2 26.8 and 28.9, of 3 26.8 and 29.9, of 4 26.8 and 28.9, of 5 26.8 and
+    // 30.8, of 6 26.9 and 30.9, of 7 33.0 and 30.9; of 8 34.5 and 31.4, so not there.
+    // Where the CTAs come to more than one per SM it costs 2 us instead (100 ell,
+    // 257 nodes: one cosmology 26.8 and 28.9, two 32.9 and 30.2)
     const int one = even(PX_THREADS / bsz > 1 ? PX_THREADS / bsz : 1);
     if (R < PX_MAXCL && one < lt && lt <= 8 && count(one) <= 2 * sms) lt = one;
     const int slots = (nblk + R - 1) / R;

@@ -387,7 +387,8 @@ PX_FN long long px_log2_d(double x, const PxTab& T) {
   return ((long long)e << 57) + T.l2[j] + f;
 }
 
-// sin(pi u), 0 <= u < 2^17; COS: and cos(pi u)
+// sin(pi u), 0 <= u < 2^17; COS: and cos(pi u).  (Beyond, the pair's low float exceeds
+// the table's step: 1e-13 at 2^18, no digits from 2^24 on.)
 template <bool COS>
 PX_FN FF px_sincospi(FF u, const PxTab& T, FF* co) {
   const float n = rintf(u.hi * 64.f);

@@ -3,7 +3,7 @@
 //
 // The covariance of angular_cl.py:120-163 is, after permuting (cls, ell) to
 // (ell, cls), block diagonal with one n_cls x n_cls block per ell.  The
-// log-likelihood of likelihood.py:9-61 therefore factors into per-ell Cholesky
+// log-likelihood of likelihood.py:9-61 therefore factors into per-ell L D L^T
 // solves: r^T C^-1 r = sum_l r_l^T A_l^-1 r_l and logdet C = sum_l logdet A_l,
 // which is what the reference's sparse path (sparse.py:295-366) computes by
 // inverse and Schur complements, and its dense path by a full inverse.

@@ -1,5 +1,7 @@
 // Tracer radial kernels and halofit rows of the plain method (precision "fp64") on
-// the Limber nodes.  Rows: see there.  Kernels (probes.py:16-129, 188-272): for a WeakLensing bin
+// the Limber nodes: both need the tables only, and few cosmologies run them in one
+// launch.  Rows: see "halofit rows" below.  Kernels (probes.py:16-129, 188-272): for
+// a WeakLensing bin
 //   q(z) = simps_{z' in [z, zmax], 256}[ n(z') clip(chi' - chi, 0) / clip(chi', 1) ] (1 + z) chi
 // times 3 H0^2 Omega_m / (2 c) and (1 + m), plus the NLA term; for a
 // NumberCounts bin n(z) b H(z).
@@ -611,10 +613,12 @@ static void launch_t64u(const Batch& b, const ConstTables* c, cudaStream_t st) {
 }
 
 void launch_tracer64(const Batch& b, const ConstTables* c, cudaStream_t st) {
-  // lanes over cosmologies from 96 on (3 bins, 513 nodes: 61 cosmologies take
-  // 104 us a warp per node and 434 us with lanes over cosmologies; 4096 about 7 ms
-  // and, 5 bins, 3.5 ms): below, idle SMs and 257-point chains cost more than
-  // the other form's repeated reads of the grid
+  // lanes over cosmologies from 96 on: for few, idle lanes and SMs and its chains of
+  // 257 points cost more than the other form's repeated reads of the grid.  us, a warp
+  // per node / lanes over cosmologies (513 nodes, then 257):
+  //   3 bins, 24 cosmologies  127 /  97,   68 /  96    5 bins, 24  176 / 128,   92 / 128
+  //           96              442 / 125,  247 /  94            96  621 / 160,  346 / 126
+  // so the forms cross between 20 and 40 cosmologies; the line lies above that
   if (!b.listed && b.n_wl_groups == 1 && b.n_wl >= 1 && b.n_wl <= 8 && b.n_items >= 96) {
     switch (b.n_wl) {
       case 1: launch_t64u<1>(b, c, st); return;

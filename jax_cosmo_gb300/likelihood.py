@@ -1,8 +1,8 @@
 """Gaussian log-likelihood (jax_cosmo/likelihood.py:9-61).
 
 The covariance of a Limber C_ell data vector is block diagonal after permuting
-(cls, ell) -> (ell, cls).  libjcg factors the per-ell n_cls x n_cls blocks by
-Cholesky in float64 (``jcg_gaussian_loglike_sparse`` / ``_dense``), which gives
+(cls, ell) -> (ell, cls).  libjcg factors the per-ell n_cls x n_cls blocks as
+L D L^T in float64 (``jcg_gaussian_loglike_sparse`` / ``_dense``), which gives
 the value of the reference's sparse path (inverse + Schur complements) and of
 its dense path (inverse or Cholesky) up to rounding.  A dense matrix that is
 not block diagonal in ell (a user covariance with ell-ell correlations) is
@@ -43,7 +43,7 @@ def _dense_n_ell(C):
 
 
 def _loglike_blocks(r_data, mu, C, n_cls, n_ell, include_logdet, dense, alpha=None):
-    """libjcg per-ell block Cholesky; also writes alpha = C^-1 (mu - data) if given."""
+    """libjcg per-ell block factorisation; also writes alpha = C^-1 (mu - data) if given."""
     device = mu.device
     B = mu.shape[0]
     wsz = ctypes.c_size_t()

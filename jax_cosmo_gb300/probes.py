@@ -6,10 +6,9 @@ kernels are computed by libjcg (FP64): the lensing efficiency integral of
 probes.py:16-74 and the density kernel of probes.py:77-99.
 
 Intrinsic alignment (``ia_bias``: the NLA model of probes.py:102-129, added to
-the shear kernel before the multiplicative bias, probes.py:200-207) and the
-three bias models of bias.py are on the accelerated path.  Not on it (they
-raise NotImplementedError): ``delta_nz`` bins (probes.py:53-64) and non-Smail
-n(z).
+the shear kernel before the multiplicative bias, probes.py:200-207), the three
+bias models of bias.py, tabulated n(z) and, for WeakLensing, ``delta_nz`` bins
+(probes.py:53-64) are on the accelerated path.
 """
 from __future__ import annotations
 
